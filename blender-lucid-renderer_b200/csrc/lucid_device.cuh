@@ -170,8 +170,10 @@ LD float ggxG2(float nl, float nv, float r) {
     if (den < GGX_EPSILON) return 0.0f;
     return 2.0f * nl * nv / den;
 }
-// Heitz 2018 VNDF sampling as written in bsdf/ggx.hpp:130-170
-LD V3 sample_vndf(V3 wo, float rough, float u1, float u2, V3 n, V3 t, V3 b) {
+// Heitz 2018 VNDF sampling as written in bsdf/ggx.hpp:130-170: the half
+// vector in the frame (n, t, b), from the polar point (p1, p2) = sqrt(u1)
+// (cos, sin)(2 pi u2).
+LD V3 sample_vndf_local(V3 wo, float rough, float p1, float p2, V3 n, V3 t, V3 b) {
     V3 wl = make_dir_or(v3(dot(wo, t), dot(wo, b), dot(wo, n)));
     float al = rough * rough;
     V3 ws = make_dir_or(v3(wl.x * al, wl.y * al, wl.z));
@@ -184,30 +186,11 @@ LD V3 sample_vndf(V3 wo, float rough, float u1, float u2, V3 n, V3 t, V3 b) {
     }
     V3 t2;
     if (!make_dir(cross(ws, t1), t2)) t2 = v3(0.f, 1.f, 0.f);
-    float r = sqrtf(u1);
-    float phi = kTWO_PI * u2;
-    float p1 = r * lucid_math::lm_cosf(phi);
-    float p2 = r * lucid_math::lm_sinf(phi);
     float s = 0.5f * (1.0f + ws.z);
     p2 = (1.0f - s) * sqrtf(1.0f - p1 * p1) + s * p2;
     V3 h = t1 * p1 + t2 * p2 + ws * sqrtf(smax(0.0f, 1.0f - p1 * p1 - p2 * p2));
     h = v3(h.x * al, h.y * al, smax(0.0f, h.z));
-    return local_to_world(make_dir_or(h), n, t, b);
-}
-LD float pdf_vndf(V3 wo, V3 h, float rough, V3 n) {
-    float nh = dot(n, h), vh = dot(wo, h), nv = dot(n, wo);
-    if (nh <= 0.0f || vh <= 0.0f || nv <= 0.0f) return 0.0f;
-    float D = ggxD(nh, rough), G1 = ggxG1(nv, rough);
-    return D * G1 / (4.0f * nv);
-}
-LD V3 sample_cos_hemi(float u1, float u2, V3 n) {
-    float r = sqrtf(u1);
-    float th = kTWO_PI * u2;
-    float x = r * lucid_math::lm_cosf(th), y = r * lucid_math::lm_sinf(th);
-    float z = sqrtf(smax(0.0f, 1.0f - u1));
-    V3 t, b;
-    onb(n, t, b);
-    return local_to_world(v3(x, y, z), n, t, b);
+    return make_dir_or(h);
 }
 LD float pdf_cos_hemi(float nl) { return smax(0.0f, nl) * kINV_PI; }
 LD RGB schlick_rgb(float c, RGB f0) {
@@ -234,15 +217,39 @@ LD RGB bsdf_weight(RGB f, float c, float pdf) {
     if (pdf < MIN_PDF) return rgb(0.f, 0.f, 0.f);
     return rgb((f.r / pdf) * c, (f.g / pdf) * c, (f.b / pdf) * c);
 }
-LD RGB eval_bsdf(const Mat& m, V3 wo, V3 wi, V3 n) {
-    float nl = dot(n, wi), nv = dot(n, wo);
+LD float spec_prob(const Mat& m) {
+    if (m.metallic > 0.99f) return 1.0f;
+    float sp = 0.5f * (1.0f + m.metallic) * (1.0f - m.roughness * 0.5f);
+    return sclamp(sp, 0.1f, 0.9f);
+}
+// evalBSDF (bsdf.hpp:132-190) and, with PDF, pdfBSDF (the same half vector,
+// GGX D and cosines serve both).  nl = dot(n, wi).  `hs`: the half vector of
+// the pdf's microfacet term when it is not wi's own (the sampled one).
+template <bool PDF>
+LD RGB eval_bsdf(const Mat& m, V3 wo, V3 wi, V3 n, float nl, float& pdf, const V3* hs = nullptr) {
+    const float nv = dot(n, wo);
+    const V3 h = make_dir_or(wo + wi);
+    const float nh = dot(n, h), vh = smax(dot(wo, h), 0.0f);
+    const float r = smax(m.roughness, MIN_ROUGHNESS);
+    const float D = ggxD(smax(nh, 0.0f), r);
+    if (PDF) {
+        pdf = 0.0f;
+        if (nl > 0.0f) {
+            // pdf_vndf (bsdf/ggx.hpp)
+            float pnh = nh, pvh = dot(wo, h), pD = D;
+            if (hs) {
+                pnh = dot(n, *hs);
+                pvh = dot(wo, *hs);
+                pD = ggxD(pnh, r);
+            }
+            float pv = 0.0f;
+            if (!(pnh <= 0.0f || pvh <= 0.0f || nv <= 0.0f)) pv = pD * ggxG1(nv, r) / (4.0f * nv);
+            const float sp = spec_prob(m);
+            pdf = (sp * pv + (1.0f - sp) * pdf_cos_hemi(nl)) * (1.0f - m.transmission);
+        }
+    }
     if (nl <= 0.0f || nv <= 0.0f) return rgb(0.f, 0.f, 0.f);
     // evalSpecular (bsdf.hpp:132-160)
-    V3 h = make_dir_or(wo + wi);
-    float nh = smax(dot(n, h), 0.0f);
-    float vh = smax(dot(wo, h), 0.0f);
-    float r = smax(m.roughness, MIN_ROUGHNESS);
-    float D = ggxD(nh, r);
     float al = r * r, a2 = al * al;
     float lL = safe_sqrt(a2 + (1.0f - a2) * nl * nl);
     float lV = safe_sqrt(a2 + (1.0f - a2) * nv * nv);
@@ -259,19 +266,6 @@ LD RGB eval_bsdf(const Mat& m, V3 wo, V3 wi, V3 n) {
     RGB kd = rgb((1.0f - Fd.r) * om, (1.0f - Fd.g) * om, (1.0f - Fd.b) * om);
     return mul(diff, kd) + sp;
 }
-LD float spec_prob(const Mat& m) {
-    if (m.metallic > 0.99f) return 1.0f;
-    float sp = 0.5f * (1.0f + m.metallic) * (1.0f - m.roughness * 0.5f);
-    return sclamp(sp, 0.1f, 0.9f);
-}
-LD float pdf_bsdf(const Mat& m, V3 wo, V3 wi, V3 n) {
-    float nl = dot(n, wi);
-    if (nl <= 0.0f) return 0.0f;
-    float sp = spec_prob(m);
-    float r = smax(m.roughness, MIN_ROUGHNESS);
-    V3 h = make_dir_or(wo + wi);
-    return (sp * pdf_vndf(wo, h, r, n) + (1.0f - sp) * pdf_cos_hemi(nl)) * (1.0f - m.transmission);
-}
 
 enum { BS_EVAL = 0, BS_PRECOMP = 1 };
 struct BsdfSample {
@@ -282,66 +276,67 @@ struct BsdfSample {
     int type;   // 0 diffuse, 1 specular, 2 transmission
 };
 // sampleBSDF (bsdf.hpp:198-345).  The glass branch draws one extra uniform.
+// The three lobes share the frame, the polar point and the final rotation
+// (the operations and operands of each are the reference's), and the two
+// reflection lobes their value and pdf.
 LD BsdfSample sample_bsdf(const Mat& m, V3 wo, V3 n, float u1, float u2, float u3, Rng& rng) {
     BsdfSample s;
-    s.wi = v3(0.f, 0.f, 1.f);
     s.kind = BS_EVAL;
     s.f = rgb(0.f, 0.f, 0.f);
     s.pdf = 0.0f;
-    s.type = 0;
-    float rough = smax(m.roughness, MIN_ROUGHNESS);
-    if (m.transmission > 0.0f && u3 < m.transmission) {
-        bool front = dot(wo, n) > 0.0f;
-        V3 fn = front ? n : -n;
+    const float rough = smax(m.roughness, MIN_ROUGHNESS);
+    const float sp = spec_prob(m);
+    const bool glass = m.transmission > 0.0f && u3 < m.transmission;
+    const bool lobe = u1 < sp;            // the microfacet lobe of an opaque sample
+    const bool front = dot(wo, n) > 0.0f;
+    const V3 fn = (glass && !front) ? -n : n;
+    V3 t, b;
+    onb(fn, t, b);
+    float ua = u1;
+    if (!glass) {
+        const float num = lobe ? u1 : u1 - sp, den = lobe ? sp : 1.0f - sp;
+        ua = num / den;
+    }
+    const float r = sqrtf(ua);
+    const float phi = kTWO_PI * u2;
+    const float p1 = r * lucid_math::lm_cosf(phi), p2 = r * lucid_math::lm_sinf(phi);
+    V3 w;
+    if (glass || lobe) w = sample_vndf_local(wo, rough, p1, p2, fn, t, b);
+    else w = v3(p1, p2, sqrtf(smax(0.0f, 1.0f - ua)));
+    w = local_to_world(w, fn, t, b);
+    if (glass) {
+        const V3 h = w;
         float eta = front ? (1.0f / m.ior) : m.ior;
-        V3 t, b;
-        onb(fn, t, b);
-        V3 h = sample_vndf(wo, rough, u1, u2, fn, t, b);
         float F = fresnel_dielectric(fabsf(dot(wo, h)), eta);
         V3 inc = -wo;
         float u4 = randf(rng);
         V3 refr;
         bool refl = (u4 < F) || !refract(inc, h, eta, refr);
+        s.type = refl ? 1 : 2;
+        s.wi = refl ? reflect(inc, h) : refr;
+        float nl = dot(fn, s.wi), nv = dot(fn, wo);
         if (refl) {
-            s.wi = reflect(inc, h);
-            float nl = dot(fn, s.wi), nv = dot(fn, wo);
-            if (nl <= 0.0f || nv <= 0.0f) return s;
-            float w = ggxG2(nl, nv, rough) / (ggxG1(nv, rough) + GGX_EPSILON);
-            s.kind = BS_PRECOMP; s.f = rgb(w, w, w); s.type = 1;
+            if (nl <= 0.0f || nv <= 0.0f) { s.type = 0; return s; }
         } else {
-            s.wi = refr;
-            float nl = fabsf(dot(s.wi, fn)), nv = fabsf(dot(wo, fn));
-            float w = ggxG2(nl, nv, rough) / (ggxG1(nv, rough) + GGX_EPSILON);
-            s.kind = BS_PRECOMP; s.f = rgb(w, w, w); s.type = 2;
+            nl = fabsf(dot(s.wi, fn));
+            nv = fabsf(dot(wo, fn));
         }
+        float g = ggxG2(nl, nv, rough) / (ggxG1(nv, rough) + GGX_EPSILON);
+        s.kind = BS_PRECOMP;
+        s.f = rgb(g, g, g);
         return s;
     }
-    float sp = spec_prob(m);
-    V3 t, b;
-    onb(n, t, b);
-    if (u1 < sp) {
-        V3 h = sample_vndf(wo, rough, u1 / sp, u2, n, t, b);
-        s.wi = reflect(-wo, h);
-        float nl = dot(n, s.wi);
-        if (nl <= 0.0f) return s;
-        RGB f = eval_bsdf(m, wo, s.wi, n);
-        float pdf = (sp * pdf_vndf(wo, h, rough, n) + (1.0f - sp) * pdf_cos_hemi(nl)) * (1.0f - m.transmission);
-        if (rough < 0.05f && m.metallic > 0.5f) {
-            s.kind = BS_PRECOMP; s.f = bsdf_weight(f, nl, pdf);
-        } else {
-            s.kind = BS_EVAL; s.f = f; s.pdf = pdf;
-        }
+    s.type = 0;
+    s.wi = lobe ? reflect(-wo, w) : w;
+    const float nl = dot(n, s.wi);
+    if (nl <= 0.0f) return s;
+    s.f = eval_bsdf<true>(m, wo, s.wi, n, nl, s.pdf, lobe ? &w : nullptr);
+    if (lobe) {
         s.type = 1;
-    } else {
-        float u1a = (u1 - sp) / (1.0f - sp);
-        s.wi = sample_cos_hemi(u1a, u2, n);
-        float nl = dot(n, s.wi);
-        if (nl <= 0.0f) return s;
-        RGB f = eval_bsdf(m, wo, s.wi, n);
-        V3 h = make_dir_or(wo + s.wi);
-        float pdf = (sp * pdf_vndf(wo, h, rough, n) + (1.0f - sp) * pdf_cos_hemi(nl)) * (1.0f - m.transmission);
-        s.kind = BS_EVAL; s.f = f; s.pdf = pdf;
-        s.type = 0;
+        if (rough < 0.05f && m.metallic > 0.5f) {
+            s.kind = BS_PRECOMP;
+            s.f = bsdf_weight(s.f, nl, s.pdf);
+        }
     }
     return s;
 }

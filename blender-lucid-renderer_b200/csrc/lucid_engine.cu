@@ -270,42 +270,46 @@ LD V3 primary_dir(const FrameParams& f, float nx, float ny) {
     return make_dir_or(v, v3(f.fwd[0], f.fwd[1], f.fwd[2]));
 }
 
-// Primary ray of wave path `id` (pybind_renderer.hpp:250-293): NDC, seed
-// (x, y, offset + s), two jitter draws when the call has more than one
-// sample; writes the path's initial state and returns the direction (the
-// origin is the camera position, tMin 0).
-LD V3 camera_ray_at(const FrameParams& f, const PathView& pv, int local, int id);
-LD V3 camera_ray(const FrameParams& f, const PathView& pv, int id) { return camera_ray_at(f, pv, id, id); }
-
-// The same for path `local` of the frame `f` stored at wave path `id`
-// (a batched job's paths start at its base in the wave).
-LD V3 camera_ray_at(const FrameParams& f, const PathView& pv, int local, int id) {
+// Primary ray of path `local` of the frame (pybind_renderer.hpp:250-293):
+// NDC, seed (x, y, offset + s), two jitter draws when the call has more than
+// one sample; returns the direction (the origin is the camera position, tMin
+// 0) and the path's RNG stream.
+LD V3 camera_dir(const FrameParams& f, int local, Rng& rng) {
     int p = local % f.npix, sl = local / f.npix;
     int gx = f.tile_x + p % f.tile_w, gy = f.tile_y + p / f.tile_w;
     float nx = (2.0f * ((float)gx + 0.5f) / (float)f.full_w - 1.0f) * f.aspect;
     float ny = 1.0f - 2.0f * ((float)gy + 0.5f) / (float)f.full_h;
     const int offset = f.dyn ? f.dyn[0] : f.sample_offset;
-    Rng rng = seed_xyz((uint32_t)gx, (uint32_t)gy, (uint32_t)(offset + f.s0 + sl));
-    V3 d;
+    rng = seed_xyz((uint32_t)gx, (uint32_t)gy, (uint32_t)(offset + f.s0 + sl));
     if (f.samples > 1 || f.jitter) {
         float jx = (randf(rng) - 0.5f) / (float)f.full_w;
         float jy = (randf(rng) - 0.5f) / (float)f.full_h;
-        d = primary_dir(f, nx + jx, ny + jy);
-    } else {
-        d = primary_dir(f, nx, ny);
+        return primary_dir(f, nx + jx, ny + jy);
     }
+    return primary_dir(f, nx, ny);
+}
+
+LD void records_begin(const PathView& pv, int id) {
+    pv.rec_prim[id] = make_int2(-1, -1);
+    pv.rec_cnt[id] = make_int4(0, 0, 0, 0);
+    pv.rec_hash[id] = 1469598103934665603ULL;
+}
+
+// The primary ray of path `local` of the frame `f` stored as wave path `id`
+// (a batched job's paths start at its base in the wave) with the path's
+// initial state.
+LD V3 camera_ray_at(const FrameParams& f, const PathView& pv, int local, int id) {
+    Rng rng;
+    const V3 d = camera_dir(f, local, rng);
     pv.rng[id] = make_ulonglong2(rng.state, rng.inc);
     pv.ray_o[id] = make_float4(f.pos[0], f.pos[1], f.pos[2], 0.0f);
     pv.ray_d[id] = make_float4(d.x, d.y, d.z, __int_as_float(0));
     pv.thr[id] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
     pv.rad[id] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (f.records) {
-        pv.rec_prim[id] = make_int2(-1, -1);
-        pv.rec_cnt[id] = make_int4(0, 0, 0, 0);
-        pv.rec_hash[id] = 1469598103934665603ULL;
-    }
+    if (f.records) records_begin(pv, id);
     return d;
 }
+LD V3 camera_ray(const FrameParams& f, const PathView& pv, int id) { return camera_ray_at(f, pv, id, id); }
 
 // Primary rays alone, for the passes that do not trace them at once.
 __global__ void k_raygen(FrameParams f, PathView pv) {
@@ -549,7 +553,7 @@ __global__ void __launch_bounds__(128) k_trace_primary_batch(PathView pv, const 
 // of the wave's scene table the path's camera ray chose.
 template <bool MULTI>
 LD const DevScene& path_scene(const DevScene& sc, const PathView& pv, int id) {
-    if constexpr (MULTI) return pv.scenes[pv.sid[id]];
+    if constexpr (MULTI) return pv.scenes[id >= 0 ? pv.sid[id] : 0];
     else return sc;
 }
 
@@ -641,14 +645,6 @@ __global__ void __launch_bounds__(128, MINB) k_trace_lb(DevScene sc0, PathView p
 }
 
 // ---------------------------------------------------------------- shade
-struct ShadeResult {
-    bool cont, shadow;
-};
-
-// One path segment: volume sampling, native-light / environment / emission
-// terms, NEE, BSDF sampling and Russian roulette.  ALGO is the integrator as
-// a compile-time constant, so each integrator's kernel carries only its own
-// branches.
 // Adds a radiance contribution c (already weighted by the path throughput)
 // to the training records of the path's guided vertices from slot `from` on
 // (c / throughput-after-vertex = radiance that arrived along its sample).
@@ -726,96 +722,101 @@ LD bool guide_eligible(const DevMaterial& dm) {
     return dm.rough_trans_ior_flags.y == 0.0f && !(rough < 0.05f && dm.albedo_metallic.w > 0.5f);
 }
 
-template <int ALGO, bool GUIDE = false>
-LD ShadeResult shade_path(const DevScene& sc, const FrameParams& f, const PathView& pv, int id) {
-    ShadeResult out;
-    out.cont = false;
-    out.shadow = false;
-    int pushed = 0;
+// A path between two segments: the ray to trace next (its depth counts the
+// segments before it), throughput, pdf of the sampler that chose the ray and
+// the RNG stream.
+struct PathRegs {
+    V3 o, d;
+    RGB T;
+    float last_pdf;
+    int depth;
+    Rng rng;
+};
+// A light sample waiting for its shadow ray.
+struct ShadowRay {
+    V3 o, d;
+    float len;
+    RGB inc;
+    int pushed;   // the first guide slot the contribution credits (a vertex's
+                  // own light sample did not arrive along its sampled direction)
+};
+struct ShadeResult {
+    bool cont, shadow;
+    RGB add;      // radiance of the event (zero: none)
+};
+struct NoSync {
+    LD void operator()() const {}
+};
+struct BlockSync {
+    LD void operator()() const { __syncthreads(); }
+};
+
+// One path segment on a path held in registers: the closest hit hh = (t, u,
+// v, prim) and the native-light hit lh = (index, t) of its ray give the
+// radiance of this event (add), the light sample (sr, when `shadow` is set)
+// and, when `cont` is set, the next ray (o, d, depth) of the path.
+//
+// The segment runs in phases — medium, hit and emission, light sample,
+// direction sample — with `sync` between them, which every lane reaches
+// whatever became of its path (`live`: the lane has one).  k_shade passes a
+// block barrier: the code of a segment is far larger than an SM's
+// instruction caches near the schedulers, and warps that march through it
+// together share every fetched line.  Events of one phase share code where
+// they do the same operations on the same operands (the light sample of a
+// medium scatter and of a surface, the two reflection lobes' directions,
+// values and pdfs), which shortens the code and keeps more lanes together.
+template <int ALGO, bool GUIDE, class Sync>
+LD ShadeResult shade_segment(const DevScene& sc, bool live, int max_depth, bool records, const PathView& pv, int id,
+                             PathRegs& ps, const float4 hh, const float2 lh, ShadowRay& sr, Sync sync) {
     constexpr int algo = ALGO;
     constexpr bool nee = algo == ALGO_NEE || algo == ALGO_MIS || algo == ALGO_VOLUME_MIS;
     constexpr bool mis = algo == ALGO_MIS || algo == ALGO_VOLUME_MIS;
-    float4 ro = pv.ray_o[id], rd = pv.ray_d[id];
-    V3 o = f3(ro), d = f3(rd);
-    int depth = __float_as_int(rd.w);
-    float4 th = pv.thr[id];
-    RGB T = c3(th);
-    float last_pdf = th.w;
-    RGB result = c3(pv.rad[id]);
-    ulonglong2 rs = pv.rng[id];
-    Rng rng;
-    rng.state = rs.x;
-    rng.inc = rs.y;
-    float4 hh = pv.hit[id];
-    int prim = __float_as_int(hh.w);
-    bool has_hit = prim >= 0;
-    float2 lh = pv.lhit[id];
-    int lidx = __float_as_int(lh.x);
-    bool has_lh = lidx >= 0;
-    V3 new_o = o, new_d = d;
-    V3 sh_o = o, sh_d = d;
-    float sh_len = 0.0f;
-    RGB sh_inc = rgb(0.f, 0.f, 0.f);
+    ShadeResult out;
+    out.cont = false;
+    out.shadow = false;
+    out.add = rgb(0.f, 0.f, 0.f);
+    const int depth = ps.depth;
+    const int prim = __float_as_int(hh.w), lidx = __float_as_int(lh.x);
+    const bool has_hit = prim >= 0, has_lh = lidx >= 0;
+    RGB T = ps.T;
+    float last_pdf = ps.last_pdf;
+    const V3 wo = -ps.d;
+    V3 p = ps.o;
+    int vi = -1;   // the volume the path scatters in before its hit
 
-    do {
-        if (algo == ALGO_VOLUME_SIMPLE) {
-            float ts = 1e6f;
-            if (has_hit) ts = smin(ts, hh.x);
-            if (has_lh) ts = smin(ts, lh.y);
-            T = mul(T, volume_transmittance(sc, o, d, ts, false));
+    // ---- medium
+    if (algo == ALGO_VOLUME_SIMPLE && live) {
+        float ts = 1e6f;
+        if (has_hit) ts = smin(ts, hh.x);
+        if (has_lh) ts = smin(ts, lh.y);
+        T = mul(T, volume_transmittance(sc, ps.o, ps.d, ts, false));
+    }
+    if (algo == ALGO_VOLUME_MIS && live) {
+        float ts = 1e6f;
+        if (has_hit) ts = smin(ts, hh.x);
+        if (has_lh) ts = smin(ts, lh.y);
+        float vt = 0.0f;
+        vi = sample_volume_distance(sc, ps.o, ps.d, ts, ps.rng, vt);
+        if (records) pv.rec_hash[id] = hpush(pv.rec_hash[id], vi >= 0 ? 1u : 0u);
+        if (vi >= 0) {
+            // scatter event (path_tracer.hpp:616-700)
+            const DevVolume& v = sc.volumes[vi];
+            T = mul(T, rgb(v.color[0] / (1.0f + v.absorption[0]), v.color[1] / (1.0f + v.absorption[1]),
+                           v.color[2] / (1.0f + v.absorption[2])));
+            p = ps.o + ps.d * vt;
         }
-        if (algo == ALGO_VOLUME_MIS) {
-            float ts = 1e6f;
-            if (has_hit) ts = smin(ts, hh.x);
-            if (has_lh) ts = smin(ts, lh.y);
-            float vt = 0.0f;
-            int vi = sample_volume_distance(sc, o, d, ts, rng, vt);
-            if (f.records) pv.rec_hash[id] = hpush(pv.rec_hash[id], vi >= 0 ? 1u : 0u);
-            if (vi >= 0) {
-                // scatter event (path_tracer.hpp:616-700)
-                const DevVolume& v = sc.volumes[vi];
-                T = mul(T, rgb(v.color[0] / (1.0f + v.absorption[0]), v.color[1] / (1.0f + v.absorption[1]),
-                               v.color[2] / (1.0f + v.absorption[2])));
-                V3 x = o + d * vt;
-                V3 wo = -d;
-                float g = v.anisotropy;
-                if (sc.num_lights > 0) {
-                    float usel = randf(rng);
-                    int li = select_light(sc, usel);
-                    const DevLight& L = sc.lights[li];
-                    float lsp = area_ratio(L.normal_area.w, sc.total_light_area);
-                    if (lsp > 1e-6f) {
-                        float u1 = randf(rng), u2 = randf(rng);
-                        LightSample ls = sample_light(L, x, u1, u2);
-                        if (ls.pdf > MIN_PDF) {
-                            RGB Tsh = volume_transmittance(sc, x, ls.dir, ls.dist, true);
-                            float ct = dot(wo, ls.dir);
-                            float pe = hg_eval(g, ct);
-                            float pl = ls.pdf * lsp;
-                            float mw = mis_power(pl, pe);
-                            RGB pw = bsdf_weight(rgb(pe, pe, pe), 1.0f, pl);
-                            RGB c = mul(pw * mw, mul(Tsh, ls.emission));
-                            sh_inc = mul(T, c);
-                            sh_o = x; sh_d = ls.dir; sh_len = ls.dist;
-                            out.shadow = true;
-                        }
-                    }
-                }
-                float u1 = randf(rng), u2 = randf(rng);
-                float ppdf;
-                V3 wi = hg_sample(g, wo, u1, u2, ppdf);
-                last_pdf = ppdf;
-                new_o = x; new_d = wi;
-                if (depth >= 3) {
-                    float rr = smin(smax3(T.r, T.g, T.b), 0.95f);
-                    if (randf(rng) > rr) break;
-                    T = T * (1.0f / rr);
-                }
-                if (!rgb_valid(T)) break;
-                out.cont = true;
-                break;
-            }
-        }
+    }
+    sync();
+
+    // ---- hit and emission
+    const bool scat = algo == ALGO_VOLUME_MIS && vi >= 0;
+    bool surf = false, has_em = false, guided = false;
+    V3 n = wo, sn = wo;
+    Mat m;
+    m.albedo = rgb(0.f, 0.f, 0.f);
+    m.metallic = m.transmission = 0.0f;
+    m.roughness = m.ior = 1.0f;
+    if (live && !scat) {
         if (has_lh && (!has_hit || lh.y < hh.x)) {
             // native light hit (path_tracer.hpp:429-452)
             const DevLight& L = sc.lights[sc.native_start + lidx];
@@ -825,216 +826,274 @@ LD ShadeResult shade_path(const DevScene& sc, const FrameParams& f, const PathVi
                 if (sc.num_lights > 0) {
                     float sp = area_ratio(L.normal_area.w, sc.total_light_area);
                     if (sp > 0.0f) {
-                        V3 lp = o + d * lh.y;
+                        V3 lp = ps.o + ps.d * lh.y;
                         V3 ln = (__float_as_int(L.pos_type.w) == LIGHT_POINT) ? normalize_nz(lp - f3(L.pos_type))
                                                                               : f3(L.normal_area);
-                        lpdf = pdf_light(L.normal_area.w, o, lp, ln) * sp;
+                        lpdf = pdf_light(L.normal_area.w, ps.o, lp, ln) * sp;
                     }
                 }
                 float mw = (last_pdf > MIN_PDF && lpdf > MIN_PDF) ? mis_power(last_pdf, lpdf) : 1.0f;
-                result = result + mul(T, em) * mw;
-                if (GUIDE) guide_credit(pv, id, mul(T, em) * mw, 0);
+                out.add = mul(T, em) * mw;
             } else {
-                result = result + mul(T, em);
+                out.add = mul(T, em);
             }
-            break;
-        }
-        if (!has_hit) {
-            result = result + mul(T, rgb(sc.env[0], sc.env[1], sc.env[2]));
-            if (GUIDE) guide_credit(pv, id, mul(T, rgb(sc.env[0], sc.env[1], sc.env[2])), 0);
-            break;
-        }
-        // surface hit: point and normal from (t, u, v, prim) as in bvh.hpp:108-128
-        V3 p = o + d * hh.x;
-        int4 pi = sc.prim_info[prim];
-        V3 fn = f3(sc.prim_fn[prim]);
-        V3 n = fn;
-        if (pi.w) {
-            float u = hh.y, v = hh.z;
-            float w = 1.0f - u - v;
-            V3 ni = f3(sc.prim_vn[3 * prim]) * w + f3(sc.prim_vn[3 * prim + 1]) * u + f3(sc.prim_vn[3 * prim + 2]) * v;
-            n = make_dir_or(ni, fn);
-        }
-        const DevMaterial& dm = sc.materials[pi.x];
-        Mat m;
-        m.albedo = c3(dm.albedo_metallic);
-        m.metallic = dm.albedo_metallic.w;
-        m.roughness = smax(dm.rough_trans_ior_flags.x, MIN_ROUGHNESS);
-        m.transmission = dm.rough_trans_ior_flags.y;
-        m.ior = dm.rough_trans_ior_flags.z;
-        RGB em = c3(dm.emission);
-        bool has_em = dm.emission.w != 0.0f;
-        apply_textures(sc, dm, prim, hh.y, hh.z, m.albedo, em, has_em);
-        V3 wo = -d;
-        bool front = dot(wo, n) > 0;
-        V3 sn = n;
-        if (m.transmission < 0.5f && !front) sn = -n;
-        if (!nee) {
-            result = result + mul(T, em);
-        } else if (!mis) {
-            if (has_em && depth == 0) result = result + mul(T, em);
-        } else if (has_em) {
-            float mw = 1.0f;
-            if (sc.num_lights > 0 && last_pdf > MIN_PDF && pi.z >= 0) {
-                const DevLight& L = sc.lights[pi.z];
-                float sp = area_ratio(L.normal_area.w, sc.total_light_area);
-                if (sp > 0.0f) {
-                    float lpdf = pdf_light(L.normal_area.w, o, p, n) * sp;
-                    if (lpdf > MIN_PDF) mw = mis_power(last_pdf, lpdf);
-                }
+            if (GUIDE) guide_credit(pv, id, out.add, 0);
+        } else if (!has_hit) {
+            out.add = mul(T, rgb(sc.env[0], sc.env[1], sc.env[2]));
+            if (GUIDE) guide_credit(pv, id, out.add, 0);
+        } else {
+            // surface hit: point and normal from (t, u, v, prim) as in bvh.hpp:108-128
+            surf = true;
+            p = ps.o + ps.d * hh.x;
+            int4 pi = sc.prim_info[prim];
+            V3 fn = f3(sc.prim_fn[prim]);
+            n = fn;
+            if (pi.w) {
+                float u = hh.y, v = hh.z;
+                float w = 1.0f - u - v;
+                V3 ni = f3(sc.prim_vn[3 * prim]) * w + f3(sc.prim_vn[3 * prim + 1]) * u + f3(sc.prim_vn[3 * prim + 2]) * v;
+                n = make_dir_or(ni, fn);
             }
-            result = result + mul(T, em) * mw;
-            if (GUIDE) guide_credit(pv, id, mul(T, em) * mw, 0);
-        }
-        bool transmissive = m.transmission > 0.5f;
-        const bool guided = GUIDE && depth < pv.gdepth && guide_eligible(dm);
-        const float* gm = GUIDE ? pv.gmix + (size_t)id * kGMixFloats : nullptr;
-        if (nee && sc.num_lights > 0 && !has_em && !transmissive) {
-            float usel = randf(rng);
-            int li = select_light(sc, usel);
-            const DevLight& L = sc.lights[li];
-            float lsp = area_ratio(L.normal_area.w, sc.total_light_area);
-            if (lsp > 1e-6f) {
-                float u1 = randf(rng), u2 = randf(rng);
-                LightSample ls = sample_light(L, p, u1, u2);
-                if (ls.pdf > MIN_PDF) {
-                    float nl = dot(sn, ls.dir);
-                    if (nl > 1e-6f) {
-                        RGB fb = eval_bsdf(m, wo, ls.dir, sn);
-                        float pl = ls.pdf * lsp;
-                        RGB c;
-                        if (mis) {
-                            float pb = pdf_bsdf(m, wo, ls.dir, sn);
-                            if (guided) pb = 0.5f * pb + 0.5f * guide_pdf_c(gm, ls.dir);
-                            float mw = mis_power(pl, pb);
-                            RGB bw = bsdf_weight(fb, nl, pl);
-                            if (algo == ALGO_VOLUME_MIS) {
-                                RGB Tsh = volume_transmittance(sc, p, ls.dir, ls.dist, true);
-                                c = mul(bw * mw, mul(Tsh, ls.emission));
-                            } else {
-                                c = mul(bw * mw, ls.emission);
-                            }
-                        } else {
-                            c = mul(bsdf_weight(fb, nl, pl), ls.emission);
-                        }
-                        sh_inc = mul(T, c);
-                        sh_o = p; sh_d = ls.dir; sh_len = ls.dist;
-                        out.shadow = true;
+            const DevMaterial& dm = sc.materials[pi.x];
+            m.albedo = c3(dm.albedo_metallic);
+            m.metallic = dm.albedo_metallic.w;
+            m.roughness = smax(dm.rough_trans_ior_flags.x, MIN_ROUGHNESS);
+            m.transmission = dm.rough_trans_ior_flags.y;
+            m.ior = dm.rough_trans_ior_flags.z;
+            RGB em = c3(dm.emission);
+            has_em = dm.emission.w != 0.0f;
+            apply_textures(sc, dm, prim, hh.y, hh.z, m.albedo, em, has_em);
+            sn = n;
+            if (m.transmission < 0.5f && !(dot(wo, n) > 0)) sn = -n;
+            if (!nee) {
+                out.add = mul(T, em);
+            } else if (!mis) {
+                if (has_em && depth == 0) out.add = mul(T, em);
+            } else if (has_em) {
+                float mw = 1.0f;
+                if (sc.num_lights > 0 && last_pdf > MIN_PDF && pi.z >= 0) {
+                    const DevLight& L = sc.lights[pi.z];
+                    float sp = area_ratio(L.normal_area.w, sc.total_light_area);
+                    if (sp > 0.0f) {
+                        float lpdf = pdf_light(L.normal_area.w, ps.o, p, n) * sp;
+                        if (lpdf > MIN_PDF) mw = mis_power(last_pdf, lpdf);
                     }
                 }
+                out.add = mul(T, em) * mw;
+                if (GUIDE) guide_credit(pv, id, out.add, 0);
+            }
+            guided = GUIDE && depth < pv.gdepth && guide_eligible(dm);
+        }
+    }
+    sync();
+
+    // ---- light sample, at a surface or at a scatter point
+    const float* gm = GUIDE ? pv.gmix + (size_t)id * kGMixFloats : nullptr;
+    if (nee && sc.num_lights > 0 && (scat || (surf && !has_em && !(m.transmission > 0.5f)))) {
+        float usel = randf(ps.rng);
+        const DevLight& L = sc.lights[select_light(sc, usel)];
+        float lsp = area_ratio(L.normal_area.w, sc.total_light_area);
+        if (lsp > 1e-6f) {
+            float u1 = randf(ps.rng), u2 = randf(ps.rng);
+            LightSample ls = sample_light(L, p, u1, u2);
+            if (ls.pdf > MIN_PDF) {
+                const float pl = ls.pdf * lsp;
+                float nl = 1.0f, pb = 0.0f;
+                RGB fb = rgb(0.f, 0.f, 0.f);
+                if (scat) {
+                    pb = hg_eval(sc.volumes[vi].anisotropy, dot(wo, ls.dir));
+                    fb = rgb(pb, pb, pb);
+                } else {
+                    nl = dot(sn, ls.dir);
+                    if (nl > 1e-6f) fb = eval_bsdf<mis>(m, wo, ls.dir, sn, nl, pb);
+                }
+                if (nl > 1e-6f) {
+                    RGB c = bsdf_weight(fb, nl, pl);
+                    if (mis) {
+                        if (guided) pb = 0.5f * pb + 0.5f * guide_pdf_c(gm, ls.dir);
+                        c = c * mis_power(pl, pb);
+                    }
+                    if (algo == ALGO_VOLUME_MIS) {
+                        RGB Tsh = volume_transmittance(sc, p, ls.dir, ls.dist, true);
+                        c = mul(c, mul(Tsh, ls.emission));
+                    } else {
+                        c = mul(c, ls.emission);
+                    }
+                    sr.inc = mul(T, c);
+                    sr.o = p;
+                    sr.d = ls.dir;
+                    sr.len = ls.dist;
+                    out.shadow = true;
+                }
             }
         }
-        V3 smp_n = (m.transmission > 0.5f) ? n : sn;
-        V3 wi;
-        float gpdf = 0.0f;
+    }
+    sync();
+
+    // ---- next direction
+    V3 wi = wo;
+    float gpdf = 0.0f;
+    if (scat) {
+        float u1 = randf(ps.rng), u2 = randf(ps.rng);
+        wi = hg_sample(sc.volumes[vi].anisotropy, wo, u1, u2, last_pdf);
+        out.cont = true;
+    } else if (surf) {
+        const V3 smp_n = (m.transmission > 0.5f) ? n : sn;
+        float usel = 0.0f;
+        if (guided) usel = randf(ps.rng);
+        float u1 = randf(ps.rng), u2 = randf(ps.rng), u3 = randf(ps.rng);
         if (guided) {
             // one-sample MIS of BSDF and guide sampling, 1/2 each (balance heuristic)
-            float usel = randf(rng);
-            float u1 = randf(rng), u2 = randf(rng), u3 = randf(rng);
-            if (usel < 0.5f) wi = sample_bsdf(m, wo, smp_n, u1, u2, u3, rng).wi;
+            if (usel < 0.5f) wi = sample_bsdf(m, wo, smp_n, u1, u2, u3, ps.rng).wi;
             else wi = guide_sample_c(gm, u1, u2, u3);
             float c = dot(smp_n, wi);
-            if (c <= 1e-6f) break;
-            gpdf = 0.5f * pdf_bsdf(m, wo, wi, smp_n) + 0.5f * guide_pdf_c(gm, wi);
-            if (!(gpdf > MIN_PDF)) break;
-            T = mul(T, bsdf_weight(eval_bsdf(m, wo, wi, smp_n), c, gpdf));
-            last_pdf = gpdf;
+            if (!(c <= 1e-6f)) {
+                float pb;
+                RGB f = eval_bsdf<true>(m, wo, wi, smp_n, c, pb);
+                gpdf = 0.5f * pb + 0.5f * guide_pdf_c(gm, wi);
+                if (gpdf > MIN_PDF) {
+                    T = mul(T, bsdf_weight(f, c, gpdf));
+                    last_pdf = gpdf;
+                    out.cont = true;
+                }
+            }
         } else {
-            float u1 = randf(rng), u2 = randf(rng), u3 = randf(rng);
-            BsdfSample bs = sample_bsdf(m, wo, smp_n, u1, u2, u3, rng);
-            if (!(bs.kind == BS_PRECOMP || bs.pdf > MIN_PDF)) break;
-            RGB w;
-            if (bs.kind == BS_PRECOMP) {
-                w = bs.f;
-            } else {
+            BsdfSample bs = sample_bsdf(m, wo, smp_n, u1, u2, u3, ps.rng);
+            RGB w = bs.f;
+            out.cont = true;
+            if (bs.kind != BS_PRECOMP) {
                 float c = fabsf(dot(smp_n, bs.wi));
-                if (c <= 1e-6f || bs.pdf < MIN_PDF) break;
-                w = bsdf_weight(bs.f, c, bs.pdf);
+                if (!(bs.pdf > MIN_PDF) || c <= 1e-6f) out.cont = false;
+                else w = bsdf_weight(bs.f, c, bs.pdf);
             }
             T = mul(T, w);
             if (mis) last_pdf = (bs.kind == BS_EVAL) ? bs.pdf : 0.0f;
             wi = bs.wi;
         }
-        if (depth >= 3) {
-            float rr = smin(smax3(T.r, T.g, T.b), 0.95f);
-            if (randf(rng) > rr) break;
-            T = T * (1.0f / rr);
-        }
-        if (!rgb_valid(T)) break;
-        new_o = p; new_d = wi;
-        out.cont = true;
-        if (guided) {
-            // warp-aggregated counters: guided vertices, then record slots
-            unsigned am = __activemask();
-            int leader = __ffs(am) - 1;
-            if ((int)lane_id() == leader) atomicAdd(&pv.gcount[1], __popc(am));
-            unsigned hsh = murmur3_finalize((unsigned)id * 0x9E3779B9u ^ (unsigned)(depth + 1) * 0x85EBCA6Bu);
-            if (hsh < pv.gkeep) {
-                unsigned km = __activemask();
-                int kl = __ffs(km) - 1, rb = 0;
-                if ((int)lane_id() == kl) rb = atomicAdd(&pv.gcount[0], __popc(km));
-                int r = __shfl_sync(km, rb, kl) + __popc(km & lanemask_lt());
-                if (r < pv.gcap) {
-                    GuideRec g;
-                    g.p[0] = (p.x - pv.glo[0]) * pv.gscale[0];
-                    g.p[1] = (p.y - pv.glo[1]) * pv.gscale[1];
-                    g.p[2] = (p.z - pv.glo[2]) * pv.gscale[2];
-                    g.n[0] = n.x; g.n[1] = n.y; g.n[2] = n.z;
-                    g.wo[0] = wo.x; g.wo[1] = wo.y; g.wo[2] = wo.z;
-                    g.wi[0] = wi.x; g.wi[1] = wi.y; g.wi[2] = wi.z;
-                    g.pdf = gpdf;
-                    g.L[0] = g.L[1] = g.L[2] = 0.0f;
-                    pv.grec[r] = g;
-                    int4 sl = pv.gslot[id];
-                    pv.gslot[id] = make_int4(r, sl.x, sl.y, -1);
-                    pv.ginv[3 * id + 2] = pv.ginv[3 * id + 1];
-                    pv.ginv[3 * id + 1] = pv.ginv[3 * id];
-                    pv.ginv[3 * id] = make_float4(T.r > 0.0f ? 1.0f / T.r : 0.0f, T.g > 0.0f ? 1.0f / T.g : 0.0f,
-                                                  T.b > 0.0f ? 1.0f / T.b : 0.0f, 0.0f);
-                    pushed = 1;
-                }
+    }
+    if (out.cont && depth >= 3) {
+        float rr = smin(smax3(T.r, T.g, T.b), 0.95f);
+        if (randf(ps.rng) > rr) out.cont = false;
+        else T = T * (1.0f / rr);
+    }
+    if (!rgb_valid(T)) out.cont = false;
+    int pushed = 0;
+    if (GUIDE && guided && out.cont) {
+        // warp-aggregated counters: guided vertices, then record slots
+        unsigned am = __activemask();
+        int leader = __ffs(am) - 1;
+        if ((int)lane_id() == leader) atomicAdd(&pv.gcount[1], __popc(am));
+        unsigned hsh = murmur3_finalize((unsigned)id * 0x9E3779B9u ^ (unsigned)(depth + 1) * 0x85EBCA6Bu);
+        if (hsh < pv.gkeep) {
+            unsigned km = __activemask();
+            int kl = __ffs(km) - 1, rb = 0;
+            if ((int)lane_id() == kl) rb = atomicAdd(&pv.gcount[0], __popc(km));
+            int r = __shfl_sync(km, rb, kl) + __popc(km & lanemask_lt());
+            if (r < pv.gcap) {
+                GuideRec g;
+                g.p[0] = (p.x - pv.glo[0]) * pv.gscale[0];
+                g.p[1] = (p.y - pv.glo[1]) * pv.gscale[1];
+                g.p[2] = (p.z - pv.glo[2]) * pv.gscale[2];
+                g.n[0] = n.x; g.n[1] = n.y; g.n[2] = n.z;
+                g.wo[0] = wo.x; g.wo[1] = wo.y; g.wo[2] = wo.z;
+                g.wi[0] = wi.x; g.wi[1] = wi.y; g.wi[2] = wi.z;
+                g.pdf = gpdf;
+                g.L[0] = g.L[1] = g.L[2] = 0.0f;
+                pv.grec[r] = g;
+                int4 sl = pv.gslot[id];
+                pv.gslot[id] = make_int4(r, sl.x, sl.y, -1);
+                pv.ginv[3 * id + 2] = pv.ginv[3 * id + 1];
+                pv.ginv[3 * id + 1] = pv.ginv[3 * id];
+                pv.ginv[3 * id] = make_float4(T.r > 0.0f ? 1.0f / T.r : 0.0f, T.g > 0.0f ? 1.0f / T.g : 0.0f,
+                                              T.b > 0.0f ? 1.0f / T.b : 0.0f, 0.0f);
+                pushed = 1;
             }
         }
-    } while (0);
-
-    if (out.cont && depth + 1 >= f.max_depth) out.cont = false;
-    pv.rng[id] = make_ulonglong2(rng.state, rng.inc);
-    pv.rad[id] = make_float4(result.r, result.g, result.b, 0.0f);
-    if (out.cont) {
-        pv.thr[id] = make_float4(T.r, T.g, T.b, last_pdf);
-        pv.ray_o[id] = make_float4(new_o.x, new_o.y, new_o.z, RAY_T_MIN);
-        pv.ray_d[id] = make_float4(new_d.x, new_d.y, new_d.z, __int_as_float(depth + 1));
     }
-    if (out.shadow) {
-        pv.sh_o[id] = make_float4(sh_o.x, sh_o.y, sh_o.z, sh_len);
-        // w: the first guide slot the NEE contribution credits (a vertex's
-        // own light sample did not arrive along its sampled direction)
-        pv.sh_d[id] = make_float4(sh_d.x, sh_d.y, sh_d.z, __int_as_float(pushed));
-        pv.sh_c[id] = make_float4(sh_inc.r, sh_inc.g, sh_inc.b, 0.0f);
+    sr.pushed = pushed;
+    if (depth + 1 >= max_depth) out.cont = false;
+    if (out.cont) {
+        ps.T = T;
+        ps.last_pdf = last_pdf;
+        ps.o = p;
+        ps.d = wi;
+        ps.depth = depth + 1;
     }
     return out;
 }
 
-// Eight resident CTAs per SM (at most 64 registers per thread, a few
-// hundred bytes of spills): the extra warps hide more of the shading
-// kernel's instruction-fetch and memory latency than the spills cost
-// (measured on the 1M-triangle scene: 4, 5, 6, 7, 8 CTAs per SM).
+// The same on the wavefront's path state: reads path `id` (-1: the lane has
+// none), shades it, writes back what changed.
+template <int ALGO, bool GUIDE>
+LD ShadeResult shade_path(const DevScene& sc, const FrameParams& f, const PathView& pv, int id) {
+    const bool live = id >= 0;
+    PathRegs ps;
+    ps.o = ps.d = v3(0.f, 0.f, 1.f);
+    ps.T = rgb(0.f, 0.f, 0.f);
+    ps.last_pdf = 0.0f;
+    ps.depth = 0;
+    ps.rng.state = ps.rng.inc = 0;
+    float4 hh = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+    float2 lh = make_float2(__int_as_float(-1), 0.f);
+    if (live) {
+        ps.o = f3(pv.ray_o[id]);
+        const float4 rd = pv.ray_d[id];
+        ps.d = f3(rd);
+        ps.depth = __float_as_int(rd.w);
+        const float4 th = pv.thr[id];
+        ps.T = c3(th);
+        ps.last_pdf = th.w;
+        const ulonglong2 rs = pv.rng[id];
+        ps.rng.state = rs.x;
+        ps.rng.inc = rs.y;
+        hh = pv.hit[id];
+        lh = pv.lhit[id];
+    }
+    ShadowRay sr;
+    const ShadeResult out =
+        shade_segment<ALGO, GUIDE>(sc, live, f.max_depth, f.records != 0, pv, id, ps, hh, lh, sr, BlockSync());
+    if (out.add.r != 0.0f || out.add.g != 0.0f || out.add.b != 0.0f) {
+        const float4 ra = pv.rad[id];
+        pv.rad[id] = make_float4(ra.x + out.add.r, ra.y + out.add.g, ra.z + out.add.b, 0.0f);
+    }
+    if (out.cont) {
+        pv.rng[id] = make_ulonglong2(ps.rng.state, ps.rng.inc);
+        pv.thr[id] = make_float4(ps.T.r, ps.T.g, ps.T.b, ps.last_pdf);
+        pv.ray_o[id] = make_float4(ps.o.x, ps.o.y, ps.o.z, RAY_T_MIN);
+        pv.ray_d[id] = make_float4(ps.d.x, ps.d.y, ps.d.z, __int_as_float(ps.depth));
+    }
+    if (out.shadow) {
+        pv.sh_o[id] = make_float4(sr.o.x, sr.o.y, sr.o.z, sr.len);
+        pv.sh_d[id] = make_float4(sr.d.x, sr.d.y, sr.d.z, __int_as_float(sr.pushed));
+        pv.sh_c[id] = make_float4(sr.inc.r, sr.inc.g, sr.inc.b, 0.0f);
+    }
+    return out;
+}
+
+// A block takes 256 queue entries at a time and its eight warps go through
+// shade_segment's phases together.  What bounds the kernel is instruction
+// fetch (a segment runs some 2,800 warp instructions of straight-line code);
+// in phase, eight warps share each fetched line.  The bench frame (1M
+// triangles, 1080p, 64 spp, volume_mis, 265 M segments) shades in 43.1 ms,
+// against 61.3 ms with warps fetching on their own and each event's code
+// written out; 128 threads 45.5, 512 42.1, 1,024 46.7 ms.  Small waves lose
+// from 512 threads on (an 800x600 1-spp frame: 307, 310, 327, 377 us for
+// 128, 256, 512, 1,024; 403 us before), so every wave takes 256.
+// MINB is the register cap: 128 * MINB threads per SM (8: 64 registers).
+constexpr int kShadeThreads = 256;
 template <int ALGO, bool GUIDE = false, int MINB = 8, bool MULTI = false>
-__global__ void __launch_bounds__(128, MINB) k_shade(DevScene sc, FrameParams f, PathView pv, int* cnt, int* cnt_next,
-                                                  int identity, int* qin, int* qout) {
+__global__ void __launch_bounds__(kShadeThreads, MINB / 2) k_shade(DevScene sc, FrameParams f, PathView pv, int* cnt,
+                                                         int* cnt_next, int identity, int* qin, int* qout) {
+    __shared__ int s_base[2];
     const int n = *(volatile int*)&cnt[0];
-    for (;;) {
-        int base = warp_fetch(&cnt[3]);
+    for (int it = 0;; it ^= 1) {
+        if (threadIdx.x == 0) s_base[it] = atomicAdd(&cnt[3], (int)blockDim.x);
+        __syncthreads();
+        const int base = s_base[it];
         if (base >= n) break;
-        int i = base + (int)lane_id();
-        int id = -1;
-        ShadeResult r;
-        r.cont = false;
-        r.shadow = false;
-        if (i < n) {
-            id = identity ? i : qin[i];
-            r = shade_path<ALGO, GUIDE>(path_scene<MULTI>(sc, pv, id), f, pv, id);
-        }
+        const int i = base + (int)threadIdx.x;
+        const int id = i < n ? (identity ? i : qin[i]) : -1;
+        const ShadeResult r = shade_path<ALGO, GUIDE>(path_scene<MULTI>(sc, pv, id), f, pv, id);
         warp_append(qout, &cnt_next[0], id, r.cont);
         warp_append(pv.qs, &cnt[1], id, r.shadow);
     }
@@ -1582,11 +1641,11 @@ __global__ void __launch_bounds__(128) k_diag_paths(DevScene sc, FrameParams f, 
                                        (sc.num_bnd_tris &&
                                         list_any(sc.bnd_tris, sc.num_bnd_tris, p, ls.dir, RAY_T_MIN, ls.dist));
                             if (!occ) {
-                                RGB fb = eval_bsdf(m, wo, ls.dir, sn);
+                                float pb;
+                                RGB fb = eval_bsdf<true>(m, wo, ls.dir, sn, nl, pb);
                                 float pl = ls.pdf * lsp;
                                 RGB nr;
                                 if (mis) {
-                                    float pb = pdf_bsdf(m, wo, ls.dir, sn);
                                     float mw = mis_power(pl, pb);
                                     nr = mul(bsdf_weight(fb, nl, pl) * mw, ls.emission);
                                 } else {
@@ -3206,7 +3265,7 @@ int Engine::render_impl(const LucidRenderParams& p, float* out_host, LucidSample
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t0, k_trace_primary_t<false>, 128, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t, k_trace, 128, 0);
     const ShadeKernel shade = ks.shade;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, shade, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, shade, kShadeThreads, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_h, k_shadow, 128, 0);
     const int g_trace0 = num_sms_ * std::max(1, occ_t0);
     const int g_trace = num_sms_ * std::max(1, occ_t), g_shade = num_sms_ * std::max(1, occ_s),
@@ -3299,7 +3358,7 @@ int Engine::render_impl(const LucidRenderParams& p, float* out_host, LucidSample
             k_bin_scatter<<<g_bin, 256, 0, st>>>(pv, cnt, depth == 0, qin, P.qb.p);
             ev_end(e);
             e = ev_begin(K_SHADE, depth);
-            shade<<<g_shade, 128, 0, st>>>(ds_->view, f, pv, cnt, cnt_next, 0, P.qb.p, qout);
+            shade<<<g_shade, kShadeThreads, 0, st>>>(ds_->view, f, pv, cnt, cnt_next, 0, P.qb.p, qout);
             ev_end(e);
             e = ev_begin(K_SHADOW, depth);
             k_shadow<<<g_shadow, 128, 0, st>>>(ds_->view, pv, cnt, f.records);
@@ -3525,7 +3584,7 @@ int Engine::render_batch(const BatchItem* items, int n, const char* algorithm, l
     int occ_t0 = 1, occ_t = 1, occ_s = 1, occ_h = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t0, k_trace_primary_batch, 128, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t, ks.trace, 128, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, ks.shade, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, ks.shade, kShadeThreads, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_h, ks.shadow, 128, 0);
     const int g_trace0 = num_sms_ * std::max(1, occ_t0), g_trace = num_sms_ * std::max(1, occ_t),
               g_shade = num_sms_ * std::max(1, occ_s), g_shadow = num_sms_ * std::max(1, occ_h);
@@ -3592,7 +3651,7 @@ int Engine::render_batch(const BatchItem* items, int n, const char* algorithm, l
             else
                 ks.trace<<<g_trace, 128, 0, st>>>(scene_tab[0], pv, cnt, 0, 0, bins);
             k_bin_scatter<<<g_bin, 256, 0, st>>>(pv, cnt, dd == 0, qin, P.qb.p);
-            ks.shade<<<g_shade, 128, 0, st>>>(scene_tab[0], fshade, pv, cnt, cnt_next, 0, P.qb.p, qout);
+            ks.shade<<<g_shade, kShadeThreads, 0, st>>>(scene_tab[0], fshade, pv, cnt, cnt_next, 0, P.qb.p, qout);
             ks.shadow<<<g_shadow, 128, 0, st>>>(scene_tab[0], pv, cnt, 0);
         }
         for (const PieceFilm& pf : films) {
@@ -3751,7 +3810,7 @@ void Engine::enqueue_iteration(void* fp, int n) {
         if (depth == 0) k_trace_primary_for(ds_->view, f.pos)<<<J.g_trace0, 128, 0, st>>>(ds_->view, f, pv, cnt, 0, bins);
         else k_trace<<<J.g_trace, 128, 0, st>>>(ds_->view, pv, cnt, 0, 0, bins);
         k_bin_scatter<<<J.g_bin, 256, 0, st>>>(pv, cnt, depth == 0, qin, P.qb.p);
-        shade<<<J.g_shade, 128, 0, st>>>(ds_->view, f, pv, cnt, cnt_next, 0, P.qb.p, qout);
+        shade<<<J.g_shade, kShadeThreads, 0, st>>>(ds_->view, f, pv, cnt, cnt_next, 0, P.qb.p, qout);
         k_shadow<<<J.g_shadow, 128, 0, st>>>(ds_->view, pv, cnt, 0);
     }
     k_film<<<(f.npix + 255) / 256, 256, 0, st>>>(f.npix, n, P.rad.p, P.film.p);
@@ -3827,7 +3886,7 @@ void Engine::job_grids_locked() {
     int occ_t = 1, occ_s = 1, occ_h = 1, occ_t0 = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t0, k_trace_primary_t<false>, 128, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t, ks.trace, 128, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, ks.shade, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, ks.shade, kShadeThreads, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_h, ks.shadow, 128, 0);
     J.g_trace0 = num_sms_ * std::max(1, occ_t0);
     J.g_trace = num_sms_ * std::max(1, occ_t);
@@ -4210,7 +4269,7 @@ int Engine::render_noalloc(const LucidRenderParams& p, float* d_out) {
             int occ[4] = {1, 1, 1, 1};
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[0], k_trace_primary_t<false>, 128, 0);
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[1], k_trace_lb<9>, 128, 0);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[2], shade, 128, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[2], shade, kShadeThreads, 0);
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[3], k_shadow_lb<9>, 128, 0);
             for (int k = 0; k < 4; ++k) g[k] = num_sms_ * std::max(1, occ[k]);
         }
@@ -4264,7 +4323,7 @@ int Engine::render_noalloc(const LucidRenderParams& p, float* d_out) {
             pv.q0 = qin;
             if (depth == 0) k_trace_primary_for(ds_->view, f.pos)<<<g_trace0, 128, 0, st>>>(ds_->view, f, pv, cnt, 0, -1);
             else k_trace_lb<9><<<g_trace, 128, 0, st>>>(ds_->view, pv, cnt, 0, 0, -1);
-            shade<<<g_shade, 128, 0, st>>>(ds_->view, f, pv, cnt, cnt_next, depth == 0, qin, qout);
+            shade<<<g_shade, kShadeThreads, 0, st>>>(ds_->view, f, pv, cnt, cnt_next, depth == 0, qin, qout);
             k_shadow_lb<9><<<g_shadow, 128, 0, st>>>(ds_->view, pv, cnt, 0);
         }
         k_film<<<(f.npix + 255) / 256, 256, 0, st>>>(f.npix, this_spw, v.rad, film);
