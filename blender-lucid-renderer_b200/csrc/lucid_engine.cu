@@ -24,6 +24,7 @@
 #include <condition_variable>
 #include <future>
 #include <cub/cub.cuh>
+#include <array>
 #include <map>
 #include <mutex>
 #include <thread>
@@ -122,7 +123,7 @@ struct PathView {
     unsigned short* cls;  // shading bin of each queue entry's pending event
     int* counters;     // per depth: [0] active, [1] shadow, [2..4] fetch cursors,
                        // [8, 8 + kBins) bin counts, then kBins bin cursors
-    int* errors;       // [0] traversal stack overflow
+    int* errors;       // [0] traversal stack overflow, from [4] on k_paths' PathsCount
     int2* rec_prim;
     int4* rec_cnt;     // bounces, nee tests, nee occluded
     unsigned long long* rec_hash;
@@ -150,6 +151,7 @@ constexpr int kCells = 1 << (3 * kCellBits);
 constexpr int kBins = kClassBins * kCells;
 constexpr int kCountersPerDepth = 8 + 2 * kBins;
 constexpr int kMaxDepth = 1024;
+constexpr int kErrorInts = 16;   // PathView::errors
 
 struct PathPool {
     long long cap = 0;
@@ -580,13 +582,14 @@ LD const DevScene& path_scene(const DevScene& sc, const PathView& pv, int id) {
 // hide node-fetch latency than the unconstrained 61 registers allow
 // (1M-triangle scene: 8 CTAs 232 ms, 9 CTAs 221 ms, 10 CTAs 225 ms).
 template <int MINB, bool MULTI = false>
-__global__ void __launch_bounds__(128, MINB) k_trace_lb(DevScene sc0, PathView pv, int* cnt, int identity, int records,
+__global__ void __launch_bounds__(128, MINB) k_trace_lb(DevScene sc0, PathView pv, int* cnt, int stop, int records,
                                                       int bins) {
     __shared__ int hist[kBins];
+    const int n = *(volatile int*)&cnt[0];
+    if (n <= stop) return;   // left to k_paths (see WavePlan)
     BinHist bh{hist};
     bh.clear(bins);
-    const int n = *(volatile int*)&cnt[0];
-    const int* q = identity ? nullptr : pv.q0;
+    const int* q = pv.q0;
     int stack[kStack];
     float stack_t[kStack];
     Trav s;
@@ -603,7 +606,7 @@ __global__ void __launch_bounds__(128, MINB) k_trace_lb(DevScene sc0, PathView p
         int r = refill(&cnt[2], n, !active, exhausted);
         if (r >= 0) {
             at = r;
-            const int id = q ? q[r] : r;
+            const int id = q[r];
             if constexpr (MULTI) sid = pv.sid[id];
             const DevScene& sc = scene();
             float4 ro = pv.st[id].ray_o, rd = pv.st[id].ray_d;
@@ -643,7 +646,7 @@ __global__ void __launch_bounds__(128, MINB) k_trace_lb(DevScene sc0, PathView p
         // a native light counts only in front of the surface hit (the shading
         // kernel's `lh.y < hh.x`): lights beyond it are not tested
         int li = (depth == 0) ? -1 : native_lights_closest(sc, s.o, s.d, res.t, lt);
-        const int id = q ? q[at] : at;
+        const int id = q[at];
         pv.hit[id].hit = make_float4(res.t, res.u, res.v, __int_as_float(res.prim));
         pv.hit[id].light = make_float4(__int_as_float(li), lt, 0.f, 0.f);
         bh.add(sc, pv, at, bins, res.prim, res.t, li, lt, s.o, s.d);
@@ -1107,9 +1110,11 @@ LD ShadeResult shade_path(const DevScene& sc, const FrameParams& f, const PathVi
 constexpr int kShadeThreads = 256;
 template <int ALGO, bool GUIDE = false, int MINB = 8, bool MULTI = false>
 __global__ void __launch_bounds__(kShadeThreads, MINB / 2) k_shade(DevScene sc, FrameParams f, PathView pv, int* cnt,
-                                                         int* cnt_next, int identity, int* qin, int* qout) {
+                                                         int* cnt_next, int identity, int stop, const int* qin,
+                                                         int* qout) {
     __shared__ int s_base[2];
     const int n = *(volatile int*)&cnt[0];
+    if (n <= stop) return;
     for (int it = 0;; it ^= 1) {
         if (threadIdx.x == 0) s_base[it] = atomicAdd(&cnt[3], (int)blockDim.x);
         __syncthreads();
@@ -1123,7 +1128,7 @@ __global__ void __launch_bounds__(kShadeThreads, MINB / 2) k_shade(DevScene sc, 
     }
 }
 
-using ShadeKernel = void (*)(DevScene, FrameParams, PathView, int*, int*, int, int*, int*);
+using ShadeKernel = void (*)(DevScene, FrameParams, PathView, int*, int*, int, int, const int*, int*);
 template <int MINB>
 static ShadeKernel shade_kernel_lb(int algo, bool guide) {
     if (guide && algo == ALGO_MIS) return k_shade<ALGO_MIS, true, MINB>;
@@ -1135,7 +1140,6 @@ static ShadeKernel shade_kernel_lb(int algo, bool guide) {
         default: return k_shade<ALGO_NEE, false, MINB>;
     }
 }
-static ShadeKernel shade_kernel(int algo, bool guide = false) { return shade_kernel_lb<8>(algo, guide); }
 // Batch waves (unguided): each path shaded in its own job's scene.
 static ShadeKernel shade_kernel_batch(int algo) {
     switch (algo) {
@@ -1153,10 +1157,12 @@ static ShadeKernel shade_kernel_batch(int algo) {
 // together so neighbouring warps shade the same kind of event.
 constexpr int kBinThreads = 256;
 static_assert(kBins % kBinThreads == 0, "bins per scatter thread");
-__global__ void __launch_bounds__(kBinThreads) k_bin_scatter(PathView pv, int* cnt, int identity, const int* qin,
-                                                             int* qb) {
+__global__ void __launch_bounds__(kBinThreads) k_bin_scatter(PathView pv, int* cnt, int identity, int stop,
+                                                             const int* qin, int* qb) {
     __shared__ int base[kBins];
     __shared__ int wsum[kBinThreads / 32];
+    const int n = *(volatile int*)&cnt[0];
+    if (n <= stop) return;
     {
         // exclusive prefix sum of the bin counts: kPer bins per thread, then a
         // block scan of the per-thread sums
@@ -1180,7 +1186,6 @@ __global__ void __launch_bounds__(kBinThreads) k_bin_scatter(PathView pv, int* c
         for (int j = 0; j < kPer; ++j) base[threadIdx.x * kPer + j] = excl + loc[j];
     }
     __syncthreads();
-    const int n = *(volatile int*)&cnt[0];
     // whole warps iterate together (match/shuffle below need every lane)
     for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
         int i = i0 + (int)threadIdx.x;
@@ -1278,6 +1283,7 @@ __global__ void __launch_bounds__(32 * kInferWarps, 1) k_guide_infer(DevScene sc
 template <int MINB, bool MULTI = false>
 __global__ void __launch_bounds__(128, MINB) k_shadow_lb(DevScene sc0, PathView pv, int* cnt, int records) {
     const int n = *(volatile int*)&cnt[1];
+    if (n == 0) return;
     int stack[kStack];
     Trav s;
     bool active = false, exhausted = false, ok = true;
@@ -1362,6 +1368,204 @@ __global__ void __launch_bounds__(128, MINB) k_shadow_lb(DevScene sc0, PathView 
     if (!ok) atomicAdd(&pv.errors[0], 1);
 }
 
+// ---------------------------------------------------------------- whole paths
+// A lane follows one path to its end with all its state in registers, then
+// takes the next: the camera paths of a small wave (depths 0; slots as in
+// k_trace_primary_t, or k_trace_primary_batch's in a batch wave), or the
+// paths at which the wavefront stopped (see WavePlan).  Every query and
+// float operation is the wavefront kernels' own, in a path's own order, so
+// the image does not depend on which of them ran.
+//
+// What bounds it is the latency of one warp's dependent instructions (a few
+// warps per scheduler, each waiting for its slowest lane), not throughput:
+// 128 registers and four resident blocks per SM, 96x64 1 spp in 204 us of
+// device time against 580 us for the wavefront's 34 launches (80 registers
+// 215 us, 64 registers 215 us; 16, 8, 4 lanes per warp 214, 206, 231 us).
+struct PathsCount {
+    int cursor;
+    int pad[3];
+    unsigned long long segments, shadows;
+};
+
+template <int ALGO, bool MULTI>
+__global__ void __launch_bounds__(128, 4) k_paths(DevScene sc0, FrameParams f0, PathView pv, const BatchJob* jobs,
+                                                   int njobs, int slots, int fma0, int depths, int stop,
+                                                   PathsCount* cnt) {
+    __shared__ int sbase[MULTI ? kMaxBatchPieces : 1];
+    if constexpr (MULTI) {
+        for (int i = threadIdx.x; i < njobs; i += blockDim.x) sbase[i] = jobs[i].slot_base;
+        __syncthreads();
+    }
+    const int* q = nullptr;
+    if (depths > 0) {
+        // the depth at which the wavefront left its paths
+        int d = 1;
+        for (;; ++d) {
+            slots = *(volatile const int*)&pv.counters[kCountersPerDepth * d];
+            if (slots <= stop || d == depths) break;
+        }
+        if (slots == 0) return;
+        q = (d & 1) ? pv.q1 : pv.q0;
+    }
+    int stack[kStack];
+    float stack_t[kStack];
+    Trav s;
+    bool active = false, exhausted = false, ok = true;
+    int id = 0, sid = 0;
+    unsigned nseg = 0, nsh = 0;
+    PathRegs ps;
+    RGB result = rgb(0.f, 0.f, 0.f);
+    auto scene = [&]() -> const DevScene& {
+        if constexpr (MULTI) return pv.scenes[sid];
+        else return sc0;
+    };
+    for (;;) {
+        const int slot0 = refill(&cnt->cursor, slots, !active, exhausted);
+        if (slot0 >= 0) {
+            if (q) {
+                id = q[slot0];
+                if constexpr (MULTI) sid = pv.sid[id];
+                const PathState& st = pv.st[id];
+                ps.o = f3(st.ray_o);
+                const float4 rd = st.ray_d, th = st.thr;
+                ps.d = f3(rd);
+                ps.depth = __float_as_int(rd.w);
+                ps.T = c3(th);
+                ps.last_pdf = th.w;
+                const ulonglong2 rs = st.rng;
+                ps.rng.state = rs.x;
+                ps.rng.inc = rs.y;
+                result = c3(pv.rad[id]);
+                active = true;
+            } else {
+                int slot = slot0, base = 0;
+                const FrameParams* f = &f0;
+                if constexpr (MULTI) {
+                    int lo = 0, hi = njobs - 1;   // the last piece whose slots start at or before the slot
+                    while (lo < hi) {
+                        const int mid = (lo + hi + 1) >> 1;
+                        if (sbase[mid] <= slot) lo = mid; else hi = mid - 1;
+                    }
+                    f = &jobs[lo].f;
+                    base = jobs[lo].path_base;
+                    sid = jobs[lo].sid;
+                    slot -= sbase[lo];
+                }
+                const int tw = f->tile_w, tiles_x = (tw + 7) / 8, per_sample = tiles_x * ((f->tile_h + 3) / 4) * 32;
+                const int sl = slot / per_sample, in = slot - sl * per_sample, tile = in >> 5;
+                const int px = (tile % tiles_x) * 8 + (in & 7), py = (tile / tiles_x) * 4 + ((in >> 3) & 3);
+                if (px < tw && py < f->tile_h) {
+                    const int local = sl * f->npix + py * tw + px;
+                    id = base + local;
+                    ps.d = camera_dir(*f, local, ps.rng);
+                    ps.o = v3(f->pos[0], f->pos[1], f->pos[2]);
+                    ps.T = rgb(1.0f, 1.0f, 1.0f);
+                    result = rgb(0.0f, 0.0f, 0.0f);
+                    ps.last_pdf = 0.0f;
+                    ps.depth = 0;
+                    if (!MULTI && f0.records) records_begin(pv, id);
+                    active = true;
+                }
+            }
+        }
+        if (__ballot_sync(0xffffffffu, active) == 0) {
+            if (__ballot_sync(0xffffffffu, !exhausted) == 0) break;
+            continue;
+        }
+        const DevScene& sc = scene();
+        HitRec h;
+        h.t = 1e30f; h.u = h.v = 0.0f; h.prim = -1;
+        float lt = 1e30f;
+        int li = -1;
+        const bool records = !MULTI && f0.records != 0;
+        if (active) {
+            // closest hit beyond the volume boundaries (k_trace_lb)
+            const float tmin = ps.depth == 0 ? 0.0f : RAY_T_MIN;
+            const bool fma = ps.depth != 0 || fma0;
+            float search = tmin;
+            trav_begin<false>(s, sc, ps.o, ps.d, tmin, 1e30f);
+            int peek = 0;
+            for (;;) {
+                while (!trav_run<false, true>(s, stack, stack_t, sc, ok, 64, fma)) {}
+                h = s.h;
+                if (!sc.num_bnd_tris) break;
+                bool restart = false;
+                for (;;) {
+                    HitRec b = s.h;
+                    if (b.prim < 0) b.t = 1e30f;
+                    boundary_closest<true>(sc, s.o, s.d, s.inv, search, b);
+                    if (b.prim < 0) { h.prim = -1; break; }
+                    if (b.prim == s.h.prim) break;
+                    search = b.t + 1e-3f;
+                    if (++peek == 8) { h.prim = -1; break; }
+                    if (s.h.prim >= 0 && s.h.t < search) {
+                        trav_begin<false>(s, sc, s.o, s.d, search, 1e30f);
+                        restart = true;
+                        break;
+                    }
+                }
+                if (!restart) break;
+            }
+            if (h.prim < 0) { h.t = 1e30f; h.u = 0.0f; h.v = 0.0f; }
+            li = ps.depth == 0 ? -1 : native_lights_closest(sc, ps.o, ps.d, h.t, lt);
+            ++nseg;
+            if (records) {
+                const int4 pi = h.prim >= 0 ? sc.prim_info[h.prim] : make_int4(-1, -1, -1, 0);
+                if (ps.depth == 0) pv.rec_prim[id] = make_int2(pi.x, pi.y);
+                pv.rec_cnt[id].x += 1;
+                unsigned long long hs = pv.rec_hash[id];
+                hs = hpush(hs, (uint32_t)pi.x);
+                hs = hpush(hs, (uint32_t)pi.y);
+                hs = hpush(hs, (uint32_t)li);
+                pv.rec_hash[id] = hs;
+            }
+        }
+        __syncwarp();
+        ShadowRay sr;
+        const ShadeResult r =
+            shade_segment<ALGO, false>(sc, active, f0.max_depth, records, pv, id, ps,
+                                       make_float4(h.t, h.u, h.v, __int_as_float(h.prim)),
+                                       make_float2(__int_as_float(li), lt), sr, NoSync());
+        result = result + r.add;
+        __syncwarp();
+        if (r.shadow) {
+            const bool occ = shadowed_skip_boundaries<true>(sc, sr.o, sr.d, sr.len, ok);
+            if (!occ) result = result + sr.inc;
+            ++nsh;
+            if (records) {
+                int4 rc = pv.rec_cnt[id];
+                rc.y += 1;
+                rc.z += occ ? 1 : 0;
+                pv.rec_cnt[id] = rc;
+                pv.rec_hash[id] = hpush(pv.rec_hash[id], 0x5EED0000u | (occ ? 1u : 0u));
+            }
+        }
+        if (active && !r.cont) {
+            pv.rad[id] = make_float4(result.r, result.g, result.b, 0.0f);
+            active = false;
+        }
+        __syncwarp();
+    }
+    nseg = __reduce_add_sync(0xffffffffu, nseg);
+    nsh = __reduce_add_sync(0xffffffffu, nsh);
+    if (lane_id() == 0 && nseg) {
+        atomicAdd(&cnt->segments, (unsigned long long)nseg);
+        atomicAdd(&cnt->shadows, (unsigned long long)nsh);
+    }
+    if (!ok) atomicAdd(&pv.errors[0], 1);
+}
+using PathsKernel = void (*)(DevScene, FrameParams, PathView, const BatchJob*, int, int, int, int, int, PathsCount*);
+template <bool MULTI>
+static PathsKernel paths_kernel(int algo) {
+    switch (algo) {
+        case ALGO_SIMPLE: return k_paths<ALGO_SIMPLE, MULTI>;
+        case ALGO_MIS: return k_paths<ALGO_MIS, MULTI>;
+        case ALGO_VOLUME_SIMPLE: return k_paths<ALGO_VOLUME_SIMPLE, MULTI>;
+        case ALGO_VOLUME_MIS: return k_paths<ALGO_VOLUME_MIS, MULTI>;
+        default: return k_paths<ALGO_NEE, MULTI>;
+    }
+}
+
 // ---------------------------------------------------------------- launch profiles
 // Resident CTAs per SM of the wavefront kernels (their register caps):
 // profile 0 is the measured optimum on the 1M-triangle scene (closest hit 9,
@@ -1432,6 +1636,22 @@ __global__ void k_output(int tw, int th, const float4* film, float4* out) {
     int x = p % tw, y = p / tw;
     float4 a = film[p];
     float r = a.x * 1.0f, g = a.y * 1.0f, b = a.z * 1.0f;
+    out[(size_t)(th - 1 - y) * tw + x] = make_float4(smax(r, 0.0f), smax(g, 0.0f), smax(b, 0.0f), 1.0f);
+}
+
+// Film sum and output in one pass, for a call whose samples are one wave.
+__global__ void __launch_bounds__(128) k_film_output(int tw, int th, int spw, const float4* rad, float4* out) {
+    const int npix = tw * th;
+    int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= npix) return;
+    int x = p % tw, y = p / tw;
+    float r = 0.0f, g = 0.0f, b = 0.0f;
+#pragma unroll 8
+    for (int s = 0; s < spw; ++s) {
+        const float4 v = rad[(size_t)s * npix + p];
+        r = r + v.x; g = g + v.y; b = b + v.z;
+    }
+    r = r * 1.0f; g = g * 1.0f; b = b * 1.0f;
     out[(size_t)(th - 1 - y) * tw + x] = make_float4(smax(r, 0.0f), smax(g, 0.0f), smax(b, 0.0f), 1.0f);
 }
 
@@ -2075,6 +2295,9 @@ Engine::~Engine() {
     ds_.reset();   // the device scene is freed with its last sharing engine
     if (pool_) { pool_->release(); delete pool_; }
     delete diag_dev_;
+    for (void* e : render_ev_)
+        if (e) cudaEventDestroy((cudaEvent_t)e);
+    if (host_counts_) cudaFreeHost(host_counts_);
     if (stream_) cudaStreamDestroy(S(stream_));
 }
 
@@ -2739,7 +2962,7 @@ int Engine::ensure_pool(long long paths, bool records) {
     CK(P.st.alloc(cap)); CK(P.hit.alloc(cap)); CK(P.sh.alloc(cap)); CK(P.rad.alloc(cap));
     CK(P.q0.alloc(cap)); CK(P.q1.alloc(cap)); CK(P.qb.alloc(cap)); CK(P.cls.alloc(cap));
     CK(P.counters.alloc((size_t)kCountersPerDepth * (kMaxDepth + 1)));
-    CK(P.errors.alloc(4));
+    CK(P.errors.alloc(kErrorInts));
     if (records) { CK(P.rec_prim.alloc(cap)); CK(P.rec_cnt.alloc(cap)); CK(P.rec_hash.alloc(cap)); }
     P.cap = cap;
     P.records = records;
@@ -2766,16 +2989,150 @@ namespace {
 //   film  : radiance 16 / path + film 32 / pixel
 //   bin   : queue id 4 + shading bin 2 + binned id 4 (scatter)       = 10 / path
 constexpr double kBytesTrace0 = 107, kBytesTrace = 63, kBytesShade = 340, kBytesShadow = 84, kBytesRaygen = 80, kBytesFilm = 16,
-                 kBytesBin = 10;
+                 kBytesBin = 10, kBytesPaths = 80;
+//   paths : prim info/normal 32 + material 48 per segment (the state stays in registers)
 //   guide : queue 4 + hit 24 + ray 32 + raw outputs 160 w              = 220 / path
 //   train : one record 64 / record (weights are read from shared memory)
-enum Kind { K_RAYGEN, K_TRACE0, K_TRACE, K_SHADE, K_SHADOW, K_FILM, K_BIN, K_GUIDE, K_TRAIN, K_NUM };
+enum Kind { K_RAYGEN, K_TRACE0, K_TRACE, K_SHADE, K_SHADOW, K_FILM, K_BIN, K_GUIDE, K_TRAIN, K_PATHS, K_NUM };
 const char* kKindNames[K_NUM] = {"k_raygen", "k_trace_primary", "k_trace", "k_shade", "k_shadow", "k_film", "k_bin",
-                                 "k_guide_infer", "k_guide_train"};
+                                 "k_guide_infer", "k_guide_train", "k_paths"};
 const double kKindBytes[K_NUM] = {kBytesRaygen, kBytesTrace0, kBytesTrace, kBytesShade, kBytesShadow, kBytesFilm,
-                                  kBytesBin, 220, 64};
+                                  kBytesBin, 220, 64, kBytesPaths};
 static_assert(K_NUM <= LUCID_MAX_KERNEL_KINDS, "kernel kinds");
 }  // namespace
+
+// ---------------------------------------------------------------- waves
+// One wave: the wavefront kernels of `depths` depths (camera rays, then per
+// depth trace, bin, shade, shadow), then k_paths for what is left of the
+// paths.  A depth > 0 whose queue holds at most `stop` paths leaves them to
+// k_paths at once: the remaining launches of the wave return on reading the
+// queue length.  depths 0: every path runs in k_paths from its camera ray.
+// stop < 0: no k_paths (guided renders; a single depth).
+//
+// Four launches of a depth take 65-80 us however few paths are queued (each
+// waits for its slowest ray), so small queues are better followed to the end
+// by one kernel.  The line is 2^17 paths, two thirds of what k_paths keeps
+// resident: a 26k- and a 77k-path wave of the all-lights scene take 582 us
+// in k_paths and 798 us with the wavefront first; the 480k paths of an
+// 800x600 frame 887 us in k_paths alone against 787 us; of `stop` = 2^15,
+// 2^16, 2^17, 2^18, 2^19 the volume frame (333x207, 5 spp, depth 16) takes
+// 1.05, 1.06, 1.06, 1.40, 1.39 ms and the 1M-triangle frame (960x540, 4 spp,
+// depth 16) 5.34, 5.08, 5.12, 5.08, 5.36 ms (2.09 and 7.3 ms with every
+// depth launched).  `depths` bounds the launches of a wave whose queue
+// shrinks as usual (two depths, and one more for each doubling from 2^19
+// paths on); where it shrinks more slowly k_paths takes a longer queue.
+constexpr long long kPathsWave = 1LL << 17;
+struct WavePlan {
+    LaunchSet ks;
+    PathsKernel paths;
+    int g_trace0 = 1, g_trace = 1, g_shade = 1, g_shadow = 1, g_bin = 1, g_paths = 1;   // blocks
+    int depths = 0, stop = -1;
+    int bins = -1;   // shading bins (BinHist); -1: the queues are shaded as they are
+};
+static WavePlan wave_plan(int device, int sms, int algo, bool guide, int profile, bool batch, bool binned,
+                          long long paths, int max_depth) {
+    WavePlan w;
+    w.ks = batch ? launch_set_batch(algo) : launch_set(algo, guide, profile);
+    w.paths = batch ? paths_kernel<true>(algo) : paths_kernel<false>(algo);
+    // the kernels' resident blocks per SM, queried once per device and set
+    static std::mutex mu;
+    static std::map<int, std::array<int, 5>>* occ = new std::map<int, std::array<int, 5>>();
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        std::array<int, 5>& o = (*occ)[((device * 8 + algo) * 2 + (guide ? 1 : 0)) * 4 + profile * 2 + (batch ? 1 : 0)];
+        if (o[0] == 0) {
+            auto query = [&](auto kernel, int threads) {
+                int n = 1;
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, 0);
+                return std::max(1, n);
+            };
+            o[1] = query(w.ks.trace, 128);
+            o[2] = query(w.ks.shade, kShadeThreads);
+            o[3] = query(w.ks.shadow, 128);
+            o[4] = query(w.paths, 128);
+            o[0] = batch ? query(k_trace_primary_batch, 128) : query(k_trace_primary_t<false>, 128);
+        }
+        w.g_trace0 = sms * o[0];
+        w.g_trace = sms * o[1];
+        w.g_shade = sms * o[2];
+        w.g_shadow = sms * o[3];
+        w.g_paths = sms * o[4];
+    }
+    w.g_bin = sms * 8;
+    if (binned)
+        w.bins = ((algo == ALGO_VOLUME_MIS || algo == ALGO_VOLUME_SIMPLE) ? kBinVolume : 0) |
+                 (paths >= kCellBinPaths ? kBinCells : 0);
+    w.depths = std::max(0, max_depth);
+    if (guide || max_depth < 1) return w;
+    if (paths <= kPathsWave) {
+        w.depths = 0;
+    } else {
+        int d = 2;
+        for (long long p = paths >> 19; p > 0; p >>= 1) ++d;
+        w.depths = std::min(max_depth, d);
+        if (max_depth > 1) w.stop = (int)kPathsWave;
+    }
+    return w;
+}
+
+// Launches one wave.  primary(pv, cnt): the camera-ray kernel; infer(depth,
+// pv, cnt, queue): guide inference before a depth's shading; mark(kind,
+// depth, launch): runs each launch (inside profiling events).
+template <class Primary, class Infer, class Mark>
+static void enqueue_wave(const WavePlan& w, const DevScene& sc, const FrameParams& f, const PathView& base, int* qb,
+                         int max_depth, cudaStream_t st, Primary primary, Infer infer, Mark mark,
+                         const BatchJob* jobs = nullptr, int njobs = 0, int slots = 0) {
+    PathsCount* pc = reinterpret_cast<PathsCount*>(base.errors + 4);
+    for (int depth = 0; depth < w.depths; ++depth) {
+        int* cnt = base.counters + kCountersPerDepth * depth;
+        int* cnt_next = base.counters + kCountersPerDepth * (depth + 1);
+        PathView pv = base;
+        // queue ping-pong: depth d reads q[d & 1] and writes q[(d + 1) & 1]
+        int* qin = (depth & 1) ? base.q1 : base.q0;
+        int* qout = (depth & 1) ? base.q0 : base.q1;
+        pv.q0 = qin;
+        const int stop = depth == 0 ? -1 : w.stop;
+        if (depth == 0)
+            mark(K_TRACE0, depth, [&] { primary(pv, cnt); });
+        else
+            mark(K_TRACE, depth, [&] { w.ks.trace<<<w.g_trace, 128, 0, st>>>(sc, pv, cnt, stop, f.records, w.bins); });
+        infer(depth, pv, cnt, qin);
+        int identity = depth == 0;
+        if (w.bins >= 0) {
+            mark(K_BIN, depth, [&] { k_bin_scatter<<<w.g_bin, kBinThreads, 0, st>>>(pv, cnt, identity, stop, qin, qb); });
+            identity = 0;
+        }
+        mark(K_SHADE, depth, [&] {
+            w.ks.shade<<<w.g_shade, kShadeThreads, 0, st>>>(sc, f, pv, cnt, cnt_next, identity, stop,
+                                                            w.bins >= 0 ? qb : qin, qout);
+        });
+        mark(K_SHADOW, depth, [&] { w.ks.shadow<<<w.g_shadow, 128, 0, st>>>(sc, pv, cnt, f.records); });
+    }
+    if (max_depth < 1 || (w.depths == max_depth && w.stop < 0)) return;
+    int grid = w.g_paths, fma0 = 0;
+    if (!jobs) {
+        const float m = std::max(std::fabs(f.pos[0]), std::max(std::fabs(f.pos[1]), std::fabs(f.pos[2])));
+        fma0 = m <= sc.coord_bound;
+        slots = ((f.tile_w + 7) / 8) * ((f.tile_h + 3) / 4) * 32 * (f.n_wave / std::max(f.npix, 1));
+    }
+    if (w.depths == 0) grid = std::min(grid, (slots + 127) / 128);
+    cudaMemsetAsync(pc, 0, sizeof(PathsCount), st);
+    mark(K_PATHS, w.depths, [&] {
+        w.paths<<<grid, 128, 0, st>>>(sc, f, base, jobs, njobs, slots, fma0, w.depths, w.stop, pc);
+    });
+}
+
+// Adds up the segments and shadow rays of a wave whose first eight counters
+// of each depth 0 .. depths are in `c` and whose k_paths totals are `pc`.
+static void wave_totals(const WavePlan& w, const int* c, const PathsCount& pc, double& seg, double& shadows) {
+    for (int d = 0; d < w.depths; ++d) {
+        if (d > 0 && c[8 * d] <= w.stop) break;
+        seg += c[8 * d];
+        shadows += c[8 * d + 1];
+    }
+    seg += (double)pc.segments;
+    shadows += (double)pc.shadows;
+}
 
 // Default paths per wave: large waves keep every depth's launches full and
 // amortise each persistent kernel's tail (measured on the 1M-triangle
@@ -2975,7 +3332,7 @@ int Engine::render_diag_impl(const LucidRenderParams& p, float* out_host, float*
     if ((long long)D.units.n < 8 * want) CK(D.units.alloc((size_t)(8 * want)));   // a few bounces per record
     if (!D.count.p) CK(D.count.alloc(2));
     CK(cudaMemsetAsync(P.film.p, 0, np * sizeof(float4), st));
-    CK(cudaMemsetAsync(P.errors.p, 0, 4 * sizeof(int), st));
+    CK(cudaMemsetAsync(P.errors.p, 0, kErrorInts * sizeof(int), st));
 
     FrameParams f{};
     for (int k = 0; k < 3; ++k) { f.pos[k] = cam_.pos[k]; f.fwd[k] = cam_.forward[k]; f.right[k] = cam_.right[k]; f.up[k] = cam_.up[k]; }
@@ -3101,8 +3458,6 @@ int Engine::render_diag_impl(const LucidRenderParams& p, float* out_host, float*
     CK(cudaStreamSynchronize(st));
     float tot = 0.0f;
     cudaEventElapsedTime(&tot, t0, t1);
-    cudaEventDestroy(t0);
-    cudaEventDestroy(t1);
     stats_.total_ms = tot;
     stats_.paths = (double)np * p.samples;
     stats_.waves = waves;
@@ -3259,8 +3614,8 @@ int Engine::render_impl(const LucidRenderParams& p, float* out_host, LucidSample
         CK(P.out.alloc(np));
         P.film_n = np;
     }
-    CK(cudaMemsetAsync(P.film.p, 0, np * sizeof(float4), st));
-    CK(cudaMemsetAsync(P.errors.p, 0, 4 * sizeof(int), st));
+    if (spw < p.samples || accumulate || guide) CK(cudaMemsetAsync(P.film.p, 0, np * sizeof(float4), st));
+    CK(cudaMemsetAsync(P.errors.p, 0, kErrorInts * sizeof(int), st));
     if (out_f64) {
         if (P.film64_n < np) {
             CK(P.film64.alloc(np * 3));
@@ -3282,20 +3637,7 @@ int Engine::render_impl(const LucidRenderParams& p, float* out_host, LucidSample
     f.npix = (int)np;
     f.records = records ? 1 : 0;
 
-    // persistent grids: a whole number of CTAs per SM
-    int occ_t = 1, occ_s = 1, occ_h = 1, occ_t0 = 1;
-    const LaunchSet ks = launch_set(algo_, guide, launch_profile_);
-    const TraceKernel k_trace = ks.trace;
-    const ShadowKernel k_shadow = ks.shadow;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t0, k_trace_primary_t<false>, 128, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t, k_trace, 128, 0);
-    const ShadeKernel shade = ks.shade;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, shade, kShadeThreads, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_h, k_shadow, 128, 0);
-    const int g_trace0 = num_sms_ * std::max(1, occ_t0);
-    const int g_trace = num_sms_ * std::max(1, occ_t), g_shade = num_sms_ * std::max(1, occ_s),
-              g_shadow = num_sms_ * std::max(1, occ_h);
-    const int g_bin = num_sms_ * 8;
+    const WavePlan w = wave_plan(device_, num_sms_, algo_, guide, launch_profile_, false, true, wave_paths, p.max_depth);
     PathView gv = P.view;   // the path view with the guide's buffers when guiding
     if (guide) {
         int rc2 = guide_buffers(wave_paths);
@@ -3315,11 +3657,6 @@ int Engine::render_impl(const LucidRenderParams& p, float* out_host, LucidSample
             attr = true;
         }
     }
-    // the shading queue is binned at every depth (the volume bit only for
-    // the integrators with media, the hit-point cells on large waves)
-    const int bins = ((algo_ == ALGO_VOLUME_MIS || algo_ == ALGO_VOLUME_SIMPLE) ? kBinVolume : 0) |
-                     (wave_paths >= kCellBinPaths ? kBinCells : 0);
-
     struct Launch { int kind; cudaEvent_t a, b; int depth; };
     std::vector<Launch> launches;
     auto ev_begin = [&](int kind, int depth) -> int {
@@ -3335,20 +3672,51 @@ int Engine::render_impl(const LucidRenderParams& p, float* out_host, LucidSample
 
     stats_ = LucidRenderStats{};
     double seg = 0, shadows = 0;
-    std::vector<int> hcnt((size_t)kCountersPerDepth * (p.max_depth + 1));
+    // pinned: the first eight counters of each depth, then the error words
+    if (!host_counts_) CK(cudaHostAlloc((void**)&host_counts_, sizeof(int) * (8 * (kMaxDepth + 1) + kErrorInts), cudaHostAllocDefault));
+    int* const hcnt = host_counts_;
+    int* const herr = hcnt + 8 * (kMaxDepth + 1);
+    const bool one_wave = spw >= p.samples;
     std::vector<double> kind_units(K_NUM, 0.0);
-    cudaEvent_t t0, t1;
-    cudaEventCreate(&t0);
-    cudaEventCreate(&t1);
+    if (!render_ev_[0]) { CK(cudaEventCreate((cudaEvent_t*)&render_ev_[0])); CK(cudaEventCreate((cudaEvent_t*)&render_ev_[1])); }
+    const cudaEvent_t t0 = (cudaEvent_t)render_ev_[0], t1 = (cudaEvent_t)render_ev_[1];
     cudaEventRecord(t0, st);
     int status = LUCID_OK;
     int waves = 0;
+    // a wave's counts, once its copies have arrived
+    auto add_totals = [&]() {
+        PathsCount pc;
+        std::memcpy(&pc, herr + 4, sizeof(pc));
+        if (w.depths >= p.max_depth && w.stop < 0) pc.segments = pc.shadows = 0;   // k_paths did not run
+        wave_totals(w, hcnt, pc, seg, shadows);
+        if (!profile) return;
+        kind_units[K_FILM] += f.n_wave;
+        for (int d = 0; d < w.depths; ++d) {
+            if (d > 0 && hcnt[8 * d] <= w.stop) break;
+            const double n = hcnt[8 * d];
+            kind_units[d == 0 ? K_TRACE0 : K_TRACE] += n;
+            kind_units[K_SHADE] += n;
+            kind_units[K_BIN] += n;
+            if (guide) kind_units[K_GUIDE] += n;
+            kind_units[K_SHADOW] += hcnt[8 * d + 1];
+        }
+        kind_units[K_PATHS] += (double)pc.segments;
+    };
+    auto fetch_counts = [&]() -> cudaError_t {
+        cudaError_t e = cudaSuccess;
+        if (w.depths > 0)
+            e = cudaMemcpy2DAsync(hcnt, 32, P.counters.p, sizeof(int) * kCountersPerDepth, 32, (size_t)w.depths,
+                                  cudaMemcpyDeviceToHost, st);
+        if (e != cudaSuccess) return e;
+        return cudaMemcpyAsync(herr, P.errors.p, kErrorInts * sizeof(int), cudaMemcpyDeviceToHost, st);
+    };
     for (int s0 = 0; s0 < p.samples; s0 += spw) {
         if (!from_async && is_cancelled()) { status = LUCID_ERR_CANCELLED; break; }
         int this_spw = std::min(spw, p.samples - s0);
         f.s0 = s0;
         f.n_wave = (int)((long long)this_spw * (long long)np);
-        CK(cudaMemsetAsync(P.counters.p, 0, sizeof(int) * kCountersPerDepth * (p.max_depth + 1), st));
+        if (p.max_depth < 1) CK(cudaMemsetAsync(P.rad.p, 0, (size_t)f.n_wave * sizeof(float4), st));   // no segment at all
+        if (w.depths > 0) CK(cudaMemsetAsync(P.counters.p, 0, sizeof(int) * kCountersPerDepth * (w.depths + 1), st));
         if (guide) {
             GuideState& G = *guide_;
             gv.gkeep = (unsigned)std::min(4294967295.0, (double)G.keep * 4294967296.0);
@@ -3356,48 +3724,32 @@ int Engine::render_impl(const LucidRenderParams& p, float* out_host, LucidSample
             CK(cudaMemsetAsync(G.count.p, 0, 2 * sizeof(int), st));
         }
         int e = 0;
-        for (int depth = 0; depth < p.max_depth; ++depth) {
-            int* cnt = P.counters.p + kCountersPerDepth * depth;
-            int* cnt_next = P.counters.p + kCountersPerDepth * (depth + 1);
-            PathView pv = gv;
-            // queue ping-pong: depth d reads q[d&1] and writes q[(d+1)&1]
-            int* qin = (depth & 1) ? P.q1.p : P.q0.p;
-            int* qout = (depth & 1) ? P.q0.p : P.q1.p;
-            pv.q0 = qin;
-            if (depth == 0) {
-                e = ev_begin(K_TRACE0, depth);
-                k_trace_primary_for(ds_->view, f.pos)<<<g_trace0, 128, 0, st>>>(ds_->view, f, pv, cnt, f.records, bins);
-            } else {
-                e = ev_begin(K_TRACE, depth);
-                k_trace<<<g_trace, 128, 0, st>>>(ds_->view, pv, cnt, 0, f.records, bins);
-            }
-            ev_end(e);
-            if (guide && depth < guide_->max_depth) {
-                e = ev_begin(K_GUIDE, depth);
-                k_guide_infer<<<num_sms_, 32 * kInferWarps, kInferSmem, st>>>(
-                    ds_->view, pv, cnt, depth == 0, qin, static_cast<const __nv_bfloat16*>(guide_->net.weights_bf16()),
-                    guide_->net.master());
-                ev_end(e);
-            }
-            e = ev_begin(K_BIN, depth);
-            k_bin_scatter<<<g_bin, 256, 0, st>>>(pv, cnt, depth == 0, qin, P.qb.p);
-            ev_end(e);
-            e = ev_begin(K_SHADE, depth);
-            shade<<<g_shade, kShadeThreads, 0, st>>>(ds_->view, f, pv, cnt, cnt_next, 0, P.qb.p, qout);
-            ev_end(e);
-            e = ev_begin(K_SHADOW, depth);
-            k_shadow<<<g_shadow, 128, 0, st>>>(ds_->view, pv, cnt, f.records);
-            ev_end(e);
-        }
+        enqueue_wave(w, ds_->view, f, gv, P.qb.p, p.max_depth, st, [&](const PathView& pv, int* cnt) {
+            k_trace_primary_for(ds_->view, f.pos)<<<w.g_trace0, 128, 0, st>>>(ds_->view, f, pv, cnt, f.records, w.bins);
+        }, [&](int depth, const PathView& pv, int* cnt, const int* qin) {
+            if (!guide || depth >= guide_->max_depth) return;
+            const int k = ev_begin(K_GUIDE, depth);
+            k_guide_infer<<<num_sms_, 32 * kInferWarps, kInferSmem, st>>>(
+                ds_->view, pv, cnt, depth == 0, qin, static_cast<const __nv_bfloat16*>(guide_->net.weights_bf16()),
+                guide_->net.master());
+            ev_end(k);
+        }, [&](int kind, int depth, auto&& launch) {
+            const int k = ev_begin(kind, depth);
+            launch();
+            ev_end(k);
+        });
+        if (records) k_records<<<(f.n_wave + 255) / 256, 256, 0, st>>>(f, P.view, d_recs.p);
+        ++waves;
+        if (one_wave && !out_f64 && !accumulate && !guide) break;   // summed straight into the output image below
         e = ev_begin(K_FILM, 0);
         if (out_f64)
             k_film_f64<<<(f.npix + 255) / 256, 256, 0, st>>>(f.npix, this_spw, P.rad.p, P.film64.p);
         else
             k_film<<<(f.npix + 255) / 256, 256, 0, st>>>(f.npix, this_spw, P.rad.p, P.film.p);
         ev_end(e);
-        if (records) k_records<<<(f.n_wave + 255) / 256, 256, 0, st>>>(f, P.view, d_recs.p);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(hcnt.data(), P.counters.p, hcnt.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
+        if (one_wave && !guide) break;   // the counts come with the image
+        CK(fetch_counts());
         int gcnt[2] = {0, 0};
         if (guide) CK(cudaMemcpyAsync(gcnt, guide_->count.p, sizeof(gcnt), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
@@ -3415,33 +3767,27 @@ int Engine::render_impl(const LucidRenderParams& p, float* out_host, LucidSample
             if (profile) kind_units[K_TRAIN] += nrec;
             G.keep = (float)std::min(1.0, 0.9 * G.steps * kGuideBatch / std::max(1.0, (double)gcnt[1]));
         }
-        for (int d = 0; d < p.max_depth; ++d) {
-            seg += hcnt[kCountersPerDepth * d];
-            shadows += hcnt[kCountersPerDepth * d + 1];
-        }
-        if (profile) {
-            kind_units[K_FILM] += f.n_wave;
-            for (int d = 0; d < p.max_depth; ++d) {
-                kind_units[d == 0 ? K_TRACE0 : K_TRACE] += hcnt[kCountersPerDepth * d];
-                kind_units[K_SHADE] += hcnt[kCountersPerDepth * d];
-                kind_units[K_BIN] += hcnt[kCountersPerDepth * d];
-                if (guide) kind_units[K_GUIDE] += hcnt[kCountersPerDepth * d];
-                kind_units[K_SHADOW] += hcnt[kCountersPerDepth * d + 1];
-            }
-        }
-        ++waves;
+        add_totals();
     }
-    int np_i = (int)np;
-    if (accumulate)
+    const int np_i = (int)np;
+    if (one_wave && waves == 0) CK(cudaMemsetAsync(P.film.p, 0, np * sizeof(float4), st));   // cancelled at once
+    if (accumulate) {
         k_accumulate<<<(np_i + 255) / 256, 256, 0, st>>>(np_i, P.film.p, (float4*)accumulate);
-    else if (out_f64)
+    } else if (out_f64) {
         k_output_f64<<<(np_i + 255) / 256, 256, 0, st>>>(p.tile_w, p.tile_h, P.film64.p, P.out64.p);
-    else
-        k_output<<<(np_i + 255) / 256, 256, 0, st>>>(p.tile_w, p.tile_h, P.film.p,
-                                                     out_device ? (float4*)out_device : P.out.p);
+    } else {
+        float4* const out = out_device ? (float4*)out_device : P.out.p;
+        if (one_wave && !guide && waves == 1) {
+            const int e = ev_begin(K_FILM, 0);
+            k_film_output<<<(np_i + 127) / 128, 128, 0, st>>>(p.tile_w, p.tile_h, p.samples, P.rad.p, out);
+            ev_end(e);
+        } else {
+            k_output<<<(np_i + 255) / 256, 256, 0, st>>>(p.tile_w, p.tile_h, P.film.p, out);
+        }
+    }
     cudaEventRecord(t1, st);
-    int herr[4] = {0, 0, 0, 0};
-    CK(cudaMemcpyAsync(herr, P.errors.p, sizeof(herr), cudaMemcpyDeviceToHost, st));
+    CK(cudaGetLastError());
+    CK(fetch_counts());
     if (out_host && !out_device)
         CK(cudaMemcpyAsync(out_host, P.out.p, np * sizeof(float4), cudaMemcpyDeviceToHost, st));
     if (out_f64)
@@ -3450,11 +3796,10 @@ int Engine::render_impl(const LucidRenderParams& p, float* out_host, LucidSample
         CK(cudaMemcpyAsync(recs, d_recs.p, np * (size_t)p.samples * sizeof(LucidSampleRecord), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     host_image.copied = true;
+    if (one_wave && !guide && waves == 1) add_totals();
     if (guide && guide_->net.failed(st) != 0) return fail(LUCID_ERR_TIMEOUT, guide_->net.error());
     float tot = 0.0f;
     cudaEventElapsedTime(&tot, t0, t1);
-    cudaEventDestroy(t0);
-    cudaEventDestroy(t1);
     stats_.total_ms = tot;
     stats_.paths = (double)np * p.samples;
     stats_.segments = seg;
@@ -3572,7 +3917,7 @@ int Engine::render_batch(const BatchItem* items, int n, const char* algorithm, l
         P.film_n = npix_all;
     }
     CK(cudaMemsetAsync(P.film.p, 0, npix_all * sizeof(float4), st));
-    CK(cudaMemsetAsync(P.errors.p, 0, 4 * sizeof(int), st));
+    CK(cudaMemsetAsync(P.errors.p, 0, kErrorInts * sizeof(int), st));
 
     // the scene table, then room for the largest wave's job table
     std::vector<DevScene> scene_tab(scenes.size());
@@ -3605,22 +3950,13 @@ int Engine::render_batch(const BatchItem* items, int n, const char* algorithm, l
         return f;
     };
 
-    const LaunchSet ks = launch_set_batch(algo);
-    int occ_t0 = 1, occ_t = 1, occ_s = 1, occ_h = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t0, k_trace_primary_batch, 128, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t, ks.trace, 128, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, ks.shade, kShadeThreads, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_h, ks.shadow, 128, 0);
-    const int g_trace0 = num_sms_ * std::max(1, occ_t0), g_trace = num_sms_ * std::max(1, occ_t),
-              g_shade = num_sms_ * std::max(1, occ_s), g_shadow = num_sms_ * std::max(1, occ_h);
-    const int g_bin = num_sms_ * 8;
     FrameParams fshade{};
     fshade.max_depth = depth;
     fshade.algo = algo;
 
     stats_ = LucidRenderStats{};
     double seg = 0, shadows = 0;
-    std::vector<int> hcnt((size_t)kCountersPerDepth * (depth + 1));
+    std::vector<int> hcnt((size_t)8 * (depth + 1));
     cudaEvent_t t0, t1;
     cudaEventCreate(&t0);
     cudaEventCreate(&t1);
@@ -3658,38 +3994,29 @@ int Engine::render_batch(const BatchItem* items, int n, const char* algorithm, l
         if (tab.empty()) return fail(LUCID_ERR_INVALID, "batch: a job piece does not fit a wave");
         CK(cudaMemcpyAsync(const_cast<BatchJob*>(d_jobs), tab.data(), tab.size() * sizeof(BatchJob),
                            cudaMemcpyHostToDevice, st));
-        CK(cudaMemsetAsync(P.counters.p, 0, sizeof(int) * kCountersPerDepth * (depth + 1), st));
         const int n_wave = (int)used;
-        const int bins = ((algo == ALGO_VOLUME_MIS || algo == ALGO_VOLUME_SIMPLE) ? kBinVolume : 0) |
-                         (n_wave >= kCellBinPaths ? kBinCells : 0);
+        const WavePlan w = wave_plan(device_, num_sms_, algo, false, 0, true, true, n_wave, depth);
+        if (w.depths > 0) CK(cudaMemsetAsync(P.counters.p, 0, sizeof(int) * kCountersPerDepth * (w.depths + 1), st));
         PathView pv = P.view;
         pv.scenes = d_scenes;
         pv.sid = P.sid.p;
-        for (int dd = 0; dd < depth; ++dd) {
-            int* cnt = P.counters.p + kCountersPerDepth * dd;
-            int* cnt_next = P.counters.p + kCountersPerDepth * (dd + 1);
-            int* qin = (dd & 1) ? P.q1.p : P.q0.p;
-            int* qout = (dd & 1) ? P.q0.p : P.q1.p;
-            pv.q0 = qin;
-            if (dd == 0)
-                k_trace_primary_batch<<<g_trace0, 128, 0, st>>>(pv, d_jobs, (int)tab.size(), (int)slots, n_wave, cnt, bins);
-            else
-                ks.trace<<<g_trace, 128, 0, st>>>(scene_tab[0], pv, cnt, 0, 0, bins);
-            k_bin_scatter<<<g_bin, 256, 0, st>>>(pv, cnt, dd == 0, qin, P.qb.p);
-            ks.shade<<<g_shade, kShadeThreads, 0, st>>>(scene_tab[0], fshade, pv, cnt, cnt_next, 0, P.qb.p, qout);
-            ks.shadow<<<g_shadow, 128, 0, st>>>(scene_tab[0], pv, cnt, 0);
-        }
+        enqueue_wave(w, scene_tab[0], fshade, pv, P.qb.p, depth, st, [&](const PathView& v, int* cnt) {
+            k_trace_primary_batch<<<w.g_trace0, 128, 0, st>>>(v, d_jobs, (int)tab.size(), (int)slots, n_wave, cnt, w.bins);
+        }, [](int, const PathView&, int*, const int*) {}, [](int, int, auto&& launch) { launch(); },
+        d_jobs, (int)tab.size(), (int)slots);
         for (const PieceFilm& pf : films) {
             const int np_j = (int)(film_off[(size_t)pf.job + 1] - film_off[(size_t)pf.job]);
             k_film<<<(np_j + 255) / 256, 256, 0, st>>>(np_j, pf.spw, P.rad.p + pf.path_base, P.film.p + film_off[pf.job]);
         }
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(hcnt.data(), P.counters.p, hcnt.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
+        PathsCount pc{};
+        if (w.depths > 0)
+            CK(cudaMemcpy2DAsync(hcnt.data(), 32, P.counters.p, sizeof(int) * kCountersPerDepth, 32, (size_t)w.depths,
+                                 cudaMemcpyDeviceToHost, st));
+        if (w.depths < depth || w.stop >= 0)
+            CK(cudaMemcpyAsync(&pc, P.errors.p + 4, sizeof(pc), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        for (int d = 0; d < depth; ++d) {
-            seg += hcnt[kCountersPerDepth * d];
-            shadows += hcnt[kCountersPerDepth * d + 1];
-        }
+        wave_totals(w, hcnt.data(), pc, seg, shadows);
         ++waves;
     }
     for (int k = 0; k < n && status == LUCID_OK; ++k) {
@@ -3801,7 +4128,6 @@ struct JobState {
     long long issued = 0;
     DBuf<int> dyn;
     FrameParams f{};
-    int g_trace0 = 0, g_trace = 0, g_shade = 0, g_shadow = 0, g_bin = 0;
     int profile = 0;   // launch profile of the job's kernels
 };
 
@@ -3818,26 +4144,11 @@ void Engine::enqueue_iteration(void* fp, int n) {
     f.s0 = 0;
     f.samples = n;
     f.n_wave = n * f.npix;
-    const LaunchSet ks = launch_set(algo_, false, J.profile);
-    const ShadeKernel shade = ks.shade;
-    const TraceKernel k_trace = ks.trace;
-    const ShadowKernel k_shadow = ks.shadow;
-    const int bins = ((algo_ == ALGO_VOLUME_MIS || algo_ == ALGO_VOLUME_SIMPLE) ? kBinVolume : 0) |
-                     ((long long)f.n_wave >= kCellBinPaths ? kBinCells : 0);
-    cudaMemsetAsync(P.counters.p, 0, sizeof(int) * kCountersPerDepth * (J.depth + 1), st);
-    for (int depth = 0; depth < J.depth; ++depth) {
-        int* cnt = P.counters.p + kCountersPerDepth * depth;
-        int* cnt_next = P.counters.p + kCountersPerDepth * (depth + 1);
-        PathView pv = P.view;
-        int* qin = (depth & 1) ? P.q1.p : P.q0.p;
-        int* qout = (depth & 1) ? P.q0.p : P.q1.p;
-        pv.q0 = qin;
-        if (depth == 0) k_trace_primary_for(ds_->view, f.pos)<<<J.g_trace0, 128, 0, st>>>(ds_->view, f, pv, cnt, 0, bins);
-        else k_trace<<<J.g_trace, 128, 0, st>>>(ds_->view, pv, cnt, 0, 0, bins);
-        k_bin_scatter<<<J.g_bin, 256, 0, st>>>(pv, cnt, depth == 0, qin, P.qb.p);
-        shade<<<J.g_shade, kShadeThreads, 0, st>>>(ds_->view, f, pv, cnt, cnt_next, 0, P.qb.p, qout);
-        k_shadow<<<J.g_shadow, 128, 0, st>>>(ds_->view, pv, cnt, 0);
-    }
+    const WavePlan w = wave_plan(device_, num_sms_, algo_, false, J.profile, false, true, f.n_wave, J.depth);
+    if (w.depths > 0) cudaMemsetAsync(P.counters.p, 0, sizeof(int) * kCountersPerDepth * (w.depths + 1), st);
+    enqueue_wave(w, ds_->view, f, P.view, P.qb.p, J.depth, st, [&](const PathView& pv, int* cnt) {
+        k_trace_primary_for(ds_->view, f.pos)<<<w.g_trace0, 128, 0, st>>>(ds_->view, f, pv, cnt, 0, w.bins);
+    }, [](int, const PathView&, int*, const int*) {}, [](int, int, auto&& launch) { launch(); });
     k_film<<<(f.npix + 255) / 256, 256, 0, st>>>(f.npix, n, P.rad.p, P.film.p);
 }
 
@@ -3863,7 +4174,7 @@ int Engine::job_begin(int w, int h, int spp, int max_depth, int chunk, bool use_
     }
     cudaStream_t st = S(stream_);
     CK(cudaMemsetAsync(P.film.p, 0, np * sizeof(float4), st));
-    CK(cudaMemsetAsync(P.errors.p, 0, 4 * sizeof(int), st));
+    CK(cudaMemsetAsync(P.errors.p, 0, kErrorInts * sizeof(int), st));
     if (!J.dyn.p) CK(J.dyn.alloc(1));
     FrameParams& f = J.f;
     f = FrameParams{};
@@ -3875,7 +4186,6 @@ int Engine::job_begin(int w, int h, int spp, int max_depth, int chunk, bool use_
     f.npix = (int)np;
     f.jitter = spp > 1 ? 1 : 0;
     J.profile = launch_profile_;
-    job_grids_locked();
     for (int k = 0; k < 2; ++k)
         if (!J.ev[k]) CK(cudaEventCreateWithFlags(&J.ev[k], cudaEventDisableTiming));
     J.issued = 0;
@@ -3903,23 +4213,6 @@ int Engine::capture_locked(int chunk) {
     return LUCID_OK;
 }
 
-// Persistent grids of the job's kernels for its launch profile: a whole
-// number of CTAs per SM.
-void Engine::job_grids_locked() {
-    JobState& J = *job_;
-    const LaunchSet ks = launch_set(algo_, false, J.profile);
-    int occ_t = 1, occ_s = 1, occ_h = 1, occ_t0 = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t0, k_trace_primary_t<false>, 128, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_t, ks.trace, 128, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, ks.shade, kShadeThreads, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_h, ks.shadow, 128, 0);
-    J.g_trace0 = num_sms_ * std::max(1, occ_t0);
-    J.g_trace = num_sms_ * std::max(1, occ_t);
-    J.g_shade = num_sms_ * std::max(1, occ_s);
-    J.g_shadow = num_sms_ * std::max(1, occ_h);
-    J.g_bin = num_sms_ * 8;
-}
-
 int Engine::set_launch_profile(int profile) {
     GpuLock gl(*this);
     if (profile < 0 || profile >= kLaunchProfiles) return fail(LUCID_ERR_INVALID, "unknown launch profile");
@@ -3935,7 +4228,6 @@ int Engine::job_set_profile(int profile, bool use_graph) {
     // iterations in flight were enqueued with the old grids; they finish first
     CK(cudaStreamSynchronize(S(stream_)));
     job_->profile = profile;
-    job_grids_locked();
     if (use_graph) return capture_locked(job_->chunk);
     if (job_->graph) { cudaGraphExecDestroy(job_->graph); job_->graph = nullptr; }
     return LUCID_OK;
@@ -4234,7 +4526,7 @@ constexpr size_t kNaShadow = na_round(sizeof(ShadowRec) * kNoAllocPaths);
 constexpr size_t kNaRad = na_round(sizeof(float4) * kNoAllocPaths);
 constexpr size_t kNaQ = na_round(sizeof(int) * kNoAllocPaths);
 constexpr size_t kNaCnt = na_round(sizeof(int) * kCountersPerDepth * (kNoAllocMaxDepth + 1));
-constexpr size_t kNaErr = na_round(sizeof(int) * 4);
+constexpr size_t kNaErr = na_round(sizeof(int) * kErrorInts);
 constexpr size_t kNaFilm = na_round(sizeof(float4) * kNoAllocPixels);
 constexpr size_t kNoAllocBytes = kNaState + kNaHit + kNaShadow + kNaRad + 2 * kNaQ + kNaCnt + kNaErr + kNaFilm;   // ~12 MB
 
@@ -4246,9 +4538,6 @@ namespace {
 // address).
 std::mutex g_noalloc_mu;
 unsigned char* g_noalloc_addr[64] = {};
-// Grid sizes (blocks) of the four wave kernels per device and integrator,
-// from the occupancy queries made on that device's first call.
-int g_noalloc_grid[64][5][4] = {};
 }  // namespace
 
 int Engine::render_noalloc(const LucidRenderParams& p, float* d_out) {
@@ -4277,9 +4566,7 @@ int Engine::render_noalloc(const LucidRenderParams& p, float* d_out) {
         return fail(LUCID_ERR_INVALID, "render_noalloc: path guiding is on; it needs allocated training and "
                                        "inference buffers (turn it off or use lucid_cuda_render_device)");
     CK(cudaSetDevice(device_));
-    const ShadeKernel shade = shade_kernel(algo_);
     unsigned char* base;
-    int grid[4];
     {
         std::lock_guard<std::mutex> lk(g_noalloc_mu);
         if (!g_noalloc_addr[device_]) {
@@ -4290,16 +4577,6 @@ int Engine::render_noalloc(const LucidRenderParams& p, float* d_out) {
             g_noalloc_addr[device_] = (unsigned char*)ptr;
         }
         base = g_noalloc_addr[device_];
-        int* g = g_noalloc_grid[device_][algo_];
-        if (g[0] == 0) {
-            int occ[4] = {1, 1, 1, 1};
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[0], k_trace_primary_t<false>, 128, 0);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[1], k_trace_lb<9>, 128, 0);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[2], shade, kShadeThreads, 0);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[3], k_shadow_lb<9>, 128, 0);
-            for (int k = 0; k < 4; ++k) g[k] = num_sms_ * std::max(1, occ[k]);
-        }
-        for (int k = 0; k < 4; ++k) grid[k] = g[k];
     }
     PathView v{};
     size_t off = 0;
@@ -4317,7 +4594,7 @@ int Engine::render_noalloc(const LucidRenderParams& p, float* d_out) {
     cudaStream_t st = S(stream_);
     // the array keeps the previous call's contents: clear what starts at zero
     CK(cudaMemsetAsync(film, 0, sizeof(float4) * np, st));
-    CK(cudaMemsetAsync(v.errors, 0, sizeof(int) * 4, st));
+    CK(cudaMemsetAsync(v.errors, 0, sizeof(int) * kErrorInts, st));
     FrameParams f{};
     for (int k = 0; k < 3; ++k) { f.pos[k] = cam_.pos[k]; f.fwd[k] = cam_.forward[k]; f.right[k] = cam_.right[k]; f.up[k] = cam_.up[k]; }
     f.aspect = (float)p.full_w / (float)p.full_h;
@@ -4327,7 +4604,6 @@ int Engine::render_noalloc(const LucidRenderParams& p, float* d_out) {
     f.samples = p.samples; f.sample_offset = p.sample_offset; f.max_depth = p.max_depth; f.algo = algo_;
     f.npix = (int)np;
     f.records = 0;
-    const int g_trace0 = grid[0], g_trace = grid[1], g_shade = grid[2], g_shadow = grid[3];
     const int spw = (int)std::max<long long>(1, std::min<long long>(p.samples, kNoAllocPaths / np));
     int status = LUCID_OK;
     for (int s0 = 0; s0 < p.samples; s0 += spw) {
@@ -4335,19 +4611,11 @@ int Engine::render_noalloc(const LucidRenderParams& p, float* d_out) {
         int this_spw = std::min(spw, p.samples - s0);
         f.s0 = s0;
         f.n_wave = (int)(this_spw * np);
-        CK(cudaMemsetAsync(v.counters, 0, sizeof(int) * kCountersPerDepth * (p.max_depth + 1), st));
-        for (int depth = 0; depth < p.max_depth; ++depth) {
-            int* cnt = v.counters + kCountersPerDepth * depth;
-            int* cnt_next = v.counters + kCountersPerDepth * (depth + 1);
-            PathView pv = v;
-            int* qin = (depth & 1) ? q1 : q0;
-            int* qout = (depth & 1) ? q0 : q1;
-            pv.q0 = qin;
-            if (depth == 0) k_trace_primary_for(ds_->view, f.pos)<<<g_trace0, 128, 0, st>>>(ds_->view, f, pv, cnt, 0, -1);
-            else k_trace_lb<9><<<g_trace, 128, 0, st>>>(ds_->view, pv, cnt, 0, 0, -1);
-            shade<<<g_shade, kShadeThreads, 0, st>>>(ds_->view, f, pv, cnt, cnt_next, depth == 0, qin, qout);
-            k_shadow_lb<9><<<g_shadow, 128, 0, st>>>(ds_->view, pv, cnt, 0);
-        }
+        const WavePlan w = wave_plan(device_, num_sms_, algo_, false, 0, false, false, f.n_wave, p.max_depth);
+        if (w.depths > 0) CK(cudaMemsetAsync(v.counters, 0, sizeof(int) * kCountersPerDepth * (w.depths + 1), st));
+        enqueue_wave(w, ds_->view, f, v, nullptr, p.max_depth, st, [&](const PathView& pv, int* cnt) {
+            k_trace_primary_for(ds_->view, f.pos)<<<w.g_trace0, 128, 0, st>>>(ds_->view, f, pv, cnt, 0, -1);
+        }, [](int, const PathView&, int*, const int*) {}, [](int, int, auto&& launch) { launch(); });
         k_film<<<(f.npix + 255) / 256, 256, 0, st>>>(f.npix, this_spw, v.rad, film);
         CK(cudaGetLastError());
         // no wait here: stream order keeps the next wave behind this film sum
@@ -4382,8 +4650,8 @@ int Engine::render_debug(int tx, int ty, int tw, int th, int fw, int fh, const c
     cudaStream_t st = S(stream_);
     PathPool& P = *pool_;
     if (P.film_n < np) { CK(P.film.alloc(np)); CK(P.out.alloc(np)); P.film_n = np; }
-    if (!P.errors.p) CK(P.errors.alloc(4));
-    CK(cudaMemsetAsync(P.errors.p, 0, 4 * sizeof(int), st));
+    if (!P.errors.p) CK(P.errors.alloc(kErrorInts));
+    CK(cudaMemsetAsync(P.errors.p, 0, kErrorInts * sizeof(int), st));
     FrameParams f{};
     for (int k = 0; k < 3; ++k) { f.pos[k] = cam_.pos[k]; f.fwd[k] = cam_.forward[k]; f.right[k] = cam_.right[k]; f.up[k] = cam_.up[k]; }
     f.aspect = (float)fw / (float)fh;

@@ -147,13 +147,14 @@ private:
     void enqueue_iteration(void* frame_params, int n);
     void job_end_locked();
     int capture_locked(int chunk);
-    void job_grids_locked();
     int build_ploc(const float4* verts, const int* sorted_ids, int n, int2* child, int2* range, float* nbox,
                    int* slot_ids, int& root);
     void free_scene();
 
     int device_ = 0;
     void* stream_ = nullptr;   // cudaStream_t
+    void* render_ev_[2] = {nullptr, nullptr};   // cudaEvent_t: start and end of a render call
+    int* host_counts_ = nullptr;                // pinned copies of a wave's counters
     int num_sms_ = 0;
     HostScene host_;
     HostCamera cam_;

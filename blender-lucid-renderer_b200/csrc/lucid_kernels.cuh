@@ -247,12 +247,15 @@ LD bool bvh_closest(const DevScene& sc, V3 o, V3 d, float tmin, HitRec& h) {
     return ok;
 }
 
-// Any hit over the BVH in [tmin, tmax]; overflow reported through ok.
+// Any hit over the BVH in [tmin, tmax]; overflow reported through ok.  FMA:
+// the slab form, as for bvh_closest.
+template <bool FMA = false>
 LD bool bvh_any(const DevScene& sc, V3 o, V3 d, float tmin, float tmax, bool& ok) {
     if (sc.num_big_tris && list_any(sc.big_tris, sc.num_big_tris, o, d, tmin, tmax)) return true;
     if (sc.num_bvh_tris == 0) return false;
     if (sc.root < 0) return test_leaf_any(sc.bvh_tris, sc.root, o, d, tmin, tmax);
     V3 inv = v3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+    const V3 ooi = v3(-o.x * inv.x, -o.y * inv.y, -o.z * inv.z);
     int stack[kStack];
     int sp = 0;
     int node = sc.root;
@@ -263,7 +266,7 @@ LD bool bvh_any(const DevScene& sc, V3 o, V3 d, float tmin, float tmax, bool& ok
             Node4 q;
             load_node4(sc.nodes, node, q);
             Hits4 hh;
-            node_hits<false>(q, o, o, inv, tmin, tmax, hh);
+            node_hits<FMA>(q, o, ooi, inv, tmin, tmax, hh);
             if (hh.n > 0) {
 #pragma unroll
                 for (int k = 3; k >= 1; --k)
@@ -365,8 +368,10 @@ LD bool trav_run_any(Trav& s, int* stack, const DevScene& sc, bool& ok, int step
 }
 
 // Runs up to `rounds` descend/test rounds; returns true when finished.
-template <bool ANY>
-LD bool trav_run(Trav& s, int* stack, float* stack_t, const DevScene& sc, bool& ok, int rounds) {
+// SEL: `fma` chooses the slab form per lane (a camera ray may start outside
+// the scene's coordinate bound); else every ray takes the FMA form.
+template <bool ANY, bool SEL = false>
+LD bool trav_run(Trav& s, int* stack, float* stack_t, const DevScene& sc, bool& ok, int rounds, bool fma = true) {
     static_assert(!ANY, "any-hit rays use trav_run_any over the 4-wide tree");
     for (int r = 0; r < rounds; ++r) {
         // descend until this lane holds a leaf (speculatively with its warp)
@@ -380,8 +385,14 @@ LD bool trav_run(Trav& s, int* stack, float* stack_t, const DevScene& sc, bool& 
             float4 a = __ldg(&n->lmin_lc), b = __ldg(&n->lmax_rc), c = __ldg(&n->rmin), e = __ldg(&n->rmax);
             int cl = __float_as_int(a.w), cr = __float_as_int(b.w);
             float tl, tr;
-            bool hl = box_hit_fma(a, b, s.ooi, s.inv, s.tmin, s.h.t, tl);
-            bool hr = box_hit_fma(c, e, s.ooi, s.inv, s.tmin, s.h.t, tr);
+            bool hl, hr;
+            if (!SEL || fma) {
+                hl = box_hit_fma(a, b, s.ooi, s.inv, s.tmin, s.h.t, tl);
+                hr = box_hit_fma(c, e, s.ooi, s.inv, s.tmin, s.h.t, tr);
+            } else {
+                hl = box_hit(a, b, s.o, s.inv, s.tmin, s.h.t, tl);
+                hr = box_hit(c, e, s.o, s.inv, s.tmin, s.h.t, tr);
+            }
             if (hl && hr) {
                 bool lfirst = tl <= tr;
                 if (s.sp < kStack) {
@@ -501,10 +512,11 @@ LD HitRec closest_skip_boundaries(const DevScene& sc, V3 o, V3 d, float tmin, bo
 }
 
 // is_shadowed_skipping_volume_boundaries (path_tracer.hpp:103-119).
+template <bool FMA = false>
 LD bool shadowed_skip_boundaries(const DevScene& sc, V3 o, V3 d, float tmax, bool& ok) {
     if (!sc.num_bnd_tris) {
         if (tmax <= 0.0f) return false;
-        return bvh_any(sc, o, d, RAY_T_MIN, tmax, ok);
+        return bvh_any<FMA>(sc, o, d, RAY_T_MIN, tmax, ok);
     }
     const V3 inv = v3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
     V3 po = o;
@@ -515,8 +527,8 @@ LD bool shadowed_skip_boundaries(const DevScene& sc, V3 o, V3 d, float tmax, boo
         HitRec b;
         b.t = rem; b.u = 0.0f; b.v = 0.0f; b.prim = -1;
         boundary_closest<true>(sc, po, d, inv, RAY_T_MIN, b);
-        if (b.prim < 0) return bvh_any(sc, po, d, RAY_T_MIN, rem, ok);
-        if (bvh_any(sc, po, d, RAY_T_MIN, b.t, ok)) return true;
+        if (b.prim < 0) return bvh_any<FMA>(sc, po, d, RAY_T_MIN, rem, ok);
+        if (bvh_any<FMA>(sc, po, d, RAY_T_MIN, b.t, ok)) return true;
         float skip = b.t + 1e-3f;
         off += skip;
         po = po + d * skip;
