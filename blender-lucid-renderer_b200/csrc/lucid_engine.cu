@@ -121,7 +121,7 @@ struct PathView {
     int* q1;
     int* qb;           // shading queue binned by event / material class
     unsigned short* cls;  // shading bin of each queue entry's pending event
-    int* counters;     // per depth: [0] active, [1] shadow, [2..4] fetch cursors,
+    int* counters;     // per depth: [0] active, [1] shadow, [2..4] fetch cursors, [5] shadow rays to trace,
                        // [8, 8 + kBins) bin counts, then kBins bin cursors
     int* errors;       // [0] traversal stack overflow, from [4] on k_paths' PathsCount
     int2* rec_prim;
@@ -338,14 +338,23 @@ __global__ void k_raygen(FrameParams f, PathView pv) {
 }
 
 // ---------------------------------------------------------------- trace
-// closest hit: descend/test rounds per lane between refills (five frames on
-// the 1M-triangle scene: 3 -> 321 ms, 4 -> 317 ms, 6 -> 362 ms)
-constexpr int kRounds = 4;
-// any hit: node visits per lane between refills (6: 3x slower; five frames:
-// 16 -> 229.7 ms, 24 -> 231.9 ms, 32 -> 240.4 ms)
-constexpr int kShadowSteps = 16;
+// Idle lanes of a warp that make it fetch new rays (1M-triangle frame, closest
+// hit + shadow rays: 8 -> 78.1 ms, 16 -> 77.2 ms, 20 -> 77.7 ms).
+constexpr int kRefill = 16;
 
 LD unsigned lanemask_lt() { return (1u << lane_id()) - 1u; }
+
+// Claims a queue index for each lane of `idle` (one atomic per warp); every
+// lane calls it.  `exhausted` is set for the warp once the queue is drained.
+LD int warp_refill(int* cursor, int n, unsigned idle, bool& exhausted) {
+    const int leader = __ffs(idle) - 1, want = __popc(idle);
+    int base = 0;
+    if ((int)lane_id() == leader) base = atomicAdd(cursor, want);
+    base = __shfl_sync(0xffffffffu, base, leader);
+    exhausted = base + want >= n;
+    const int r = base + __popc(idle & lanemask_lt());
+    return ((idle >> lane_id()) & 1u) && r < n ? r : -1;
+}
 
 // Per-lane dynamic refill: lanes without a ray claim new ones together (one
 // atomic per warp per round); `exhausted` stops claiming once the queue is
@@ -576,26 +585,23 @@ LD const DevScene& path_scene(const DevScene& sc, const PathView& pv, int id) {
     else return sc;
 }
 
-// Closest hit of extension rays (persistent, dynamic refill), including the
-// skip-volume-boundary rule (path_tracer.hpp:82-95) and native lights.
-// Nine resident CTAs per SM (at most 56 registers): one more warp group to
-// hide node-fetch latency than the unconstrained 61 registers allow
-// (1M-triangle scene: 8 CTAs 232 ms, 9 CTAs 221 ms, 10 CTAs 225 ms).
+// Closest BVH hit of extension rays (persistent, dynamic refill).  A round
+// ends with few of a warp's rays done (two lanes of 32 on the 1M-triangle
+// scene), so nothing but the traversal happens here: what a finished ray
+// needs besides — the triangles kept out of the BVH, volume boundaries,
+// native lights, its shading bin — is k_trace_post's, with every lane at
+// work.  (All of it at the end of a ray, in here: 65.6 ms a frame on that
+// scene.)
 template <int MINB, bool MULTI = false>
-__global__ void __launch_bounds__(128, MINB) k_trace_lb(DevScene sc0, PathView pv, int* cnt, int stop, int records,
-                                                      int bins) {
-    __shared__ int hist[kBins];
+__global__ void __launch_bounds__(128, MINB) k_trace_lb(DevScene sc0, PathView pv, int* cnt, int stop) {
     const int n = *(volatile int*)&cnt[0];
     if (n <= stop) return;   // left to k_paths (see WavePlan)
-    BinHist bh{hist};
-    bh.clear(bins);
     const int* q = pv.q0;
-    int stack[kStack];
-    float stack_t[kStack];
+    int2 stack[kStack];
     Trav s;
-    bool active = false, exhausted = false, ok = true;
-    int at = 0, depth = 0, peek = 0, sid = 0;
-    float search = 0.0f;
+    trav_none(s);
+    bool exhausted = false, ok = true;
+    int id = -1, sid = 0;
     // the lane's scene: the kernel's, or in a batch wave its ray's entry of
     // the wave's scene table (kept in a register between refills)
     auto scene = [&]() -> const DevScene& {
@@ -603,56 +609,83 @@ __global__ void __launch_bounds__(128, MINB) k_trace_lb(DevScene sc0, PathView p
         else return sc0;
     };
     for (;;) {
-        int r = refill(&cnt[2], n, !active, exhausted);
-        if (r >= 0) {
-            at = r;
-            const int id = q[r];
-            if constexpr (MULTI) sid = pv.sid[id];
-            const DevScene& sc = scene();
-            float4 ro = pv.st[id].ray_o, rd = pv.st[id].ray_d;
-            depth = __float_as_int(rd.w);
-            trav_begin<false>(s, sc, f3(ro), f3(rd), ro.w, 1e30f);
-            search = ro.w;
-            peek = 0;
-            active = true;
+        const unsigned idle = __ballot_sync(0xffffffffu, id < 0);
+        if (__popc(idle) >= kRefill && !exhausted) {
+            const int r = warp_refill(&cnt[2], n, idle, exhausted);
+            if (r >= 0) {
+                id = q[r];
+                if constexpr (MULTI) sid = pv.sid[id];
+                const float4 ro = pv.st[id].ray_o, rd = pv.st[id].ray_d;
+                trav_begin<false, false>(s, scene(), f3(ro), f3(rd), ro.w, 1e30f);
+            }
+        } else if (idle == 0xffffffffu) {
+            break;
         }
-        if (__ballot_sync(0xffffffffu, active) == 0) break;
-        if (!active) continue;
-        const DevScene& sc = scene();
-        if (!trav_run<false>(s, stack, stack_t, sc, ok, kRounds)) continue;
-        HitRec res = s.h;
+        warp_step(s, __popc(__ballot_sync(0xffffffffu, id >= 0)), stack, scene(), ok);
+        if (id >= 0 && trav_done(s)) {
+            pv.hit[id].hit = make_float4(s.h.t, s.h.u, s.h.v, __int_as_float(s.h.prim));
+            id = -1;
+        }
+    }
+    if (!ok) atomicAdd(&pv.errors[0], 1);
+}
+
+// The rest of a closest-hit query, one ray a lane in queue order: from the
+// closest BVH hit to the hit beyond the volume boundaries
+// (path_tracer.hpp:82-95), the native light in front of it, the shading bin
+// and the block's bin histogram.  `traced` 0: the scene has no BVH and
+// k_trace_lb did not run.
+constexpr int kPostThreads = 256;
+template <bool MULTI>
+__global__ void __launch_bounds__(kPostThreads) k_trace_post(DevScene sc0, PathView pv, int* cnt, int stop, int traced,
+                                                             int records, int bins) {
+    __shared__ int hist[kBins];
+    const int n = *(volatile int*)&cnt[0];
+    if (n <= stop) return;
+    BinHist bh{hist};
+    bh.clear(bins);
+    bool ok = true;
+    for (int i = blockIdx.x * kPostThreads + threadIdx.x; i < n; i += gridDim.x * kPostThreads) {
+        const int id = pv.q0[i];
+        const DevScene& sc = path_scene<MULTI>(sc0, pv, id);
+        const float4 ro = pv.st[id].ray_o, rd = pv.st[id].ray_d;
+        const V3 o = f3(ro), d = f3(rd);
+        HitRec real;
+        real.t = 1e30f; real.u = real.v = 0.0f; real.prim = -1;
+        if (traced) {
+            const float4 h = pv.hit[id].hit;
+            real.t = h.x; real.u = h.y; real.v = h.z; real.prim = __float_as_int(h.w);
+        }
+        if (sc.num_big_tris) list_closest(sc.big_tris, sc.num_big_tris, o, d, ro.w, real);
+        HitRec res = real;
         if (sc.num_bnd_tris) {
-            // resolve the closest real surface against boundary-only hits
-            bool restart = false;
-            for (;;) {
-                HitRec real = s.h;
+            const V3 inv = v3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+            float search = ro.w;
+            for (int peek = 0;;) {
                 HitRec b = real;
                 if (real.prim < 0) b.t = 1e30f;
-                boundary_closest<true>(sc, s.o, s.d, s.inv, search, b);
-                if (b.prim < 0) { res.prim = -1; res.t = 1e30f; break; }
+                boundary_closest<true>(sc, o, d, inv, search, b);
+                if (b.prim < 0) { res.prim = -1; break; }
                 if (b.prim == real.prim) { res = real; break; }
                 search = b.t + 1e-3f;
-                if (++peek == 8) { res.prim = -1; res.t = 1e30f; break; }
+                if (++peek == 8) { res.prim = -1; break; }
                 if (real.prim >= 0 && real.t < search) {
-                    trav_begin<false>(s, sc, s.o, s.d, search, 1e30f);
-                    restart = true;
-                    break;
+                    // the surface lies within the skipped millimetre: look again behind it
+                    real.t = 1e30f; real.u = real.v = 0.0f; real.prim = -1;
+                    ok &= bvh_closest<true>(sc, o, d, search, real);
                 }
             }
-            if (restart) continue;
         }
         if (res.prim < 0) { res.t = 1e30f; res.u = 0.0f; res.v = 0.0f; }
         float lt = 1e30f;
         // a native light counts only in front of the surface hit (the shading
         // kernel's `lh.y < hh.x`): lights beyond it are not tested
-        int li = (depth == 0) ? -1 : native_lights_closest(sc, s.o, s.d, res.t, lt);
-        const int id = q[at];
+        const int li = native_lights_closest(sc, o, d, res.t, lt);
         pv.hit[id].hit = make_float4(res.t, res.u, res.v, __int_as_float(res.prim));
         pv.hit[id].light = make_float4(__int_as_float(li), lt, 0.f, 0.f);
-        bh.add(sc, pv, at, bins, res.prim, res.t, li, lt, s.o, s.d);
+        bh.add(sc, pv, i, bins, res.prim, res.t, li, lt, o, d);
         if (records) {
-            int4 pi = res.prim >= 0 ? sc.prim_info[res.prim] : make_int4(-1, -1, -1, 0);
-            if (depth == 0) pv.rec_prim[id] = make_int2(pi.x, pi.y);
+            const int4 pi = res.prim >= 0 ? sc.prim_info[res.prim] : make_int4(-1, -1, -1, 0);
             pv.rec_cnt[id].x += 1;
             unsigned long long hs = pv.rec_hash[id];
             hs = hpush(hs, (uint32_t)pi.x);
@@ -660,7 +693,6 @@ __global__ void __launch_bounds__(128, MINB) k_trace_lb(DevScene sc0, PathView p
             hs = hpush(hs, (uint32_t)li);
             pv.rec_hash[id] = hs;
         }
-        active = false;
     }
     bh.flush(bins, cnt);
     if (!ok) atomicAdd(&pv.errors[0], 1);
@@ -1272,98 +1304,136 @@ __global__ void __launch_bounds__(32 * kInferWarps, 1) k_guide_infer(DevScene sc
 }
 
 // ---------------------------------------------------------------- shadow
-// Shadow rays (persistent, dynamic refill): is_shadowed_skipping_volume_
-// boundaries (path_tracer.hpp:103-119) with any-hit BVH queries; a segment
-// ends at the nearest boundary-only hit, past which the probe advances 1 mm.
-// The boundary triangles are tested one after another, without the group
-// boxes the closest-hit kernels use: on the 1M-triangle scene the box tests
-// made this kernel 4 % slower (more registers at its 56-register cap),
-// while they save the closest-hit kernels 7 %.
-// Nine resident CTAs per SM as for k_trace (shadow time -0.7 %; 10: +4 %).
+// A shadow ray's verdict (is_shadowed_skipping_volume_boundaries,
+// path_tracer.hpp:103-119): adds the light sample when unoccluded.
+LD void shadow_done(const PathView& pv, int at, bool occ, int records) {
+    if (!occ) {
+        const float4 c = pv.sh[at].c;
+        const int id = __float_as_int(c.w);
+        const float4 ra = pv.rad[id];
+        pv.rad[id] = make_float4(ra.x + c.x, ra.y + c.y, ra.z + c.z, 0.0f);
+        if (pv.grec) guide_credit(pv, id, rgb(c.x, c.y, c.z), __float_as_int(pv.sh[at].d.w));
+    }
+    if (records) {
+        const int id = __float_as_int(pv.sh[at].c.w);
+        int4 rc = pv.rec_cnt[id];
+        rc.y += 1;
+        rc.z += occ ? 1 : 0;
+        pv.rec_cnt[id] = rc;
+        pv.rec_hash[id] = hpush(pv.rec_hash[id], 0x5EED0000u | (occ ? 1u : 0u));
+    }
+}
+
+// What of a shadow ray needs no BVH, one ray a lane: the end of its first
+// segment at the nearest volume boundary and the triangles kept out of the
+// BVH.  Rays decided here are done; a ray that would add nothing (a spot
+// light outside its cone) is dropped, unless per-sample records count it.  On
+// the 1M-triangle 960x540 frame the two full-lane passes take 98 us (this)
+// and 180 us (k_trace_post) of the 1.0 and 1.0 ms of shadow rays and closest
+// hits.
+// The others go to k_shadow_lb's queue (pv.q0, whose depth is shaded by now)
+// with their segment's end (in the hit records, which are free until the
+// next trace).
+template <bool MULTI>
+__global__ void __launch_bounds__(kPostThreads) k_shadow_pre(DevScene sc0, PathView pv, int* cnt, int records) {
+    const int n = *(volatile int*)&cnt[1];
+    float* const seg_end = reinterpret_cast<float*>(pv.hit);
+    for (int i0 = blockIdx.x * kPostThreads; i0 < n; i0 += gridDim.x * kPostThreads) {
+        const int at = i0 + (int)threadIdx.x;
+        bool trace = false;
+        float bt = -1.0f;
+        if (at < n) {
+            const float4 so = pv.sh[at].o, sd = pv.sh[at].d, c = pv.sh[at].c;
+            const DevScene& sc = path_scene<MULTI>(sc0, pv, __float_as_int(c.w));
+            if (records || c.x != 0.0f || c.y != 0.0f || c.z != 0.0f) {
+                const V3 o = f3(so), d = f3(sd);
+                const float rem = so.w;
+                bool done = true, occ = false;
+                if (!(rem <= 0.0f)) {
+                    if (sc.num_bnd_tris) {
+                        HitRec b; b.t = rem; b.u = 0.f; b.v = 0.f; b.prim = -1;
+                        boundary_closest_all(sc, o, d, RAY_T_MIN, b);
+                        if (b.prim >= 0) bt = b.t;
+                    }
+                    if (sc.num_big_tris)
+                        occ = list_any(sc.big_tris, sc.num_big_tris, o, d, RAY_T_MIN, bt >= 0.0f ? bt : rem);
+                    done = occ || (sc.num_bvh_tris == 0 && bt < 0.0f);
+                }
+                if (done) shadow_done(pv, at, occ, records);
+                trace = !done;
+            }
+        }
+        const int j = warp_append(&cnt[5], trace);
+        if (trace) {
+            pv.q0[j] = at;
+            seg_end[j] = bt;
+        }
+    }
+}
+
+// Shadow rays over the BVH (persistent, dynamic refill); a segment ends at
+// the nearest boundary-only hit, past which the probe advances 1 mm.  As for
+// k_trace_lb, few lanes start or finish a ray at a time, so a ray's first
+// segment is prepared by k_shadow_pre (in here: 46.9 ms a frame on the
+// 1M-triangle scene).
 template <int MINB, bool MULTI = false>
 __global__ void __launch_bounds__(128, MINB) k_shadow_lb(DevScene sc0, PathView pv, int* cnt, int records) {
-    const int n = *(volatile int*)&cnt[1];
+    const int n = *(volatile int*)&cnt[5];
     if (n == 0) return;
+    const float* const seg_end = reinterpret_cast<const float*>(pv.hit);
     int stack[kStack];
     Trav s;
-    bool active = false, exhausted = false, ok = true;
-    int at = 0, peek = 0, sid = 0;
+    trav_none(s);
+    bool exhausted = false, ok = true;
+    int at = -1, peek = 0, sid = 0;
     float tmax = 0.0f, off = 0.0f, bt = -1.0f;
-    V3 po = v3(0.f, 0.f, 0.f), d = v3(0.f, 0.f, 1.f);
     // the lane's scene (a batch wave: its ray's entry of the scene table)
     auto scene = [&]() -> const DevScene& {
         if constexpr (MULTI) return pv.scenes[sid];
         else return sc0;
     };
     for (;;) {
-        int r = refill(&cnt[4], n, !active, exhausted);
-        int outcome = -1;   // -1 running, 0 unoccluded, 1 occluded
-        if (r >= 0) {
-            at = r;
-            if constexpr (MULTI) sid = pv.sid[__float_as_int(pv.sh[at].c.w)];
+        const unsigned idle = __ballot_sync(0xffffffffu, at < 0);
+        if (__popc(idle) >= kRefill && !exhausted) {
+            const int r = warp_refill(&cnt[4], n, idle, exhausted);
+            if (r >= 0) {
+                at = pv.q0[r];
+                bt = seg_end[r];
+                if constexpr (MULTI) sid = pv.sid[__float_as_int(pv.sh[at].c.w)];
+                const float4 so = pv.sh[at].o, sd = pv.sh[at].d;
+                tmax = so.w; off = 0.0f; peek = 0;
+                trav_begin<true, false>(s, scene(), f3(so), f3(sd), RAY_T_MIN, bt >= 0.0f ? bt : tmax);
+            }
+        } else if (idle == 0xffffffffu) {
+            break;
+        }
+        warp_step_any(s, __popc(__ballot_sync(0xffffffffu, at >= 0)), stack, scene(), ok);
+        if (at >= 0 && trav_done(s)) {
             const DevScene& sc = scene();
-            float4 so = pv.sh[at].o, sd = pv.sh[at].d;
-            po = f3(so); d = f3(sd); tmax = so.w; off = 0.0f; peek = 0;
-            active = true;
-            // first segment
-            float rem = tmax - off;
-            if (rem <= 0.0f) outcome = 0;
-            else {
-                bt = -1.0f;
-                if (sc.num_bnd_tris) {
+            bool occ = s.any_hit, next = false;
+            if (!occ && bt >= 0.0f) {
+                // skip past the boundary hit and start the next segment
+                const float skip = bt + 1e-3f;
+                off += skip;
+                const V3 po = s.o + s.d * skip, d = s.d;
+                const float rem = tmax - off;
+                if (++peek < 8 && !(rem <= 0.0f)) {
+                    bt = -1.0f;
                     HitRec b; b.t = rem; b.u = 0.f; b.v = 0.f; b.prim = -1;
                     boundary_closest_all(sc, po, d, RAY_T_MIN, b);
                     if (b.prim >= 0) bt = b.t;
-                }
-                trav_begin<true>(s, sc, po, d, RAY_T_MIN, bt >= 0.0f ? bt : rem);
-                if (s.any_hit) outcome = 1;
-            }
-        }
-        if (__ballot_sync(0xffffffffu, active) == 0) break;
-        if (!active) continue;
-        if (outcome < 0) {
-            const DevScene& sc = scene();
-            if (!trav_run_any(s, stack, sc, ok, kShadowSteps)) continue;
-            if (s.any_hit) outcome = 1;
-            else if (bt < 0.0f) outcome = 0;
-            else {
-                // skip past the boundary hit and start the next segment
-                float skip = bt + 1e-3f;
-                off += skip;
-                po = po + d * skip;
-                if (++peek == 8) outcome = 0;
-                else {
-                    float rem = tmax - off;
-                    if (rem <= 0.0f) outcome = 0;
-                    else {
-                        bt = -1.0f;
-                        HitRec b; b.t = rem; b.u = 0.f; b.v = 0.f; b.prim = -1;
-                        boundary_closest_all(sc, po, d, RAY_T_MIN, b);
-                        if (b.prim >= 0) bt = b.t;
-                        trav_begin<true>(s, sc, po, d, RAY_T_MIN, bt >= 0.0f ? bt : rem);
-                        if (s.any_hit) outcome = 1;
-                    }
+                    trav_begin<true>(s, sc, po, d, RAY_T_MIN, bt >= 0.0f ? bt : rem);
+                    occ = s.any_hit;
+                    next = !occ;
                 }
             }
-            if (outcome < 0) continue;
+            if (!next) {
+                shadow_done(pv, at, occ, records);
+                trav_none(s);
+                at = -1;
+            }
         }
-        bool occ = outcome == 1;
-        if (!occ) {
-            const float4 c = pv.sh[at].c;
-            const int id = __float_as_int(c.w);
-            const float4 ra = pv.rad[id];
-            pv.rad[id] = make_float4(ra.x + c.x, ra.y + c.y, ra.z + c.z, 0.0f);
-            if (pv.grec) guide_credit(pv, id, rgb(c.x, c.y, c.z), __float_as_int(pv.sh[at].d.w));
-        }
-        if (records) {
-            const int id = __float_as_int(pv.sh[at].c.w);
-            int4 rc = pv.rec_cnt[id];
-            rc.y += 1;
-            rc.z += occ ? 1 : 0;
-            pv.rec_cnt[id] = rc;
-            pv.rec_hash[id] = hpush(pv.rec_hash[id], 0x5EED0000u | (occ ? 1u : 0u));
-        }
-        active = false;
+        __syncwarp();
     }
     if (!ok) atomicAdd(&pv.errors[0], 1);
 }
@@ -1407,8 +1477,7 @@ __global__ void __launch_bounds__(128, 4) k_paths(DevScene sc0, FrameParams f0, 
         if (slots == 0) return;
         q = (d & 1) ? pv.q1 : pv.q0;
     }
-    int stack[kStack];
-    float stack_t[kStack];
+    int2 stack[kStack];
     Trav s;
     bool active = false, exhausted = false, ok = true;
     int id = 0, sid = 0;
@@ -1478,19 +1547,25 @@ __global__ void __launch_bounds__(128, 4) k_paths(DevScene sc0, FrameParams f0, 
         float lt = 1e30f;
         int li = -1;
         const bool records = !MULTI && f0.records != 0;
-        if (active) {
-            // closest hit beyond the volume boundaries (k_trace_lb)
-            const float tmin = ps.depth == 0 ? 0.0f : RAY_T_MIN;
-            const bool fma = ps.depth != 0 || fma0;
-            float search = tmin;
-            trav_begin<false>(s, sc, ps.o, ps.d, tmin, 1e30f);
-            int peek = 0;
-            for (;;) {
-                while (!trav_run<false, true>(s, stack, stack_t, sc, ok, 64, fma)) {}
+        // closest hit beyond the volume boundaries (k_trace_lb, k_trace_post)
+        const bool fma = ps.depth != 0 || fma0;
+        const V3 sub = fma ? v3(0.f, 0.f, 0.f) : ps.o;
+        float search = ps.depth == 0 ? 0.0f : RAY_T_MIN;
+        auto begin = [&] {
+            trav_begin<false>(s, sc, ps.o, ps.d, search, 1e30f);
+            if (!fma) s.ooi = v3(0.f, 0.f, 0.f);
+        };
+        trav_none(s);
+        if (active) begin();
+        bool query = active;   // looking for the closest hit from `search` on
+        int peek = 0;
+        while (__ballot_sync(0xffffffffu, query) != 0) {
+            for (unsigned m; (m = __ballot_sync(0xffffffffu, !trav_done(s))) != 0;)
+                warp_step<true>(s, __popc(m), stack, sc, ok, sub);
+            if (query) {
+                query = false;
                 h = s.h;
-                if (!sc.num_bnd_tris) break;
-                bool restart = false;
-                for (;;) {
+                while (sc.num_bnd_tris) {
                     HitRec b = s.h;
                     if (b.prim < 0) b.t = 1e30f;
                     boundary_closest<true>(sc, s.o, s.d, s.inv, search, b);
@@ -1499,13 +1574,15 @@ __global__ void __launch_bounds__(128, 4) k_paths(DevScene sc0, FrameParams f0, 
                     search = b.t + 1e-3f;
                     if (++peek == 8) { h.prim = -1; break; }
                     if (s.h.prim >= 0 && s.h.t < search) {
-                        trav_begin<false>(s, sc, s.o, s.d, search, 1e30f);
-                        restart = true;
+                        begin();
+                        query = true;
                         break;
                     }
                 }
-                if (!restart) break;
             }
+            __syncwarp();
+        }
+        if (active) {
             if (h.prim < 0) { h.t = 1e30f; h.u = 0.0f; h.v = 0.0f; }
             li = ps.depth == 0 ? -1 : native_lights_closest(sc, ps.o, ps.d, h.t, lt);
             ++nseg;
@@ -1572,7 +1649,7 @@ static PathsKernel paths_kernel(int algo) {
 // shading 8, shadow 9); profile 1 gives each kernel more registers and fewer
 // spills (8, 6, 8), which scenes with short paths or few triangles can
 // prefer.  The request loop's autotuner picks per job shape.
-using TraceKernel = void (*)(DevScene, PathView, int*, int, int, int);
+using TraceKernel = void (*)(DevScene, PathView, int*, int);
 using ShadowKernel = void (*)(DevScene, PathView, int*, int);
 struct LaunchSet {
     TraceKernel trace;
@@ -2271,9 +2348,10 @@ __global__ void k_gather_tris(const float4* tri, const int* sorted_ids, int n, f
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     int prim = sorted_ids[k];
-    out[3 * k] = tri[3 * prim];
-    out[3 * k + 1] = tri[3 * prim + 1];
-    out[3 * k + 2] = tri[3 * prim + 2];
+    out[4 * k] = tri[3 * prim];
+    out[4 * k + 1] = tri[3 * prim + 1];
+    out[4 * k + 2] = tri[3 * prim + 2];
+    out[4 * k + 3] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // ---------------------------------------------------------------- Engine
@@ -2753,7 +2831,7 @@ int Engine::build_bvh() {
     CK(d_temp.alloc(temp));
     CK(cub::DeviceRadixSort::SortPairs(d_temp.p, temp, d_keys.p, d_keys_sorted.p, d_vals.p, d_vals_sorted.p, n, 0, 63,
                                        st));
-    CK(D.bvh_tris.alloc((size_t)3 * n));
+    CK(D.bvh_tris.alloc((size_t)4 * n));
     v.bvh_tris = D.bvh_tris.p;
     if (n <= 4) {
         k_gather_tris<<<(n + 255) / 256, 256, 0, st>>>(d_tri.p, d_vals_sorted.p, n, D.bvh_tris.p);
@@ -3025,7 +3103,7 @@ constexpr long long kPathsWave = 1LL << 17;
 struct WavePlan {
     LaunchSet ks;
     PathsKernel paths;
-    int g_trace0 = 1, g_trace = 1, g_shade = 1, g_shadow = 1, g_bin = 1, g_paths = 1;   // blocks
+    int g_trace0 = 1, g_trace = 1, g_shade = 1, g_shadow = 1, g_bin = 1, g_paths = 1, g_post = 1;   // blocks
     int depths = 0, stop = -1;
     int bins = -1;   // shading bins (BinHist); -1: the queues are shaded as they are
 };
@@ -3059,6 +3137,7 @@ static WavePlan wave_plan(int device, int sms, int algo, bool guide, int profile
         w.g_paths = sms * o[4];
     }
     w.g_bin = sms * 8;
+    w.g_post = sms * 4;
     if (binned)
         w.bins = ((algo == ALGO_VOLUME_MIS || algo == ALGO_VOLUME_SIMPLE) ? kBinVolume : 0) |
                  (paths >= kCellBinPaths ? kBinCells : 0);
@@ -3095,7 +3174,12 @@ static void enqueue_wave(const WavePlan& w, const DevScene& sc, const FrameParam
         if (depth == 0)
             mark(K_TRACE0, depth, [&] { primary(pv, cnt); });
         else
-            mark(K_TRACE, depth, [&] { w.ks.trace<<<w.g_trace, 128, 0, st>>>(sc, pv, cnt, stop, f.records, w.bins); });
+            mark(K_TRACE, depth, [&] {
+                const int traced = jobs || sc.num_bvh_tris > 0;
+                if (traced) w.ks.trace<<<w.g_trace, 128, 0, st>>>(sc, pv, cnt, stop);
+                const auto post = jobs ? k_trace_post<true> : k_trace_post<false>;
+                post<<<w.g_post, kPostThreads, 0, st>>>(sc, pv, cnt, stop, traced, f.records, w.bins);
+            });
         infer(depth, pv, cnt, qin);
         int identity = depth == 0;
         if (w.bins >= 0) {
@@ -3106,7 +3190,12 @@ static void enqueue_wave(const WavePlan& w, const DevScene& sc, const FrameParam
             w.ks.shade<<<w.g_shade, kShadeThreads, 0, st>>>(sc, f, pv, cnt, cnt_next, identity, stop,
                                                             w.bins >= 0 ? qb : qin, qout);
         });
-        mark(K_SHADOW, depth, [&] { w.ks.shadow<<<w.g_shadow, 128, 0, st>>>(sc, pv, cnt, f.records); });
+        mark(K_SHADOW, depth, [&] {
+            const auto pre = jobs ? k_shadow_pre<true> : k_shadow_pre<false>;
+            pre<<<w.g_post, kPostThreads, 0, st>>>(sc, pv, cnt, f.records);
+            if (jobs || sc.num_bvh_tris > 0 || sc.num_bnd_tris > 0)
+                w.ks.shadow<<<w.g_shadow, 128, 0, st>>>(sc, pv, cnt, f.records);
+        });
     }
     if (max_depth < 1 || (w.depths == max_depth && w.stop < 0)) return;
     int grid = w.g_paths, fma0 = 0;

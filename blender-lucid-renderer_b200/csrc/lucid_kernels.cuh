@@ -65,6 +65,25 @@ LD void load_tri(const float4* tris, int k, V3& v0, V3& e1, V3& e2, int& prim) {
     prim = __float_as_int(a.w);
 }
 
+// 32 bytes at a 32-byte boundary in one load.  Lanes of a warp visit different
+// nodes and triangles, so a load costs the L1 one pass per lane and
+// instruction whatever its width: a 64-byte node or triangle takes two
+// passes this way, four with 16-byte loads (the traversal kernels kept the
+// L1's data path 62 % busy with those).
+LD void ldg32(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+// Triangle k of the BVH's array: 64 bytes each (v0 | prim, e1, e2, unused).
+LD void load_bvh_tri(const float4* tris, int k, V3& v0, V3& e1, V3& e2, int& prim) {
+    float4 a, b, c, d;
+    ldg32(tris + 4 * k, a, b);
+    ldg32(tris + 4 * k + 2, c, d);
+    v0 = f3(a); e1 = f3(b); e2 = f3(c);
+    prim = __float_as_int(a.w);
+}
+
 // Closest-hit tie rule: on equal t the larger global prim id wins.  Global
 // ids are mesh-major, so across meshes this is the reference's "later mesh
 // wins" (bvh.hpp:167-174 passes the running t as an inclusive bound).
@@ -74,7 +93,7 @@ LD void test_leaf_closest(const float4* tris, int code, V3 o, V3 d, float tmin, 
     for (int k = start; k < start + count; ++k) {
         V3 v0, e1, e2;
         int prim;
-        load_tri(tris, k, v0, e1, e2, prim);
+        load_bvh_tri(tris, k, v0, e1, e2, prim);
         float t, u, v;
         if (isect_tri(o, d, v0, e1, e2, tmin, h.t, t, u, v)) {
             if (t < h.t || prim > h.prim) { h.t = t; h.u = u; h.v = v; h.prim = prim; }
@@ -87,7 +106,7 @@ LD bool test_leaf_any(const float4* tris, int code, V3 o, V3 d, float tmin, floa
     for (int k = start; k < start + count; ++k) {
         V3 v0, e1, e2;
         int prim;
-        load_tri(tris, k, v0, e1, e2, prim);
+        load_bvh_tri(tris, k, v0, e1, e2, prim);
         float t, u, v;
         if (isect_tri(o, d, v0, e1, e2, tmin, tmax, t, u, v)) return true;
     }
@@ -162,8 +181,9 @@ struct Node4 {
 };
 LD void load_node4(const DevNode4* nodes, int i, Node4& q) {
     const float4* p = reinterpret_cast<const float4*>(nodes + i);
-    q.x0 = __ldg(p); q.x1 = __ldg(p + 1); q.y0 = __ldg(p + 2); q.y1 = __ldg(p + 3);
-    q.z0 = __ldg(p + 4); q.z1 = __ldg(p + 5);
+    ldg32(p, q.x0, q.x1);
+    ldg32(p + 2, q.y0, q.y1);
+    ldg32(p + 4, q.z0, q.z1);
     q.c = __ldg(reinterpret_cast<const int4*>(p + 6));
 }
 LD float lane4(const float4& v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
@@ -224,7 +244,9 @@ LD bool bvh_closest(const DevScene& sc, V3 o, V3 d, float tmin, HitRec& h) {
     bool ok = true;
     while (true) {
         const DevNode* n = sc.nodes2 + node;
-        float4 a = __ldg(&n->lmin_lc), b = __ldg(&n->lmax_rc), c = __ldg(&n->rmin), e = __ldg(&n->rmax);
+        float4 a, b, c, e;
+        ldg32(&n->lmin_lc, a, b);
+        ldg32(&n->rmin, c, e);
         int cl = __float_as_int(a.w), cr = __float_as_int(b.w);
         float tl, tr;
         bool hl = FMA ? box_hit_fma(a, b, ooi, inv, tmin, h.t, tl) : box_hit(a, b, o, inv, tmin, h.t, tl);
@@ -283,26 +305,40 @@ LD bool bvh_any(const DevScene& sc, V3 o, V3 d, float tmin, float tmax, bool& ok
     return false;
 }
 
-// ---- resumable while-while traversal for the persistent kernels ----
-// Aila & Laine ("Understanding the efficiency of ray traversal on GPUs",
-// HPG 2009): each lane descends internal nodes until it has found a leaf,
-// postponing the leaf; the warp leaves the descent loop once every lane holds
-// a leaf (or is done), then all lanes test their leaves together.  The stack
-// keeps each entry's entry distance so closest-hit queries skip entries that
-// a nearer hit has made unreachable.  A lane runs a bounded number of
-// descend/test rounds between work refills.
+// ---- warp-synchronous traversal ----
+// A lane's query is a small state machine (Trav); the lanes of a warp step it
+// together (warp_step).  A leaf reached is postponed (Aila and Laine,
+// "Understanding the efficiency of ray traversal on GPUs", HPG 2009): the
+// lane goes on to the next node and tests the leaf's triangles when its warp
+// does, stopping only at a second leaf.  The top of the stack is kept in
+// registers, so a pop waits for no load: the next entry arrives behind the
+// popped node's fetch.
 struct Trav {
     V3 o, d, inv, ooi;   // ooi = -o * inv
     float tmin;
     HitRec h;        // closest: running best; any: h.t is the fixed limit
-    int node;        // next entry (internal node index or leaf code), or kTravDone
+    int node;        // internal node to visit, leaf code (while another leaf is
+                     // postponed), kTravPop or kTravDone
     int leaf;        // postponed leaf code, 0 when none
-    int sp;
+    int sp;          // stack entries, the top one included
+    int top;         // the top entry: code, and (closest hit) entry distance
+    float top_t;
     bool any_hit;
 };
 constexpr int kTravDone = 0x7fffffff;
+constexpr int kTravPop = 0x7ffffffe;   // take the next stack entry
 
-template <bool ANY>
+LD void trav_settle(Trav& s);
+// No query: what idle lanes hold.
+LD void trav_none(Trav& s) {
+    s.node = kTravDone;
+    s.leaf = 0;
+    s.sp = 0;
+    s.any_hit = false;
+}
+// Starts a query over the BVH alone (LIST false) or after the triangles kept
+// out of it.
+template <bool ANY, bool LIST = true>
 LD void trav_begin(Trav& s, const DevScene& sc, V3 o, V3 d, float tmin, float tmax) {
     s.o = o; s.d = d;
     s.inv = v3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
@@ -310,10 +346,12 @@ LD void trav_begin(Trav& s, const DevScene& sc, V3 o, V3 d, float tmin, float tm
     s.tmin = tmin;
     s.h.t = tmax; s.h.u = 0.0f; s.h.v = 0.0f; s.h.prim = -1;
     s.sp = 0;
+    s.top = 0;
+    s.top_t = 0.0f;
     s.leaf = 0;
     s.any_hit = false;
     s.node = kTravDone;
-    if (sc.num_big_tris) {
+    if (LIST && sc.num_big_tris) {
         if (ANY) {
             if (list_any(sc.big_tris, sc.num_big_tris, o, d, tmin, tmax)) { s.any_hit = true; return; }
         } else {
@@ -321,117 +359,195 @@ LD void trav_begin(Trav& s, const DevScene& sc, V3 o, V3 d, float tmin, float tm
         }
     }
     if (sc.num_bvh_tris == 0) return;
-    s.node = ANY ? sc.root : sc.root2;   // a leaf code when the whole BVH is one leaf
+    s.node = ANY ? sc.root : sc.root2;
+    trav_settle(s);   // the whole BVH may be one leaf
 }
 
-LD int trav_pop(Trav& s, const int* stack, const float* stack_t) {
-    while (s.sp > 0) {
-        --s.sp;
-        if (stack_t[s.sp] <= s.h.t * 1.00000095367431640625f) return stack[s.sp];
+LD bool trav_inner(int node) { return (unsigned)node < (unsigned)kTravDone; }   // a node to visit, or kTravPop
+LD bool trav_done(const Trav& s) { return s.node == kTravDone && s.leaf == 0; }
+
+// Closest hit.  Stack entries are (code, entry distance).
+LD void trav_push(Trav& s, int2* stack, int code, float t, bool& ok) {
+    if (s.sp > 0) {
+        if (s.sp <= kStack) stack[s.sp - 1] = make_int2(s.top, __float_as_int(s.top_t));
+        else ok = false;
     }
-    return kTravDone;
+    s.top = code;
+    s.top_t = t;
+    ++s.sp;
 }
-
-// Any-hit stepping for shadow rays: leaves are tested as soon as they are
-// reached (an occluder found early ends the ray), one node or leaf per step.
-LD bool trav_run_any(Trav& s, int* stack, const DevScene& sc, bool& ok, int steps) {
-    for (int k = 0; k < steps; ++k) {
-        if (s.node == kTravDone) return true;
-        if (s.node < 0) {
-            if (test_leaf_any(sc.bvh_tris, s.node, s.o, s.d, s.tmin, s.h.t)) {
-                s.any_hit = true;
-                s.node = kTravDone;
-                return true;
-            }
-        } else {
-            Node4 q;
-            load_node4(sc.nodes, s.node, q);
-            Hits4 hh;
-            node_hits<true>(q, s.o, s.ooi, s.inv, s.tmin, s.h.t, hh);
-            if (hh.n > 0) {
-#pragma unroll
-                for (int j = 3; j >= 1; --j)
-                    if (hh.n > j) {
-                        if (s.sp < kStack) stack[s.sp++] = hh.c[j]; else ok = false;
-                    }
-                s.node = hh.c[0];
-                continue;
-            }
-        }
+// A leaf reached while none is postponed becomes the postponed one; a lane
+// without a node then takes the top entry, or drops it where a nearer hit has
+// made it unreachable (and takes the next at its next step).
+LD void trav_settle(Trav& s) {
+    if (s.node < 0 && s.leaf == 0) {
+        s.leaf = s.node;
+        s.node = kTravPop;
+    }
+}
+LD void trav_pop(Trav& s, const int2* stack) {
+    while (s.node == kTravPop) {
         if (s.sp == 0) {
             s.node = kTravDone;
-            return true;
+            break;
         }
-        s.node = stack[--s.sp];
+        if (s.top_t <= s.h.t * 1.00000095367431640625f) s.node = s.top;
+        if (--s.sp > 0) {
+            const int2 e = stack[s.sp - 1];
+            s.top = e.x;
+            s.top_t = __int_as_float(e.y);
+        }
+        trav_settle(s);
     }
-    return false;
 }
 
-// Runs up to `rounds` descend/test rounds; returns true when finished.
-// SEL: `fma` chooses the slab form per lane (a camera ray may start outside
-// the scene's coordinate bound); else every ray takes the FMA form.
-template <bool ANY, bool SEL = false>
-LD bool trav_run(Trav& s, int* stack, float* stack_t, const DevScene& sc, bool& ok, int rounds, bool fma = true) {
-    static_assert(!ANY, "any-hit rays use trav_run_any over the 4-wide tree");
-    for (int r = 0; r < rounds; ++r) {
-        // descend until this lane holds a leaf (speculatively with its warp)
-        while (s.node != kTravDone && s.leaf == 0) {
-            if (s.node < 0) {                      // a leaf reached by popping
-                s.leaf = s.node;
-                s.node = trav_pop(s, stack, stack_t);
-                break;
-            }
-            const DevNode* n = sc.nodes2 + s.node;
-            float4 a = __ldg(&n->lmin_lc), b = __ldg(&n->lmax_rc), c = __ldg(&n->rmin), e = __ldg(&n->rmax);
-            int cl = __float_as_int(a.w), cr = __float_as_int(b.w);
-            float tl, tr;
-            bool hl, hr;
-            if (!SEL || fma) {
-                hl = box_hit_fma(a, b, s.ooi, s.inv, s.tmin, s.h.t, tl);
-                hr = box_hit_fma(c, e, s.ooi, s.inv, s.tmin, s.h.t, tr);
-            } else {
-                hl = box_hit(a, b, s.o, s.inv, s.tmin, s.h.t, tl);
-                hr = box_hit(c, e, s.o, s.inv, s.tmin, s.h.t, tr);
-            }
-            if (hl && hr) {
-                bool lfirst = tl <= tr;
-                if (s.sp < kStack) {
-                    stack[s.sp] = lfirst ? cr : cl;
-                    stack_t[s.sp] = lfirst ? tr : tl;
-                    ++s.sp;
-                } else {
-                    ok = false;
-                }
-                s.node = lfirst ? cl : cr;
-            } else if (hl) {
-                s.node = cl;
-            } else if (hr) {
-                s.node = cr;
-            } else {
-                s.node = trav_pop(s, stack, stack_t);
-            }
-            if (s.node != kTravDone && s.node < 0) {   // postpone the leaf, keep descending
-                s.leaf = s.node;
-                s.node = trav_pop(s, stack, stack_t);
-            }
-            if (!__any_sync(__activemask(), s.leaf == 0 && s.node != kTravDone)) break;
+// Either slab form in one: box_hit_fma with (sub, add) = (0, ooi), box_hit
+// with (sub, add) = (o, 0), each product and sum as written there.
+LD bool box_hit_sel(float4 bmin, float4 bmax, V3 sub, V3 add, V3 inv, float tmin, float tfar_lim, float& tn) {
+    return box_hit_fma(make_float4(bmin.x - sub.x, bmin.y - sub.y, bmin.z - sub.z, 0.0f),
+                       make_float4(bmax.x - sub.x, bmax.y - sub.y, bmax.z - sub.z, 0.0f), add, inv, tmin, tfar_lim, tn);
+}
+
+// Visits the internal node s.node of the binary tree (if it is one) and takes
+// the next entry where that leaves nothing.  SEL: the slab form is the lane's
+// choice (a camera ray may start outside the scene's coordinate bound): `sub`
+// and s.ooi as box_hit_sel takes them; else the FMA form.
+template <bool SEL = false>
+LD void trav_node(Trav& s, int2* stack, const DevScene& sc, bool& ok, V3 sub = v3(0.f, 0.f, 0.f)) {
+    trav_pop(s, stack);
+    if (trav_inner(s.node)) {
+        const DevNode* n = sc.nodes2 + s.node;
+        float4 a, b, c, e;
+        ldg32(&n->lmin_lc, a, b);
+        ldg32(&n->rmin, c, e);
+        const int cl = __float_as_int(a.w), cr = __float_as_int(b.w);
+        float tl, tr;
+        bool hl, hr;
+        if (SEL) {
+            hl = box_hit_sel(a, b, sub, s.ooi, s.inv, s.tmin, s.h.t, tl);
+            hr = box_hit_sel(c, e, sub, s.ooi, s.inv, s.tmin, s.h.t, tr);
+        } else {
+            hl = box_hit_fma(a, b, s.ooi, s.inv, s.tmin, s.h.t, tl);
+            hr = box_hit_fma(c, e, s.ooi, s.inv, s.tmin, s.h.t, tr);
         }
-        if (s.leaf != 0) {
-            if (ANY) {
-                if (test_leaf_any(sc.bvh_tris, s.leaf, s.o, s.d, s.tmin, s.h.t)) {
-                    s.any_hit = true;
-                    s.node = kTravDone;
-                    s.leaf = 0;
-                    return true;
-                }
-            } else {
-                test_leaf_closest(sc.bvh_tris, s.leaf, s.o, s.d, s.tmin, s.h);
-            }
-            s.leaf = 0;
-        }
-        if (s.node == kTravDone) return true;
+        const bool lfirst = hl && (!hr || tl <= tr);
+        s.node = lfirst ? cl : hr ? cr : kTravPop;
+        if (hl && hr) trav_push(s, stack, lfirst ? cr : cl, lfirst ? tr : tl, ok);
+        trav_settle(s);
     }
-    return false;
+}
+
+// Tests the next triangle of the postponed leaf (closest hit).
+LD void trav_tri(Trav& s, const DevScene& sc) {
+    const int w = ~s.leaf, k = w >> 3, more = w & 7;
+    V3 v0, e1, e2;
+    int prim;
+    load_bvh_tri(sc.bvh_tris, k, v0, e1, e2, prim);
+    float t, u, v;
+    if (isect_tri(s.o, s.d, v0, e1, e2, s.tmin, s.h.t, t, u, v)) {
+        if (t < s.h.t || prim > s.h.prim) { s.h.t = t; s.h.u = u; s.h.v = v; s.h.prim = prim; }
+    }
+    s.leaf = more ? ~(((k + 1) << 3) | (more - 1)) : 0;
+    trav_settle(s);
+}
+
+// Any hit: the same over the 4-wide tree, its stack holding codes only.
+LD void trav_push_any(Trav& s, int* stack, int code, bool& ok) {
+    if (s.sp > 0) {
+        if (s.sp <= kStack) stack[s.sp - 1] = s.top;
+        else ok = false;
+    }
+    s.top = code;
+    ++s.sp;
+}
+LD void trav_pop_any(Trav& s, const int* stack) {
+    while (s.node == kTravPop) {
+        if (s.sp == 0) {
+            s.node = kTravDone;
+            break;
+        }
+        s.node = s.top;
+        if (--s.sp > 0) s.top = stack[s.sp - 1];
+        trav_settle(s);
+    }
+}
+LD void trav_node_any(Trav& s, int* stack, const DevScene& sc, bool& ok) {
+    trav_pop_any(s, stack);
+    if (trav_inner(s.node)) {
+        Node4 q;
+        load_node4(sc.nodes, s.node, q);
+        Hits4 hh;
+        node_hits<true>(q, s.o, s.ooi, s.inv, s.tmin, s.h.t, hh);
+#pragma unroll
+        for (int j = 3; j >= 1; --j)
+            if (hh.n > j) trav_push_any(s, stack, hh.c[j], ok);
+        s.node = hh.n > 0 ? hh.c[0] : kTravPop;
+        trav_settle(s);
+    }
+}
+LD void trav_tri_any(Trav& s, const DevScene& sc) {
+    const int w = ~s.leaf, k = w >> 3, more = w & 7;
+    V3 v0, e1, e2;
+    int prim;
+    load_bvh_tri(sc.bvh_tris, k, v0, e1, e2, prim);
+    float t, u, v;
+    if (isect_tri(s.o, s.d, v0, e1, e2, s.tmin, s.h.t, t, u, v)) {
+        s.any_hit = true;
+        s.leaf = 0;
+        s.node = kTravDone;
+        return;
+    }
+    s.leaf = more ? ~(((k + 1) << 3) | (more - 1)) : 0;
+    trav_settle(s);
+}
+
+// A warp's traversals, stepped together: node visits while at least half of
+// the `active` lanes make one, then triangle tests while a third make one.
+// Every active lane that is not done has a visit or a test to make, so one
+// of the two loops runs unless more lanes are done than the caller waits
+// for; then the larger group steps once.  Every lane of the warp calls it;
+// lanes with nothing to do have node kTravDone, leaf 0.
+//
+// The kernels are bound by instruction issue (62-68 % of the slots), so what
+// counts is the lanes at work per instruction.  Loops that each lane left on
+// its own (7.0 lanes a node visit, 3.8 a triangle test on the 1M-triangle
+// frame) took 56.7 ms for closest hit and 41.9 ms for shadow rays, one step
+// of the larger group at a time 49.5 and 42.5 ms (its votes cost as much as
+// a third of a visit), this 42.7 and 34.5 ms.  Lines of (1/2, 1/3), (1/3,
+// 1/3), (1/4, 1/4), (1/2, 1/2): 42.7, 43.3, 43.5, 43.6 ms.
+template <class Node, class Tri>
+LD void warp_steps(const Trav& s, int active, Node node, Tri tri) {
+    const int tn = max(1, active / 2), tt = max(1, active / 3);
+    bool moved = false;
+    for (;;) {
+        const bool g = trav_inner(s.node);
+        if (__popc(__ballot_sync(0xffffffffu, g)) < tn) break;
+        if (g) node();
+        moved = true;
+        __syncwarp();
+    }
+    for (;;) {
+        const bool g = s.leaf != 0;
+        if (__popc(__ballot_sync(0xffffffffu, g)) < tt) break;
+        if (g) tri();
+        moved = true;
+        __syncwarp();
+    }
+    if (moved) return;
+    const bool g = trav_inner(s.node), l = s.leaf != 0;
+    if (__popc(__ballot_sync(0xffffffffu, g)) >= __popc(__ballot_sync(0xffffffffu, l))) {
+        if (g) node();
+    } else {
+        if (l) tri();
+    }
+    __syncwarp();
+}
+template <bool SEL = false>
+LD void warp_step(Trav& s, int active, int2* stack, const DevScene& sc, bool& ok, V3 sub = v3(0.f, 0.f, 0.f)) {
+    warp_steps(s, active, [&] { trav_node<SEL>(s, stack, sc, ok, sub); }, [&] { trav_tri(s, sc); });
+}
+LD void warp_step_any(Trav& s, int active, int* stack, const DevScene& sc, bool& ok) {
+    warp_steps(s, active, [&] { trav_node_any(s, stack, sc, ok); }, [&] { trav_tri_any(s, sc); });
 }
 
 // Closest boundary-only triangle in [tmin, h.t] over the whole list, one

@@ -53,7 +53,7 @@ struct DevVolume {
 
 // Flattened BVH2 node: both children's boxes inline (64 B).  A child index
 // >= 0 is an internal node; < 0 encodes a leaf ~((start << 3) | (count - 1))
-// over the BVH-ordered triangle array.
+// over the BVH-ordered triangle array.  Read as two 32-byte halves (ldg32).
 struct alignas(16) DevNode {
     float4 lmin_lc;   // left box min xyz, left child (int bits)
     float4 lmax_rc;   // left box max xyz, right child (int bits)
@@ -72,7 +72,7 @@ struct alignas(16) DevNode4 {
 constexpr int kEmptyChild = 0x7fffffff;
 
 struct DevScene {
-    // geometry in BVH order: 3 float4 per triangle (v0 | prim id, e1, e2)
+    // geometry in BVH order: 4 float4 per triangle (v0 | prim id, e1, e2, unused)
     const float4* bvh_tris;
     const DevNode4* nodes;    // 4-wide tree (any-hit queries), root `root`
     const DevNode* nodes2;    // binary tree (closest-hit queries), root `root2`
