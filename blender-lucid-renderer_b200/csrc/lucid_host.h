@@ -2,13 +2,30 @@
 #pragma once
 
 #include <array>
+#include <memory>
+#include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "lucid_types.h"
 #include "../../include/lucid_cuda.h"
 
 namespace lucid {
+
+// A vector whose resize leaves new elements uninitialised: the per-prim arrays
+// are sized once and then filled on all host threads.
+template <class T>
+struct RawAllocator : std::allocator<T> {
+    template <class U>
+    struct rebind { using other = RawAllocator<U>; };
+    template <class U>
+    void construct(U* p) { ::new (static_cast<void*>(p)) U; }
+    template <class U, class... Args>
+    void construct(U* p, Args&&... args) { ::new (static_cast<void*>(p)) U(std::forward<Args>(args)...); }
+};
+template <class T>
+using PrimVec = std::vector<T, RawAllocator<T>>;
 
 // Flattened scene ready for upload.  Triangles are numbered globally in
 // mesh-major order ("prim id"), which is also the reference's hit-order
@@ -17,15 +34,15 @@ struct HostScene {
     int num_meshes = 0;
     int num_prims = 0;
     // per prim
-    std::vector<float4> tri;        // 3 per prim: v0 | prim id bits, e1 = v1 - v0, e2 = v2 - v0
-    std::vector<float4> verts;      // 3 per prim: v0, v1, v2 (bounds for the BVH build)
-    std::vector<int4> prim_info;    // mesh, local tri, light index, smooth
-    std::vector<float4> prim_fn;    // face normal
-    std::vector<float4> prim_vn;    // 3 per prim: vertex normals
-    std::vector<unsigned char> prim_boundary;
+    PrimVec<float4> tri;        // 3 per prim: v0 | prim id bits, e1 = v1 - v0, e2 = v2 - v0
+    PrimVec<float4> verts;      // 3 per prim: v0, v1, v2 (bounds for the BVH build)
+    PrimVec<int4> prim_info;    // mesh, local tri, light index, smooth
+    PrimVec<float4> prim_fn;    // face normal
+    PrimVec<float4> prim_vn;    // 3 per prim: vertex normals
+    PrimVec<unsigned char> prim_boundary;
     std::vector<DevMaterial> materials;
     std::vector<float4> tex_ops;    // node program steps of textured materials
-    std::vector<float4> prim_uv;    // 2 per prim when any mesh has UVs, else empty
+    PrimVec<float4> prim_uv;    // 2 per prim when any mesh has UVs, else empty
     std::vector<DevLight> lights;
     std::vector<float> cdf;
     std::vector<int> light_guide;   // kLightGuide + 1 entries

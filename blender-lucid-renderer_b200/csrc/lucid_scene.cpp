@@ -16,6 +16,7 @@
 #include <map>
 #include <nlohmann/json.hpp>
 #include <stdexcept>
+#include <system_error>
 
 #include <vector_functions.h>
 
@@ -241,24 +242,32 @@ void light_cdf(HostScene& S) {
     }
 }
 
+// A mesh's geometry as its loader holds it (kept alive until the scene is
+// finished) and where its prims start.
+struct MeshSrc {
+    const float* v;      // 3 per vertex
+    const int* t;        // 3 per triangle
+    const float* tn;     // 9 per triangle (vertex normals), ntn triangles' worth
+    const std::array<float, 6>* uv;
+    int nv, nt;
+    size_t ntn, nuv;
+    bool tn_unit;        // the normals are normalised already
+    bool smooth, boundary, emissive;
+    float em[3];
+    int first;
+};
 // Scene assembly shared by the JSON and the array loaders: meshes in order,
 // then the native lights, then SceneLights (emissive triangles first).
 struct Assembly {
+    std::vector<MeshSrc> meshes;
     std::vector<DevLight> emissive_lights;
-    float total = 0.0f;
-    int mesh_index = 0;
 };
 
-// One mesh's material, prims, face/vertex normals and emissive-triangle
-// lights (pybind_renderer.hpp:1346-1503, scene.hpp:214-222,
-// scene_lights.hpp:79-101).  tn: normalised per-triangle vertex normals
-// (used when smooth), or empty.
-void emit_mesh(HostScene& S, Assembly& A, const std::vector<F3>& verts, const std::vector<std::array<int, 3>>& tris,
-               const std::vector<std::array<F3, 3>>& tn, bool has_tn, bool smooth, const float alb_in[3],
-               float metallic, float roughness, const float em_in[3], float transmission, float ior, bool boundary,
-               DevVolume vol, bool vol_has_grid, const std::vector<float>& grid,
-               const std::vector<std::array<float, 6>>& uvs = {}, const NodeMaterial* nm = nullptr) {
-    const int mesh_index = A.mesh_index;
+// One mesh's material and volume (pybind_renderer.hpp:1346-1503); its prims
+// follow in emit_prims.
+void emit_mesh(HostScene& S, Assembly& A, MeshSrc src, const float alb_in[3], float metallic, float roughness,
+               const float em_in[3], float transmission, float ior, DevVolume vol, bool vol_has_grid,
+               const std::vector<float>& grid, const NodeMaterial* nm = nullptr) {
     // use_nodes: every parameter comes from the node graph
     // (getMaterialParams / getEmission, integrator/path_tracer.hpp:45-72)
     float alb[3] = {alb_in[0], alb_in[1], alb_in[2]}, em[3] = {em_in[0], em_in[1], em_in[2]};
@@ -267,78 +276,150 @@ void emit_mesh(HostScene& S, Assembly& A, const std::vector<F3>& verts, const st
         metallic = nm->metallic; roughness = nm->roughness; transmission = nm->transmission; ior = nm->ior;
     }
     const bool textured = nm && (nm->albedo_n > 0 || nm->emission_n > 0);
-    for (const auto& t : tris)
-        for (int k = 0; k < 3; ++k)
-            if (t[k] < 0 || t[k] >= (int)verts.size())
-                throw std::runtime_error("mesh " + std::to_string(mesh_index) + ": triangle index out of range");
     if (vol_has_grid) {
         vol.grid_offset = (long long)S.grid.size();
         S.grid.insert(S.grid.end(), grid.begin(), grid.end());
         S.volumes.push_back(vol);
     }
-    S.num_boundary_meshes += boundary;
-    const bool emissive = is_emissive(em);
-    DevMaterial dm = make_material(alb, metallic, roughness, em, transmission, ior, boundary, textured);
+    S.num_boundary_meshes += src.boundary;
+    DevMaterial dm = make_material(alb, metallic, roughness, em, transmission, ior, src.boundary, textured);
     dm.program.x = nm ? nm->albedo_start : 0;
     dm.program.y = nm ? nm->albedo_n : 0;
     dm.program.z = nm ? nm->emission_start : 0;
     dm.program.w = nm ? nm->emission_n : 0;
     S.materials.push_back(dm);
-    for (size_t ti = 0; ti < tris.size(); ++ti) {
-        const auto& t = tris[ti];
-        F3 a = verts[t[0]], b = verts[t[1]], c = verts[t[2]];
-        F3 e1 = sub(b, a), e2 = sub(c, a);
-        F3 fn = dir_or(cross3(e1, e2), F3{0, 1, 0});
-        int prim = S.num_prims++;
-        S.tri.push_back(f4(a, ibits(prim)));
-        S.tri.push_back(f4(e1, 0.0f));
-        S.tri.push_back(f4(e2, 0.0f));
-        S.verts.push_back(f4(a, 0.0f));
-        S.verts.push_back(f4(b, 0.0f));
-        S.verts.push_back(f4(c, 0.0f));
-        bool sm = has_tn && ti < tn.size() && smooth;
-        int light_index = -1;
-        if (emissive) {
-            float area = std::sqrt(len2(cross3(e1, e2))) * 0.5f;
-            if (area > 1e-6f) {
-                DevLight d;
-                std::memset(&d, 0, sizeof(d));
-                d.pos_type = f4(F3{0, 0, 0}, ibits(LIGHT_EMISSIVE));
-                d.normal_area = f4(fn, area);
-                d.emission_radius = f4(F3{em[0], em[1], em[2]}, 0.0f);
-                d.v0_shape = f4(a, ibits(0));
-                d.v1_cosc = f4(b, 0.0f);
-                d.v2_blend = f4(c, 0.0f);
-                light_index = (int)A.emissive_lights.size();
-                A.emissive_lights.push_back(d);
-                A.total += area;
+    src.emissive = is_emissive(em);
+    for (int c = 0; c < 3; ++c) src.em[c] = em[c];
+    src.first = S.num_prims;
+    S.num_prims += src.nt;
+    A.meshes.push_back(src);
+}
+
+bool index_in_range(const MeshSrc& m, int ti) {
+    for (int k = 0; k < 3; ++k)
+        if (m.t[3 * (size_t)ti + k] < 0 || m.t[3 * (size_t)ti + k] >= m.nv) return false;
+    return true;
+}
+[[noreturn]] void bad_index(size_t mesh) {
+    throw std::runtime_error("mesh " + std::to_string(mesh) + ": triangle index out of range");
+}
+// The first mesh with a triangle index out of range, if any, is the error.
+void check_indices(const Assembly& A) {
+    for (size_t k = 0; k < A.meshes.size(); ++k)
+        for (int ti = 0; ti < A.meshes[k].nt; ++ti)
+            if (!index_in_range(A.meshes[k], ti)) bad_index(k);
+}
+
+// Every mesh's prims, face and vertex normals and UVs (scene.hpp:214-222,
+// pybind_renderer.hpp:1296-1336), written in place by all host threads in
+// pieces of kEmitPiece triangles (a push_back at a time on one thread took
+// 36 of the 83 ms that a 258k-triangle scene takes to load), then the
+// emissive-triangle lights in prim order (scene_lights.hpp:79-101).
+constexpr int kEmitPiece = 4096;
+void emit_prims(HostScene& S, Assembly& A) {
+    const size_t n = (size_t)S.num_prims;
+    bool any_uv = false;
+    for (const MeshSrc& m : A.meshes) any_uv = any_uv || (m.nuv > 0 && m.nt > 0);
+    S.tri.resize(3 * n); S.verts.resize(3 * n); S.prim_info.resize(n); S.prim_fn.resize(n); S.prim_vn.resize(3 * n);
+    S.prim_boundary.resize(n);
+    if (any_uv) S.prim_uv.resize(2 * n);
+    std::vector<std::pair<int, int>> pieces;   // (mesh, first triangle)
+    for (size_t k = 0; k < A.meshes.size(); ++k)
+        for (int ti = 0; ti < A.meshes[k].nt; ti += kEmitPiece) pieces.push_back({(int)k, ti});
+    std::atomic<size_t> next{0};
+    std::atomic<size_t> bad{A.meshes.size()};
+    auto work = [&] {
+        for (size_t w; (w = next.fetch_add(1)) < pieces.size();) {
+            const int k = pieces[w].first;
+            const MeshSrc& m = A.meshes[(size_t)k];
+            const int end = (int)std::min<long long>(m.nt, (long long)pieces[w].second + kEmitPiece);
+            for (int ti = pieces[w].second; ti < end; ++ti) {
+                if (!index_in_range(m, ti)) {
+                    size_t b = bad.load();
+                    while ((size_t)k < b && !bad.compare_exchange_weak(b, (size_t)k)) {}
+                    break;
+                }
+                const int* t = m.t + 3 * (size_t)ti;
+                auto vert = [&](int i) { const float* q = m.v + 3 * (size_t)i; return F3{q[0], q[1], q[2]}; };
+                const F3 a = vert(t[0]), b = vert(t[1]), c = vert(t[2]);
+                const F3 e1 = sub(b, a), e2 = sub(c, a);
+                const F3 fn = dir_or(cross3(e1, e2), F3{0, 1, 0});
+                const size_t p = (size_t)m.first + (size_t)ti;
+                S.tri[3 * p] = f4(a, ibits((int)p));
+                S.tri[3 * p + 1] = f4(e1, 0.0f);
+                S.tri[3 * p + 2] = f4(e2, 0.0f);
+                S.verts[3 * p] = f4(a, 0.0f);
+                S.verts[3 * p + 1] = f4(b, 0.0f);
+                S.verts[3 * p + 2] = f4(c, 0.0f);
+                const bool sm = m.tn && (size_t)ti < m.ntn && m.smooth;
+                int4 pi;
+                pi.x = k; pi.y = ti; pi.z = -1; pi.w = sm ? 1 : 0;
+                S.prim_info[p] = pi;
+                S.prim_fn[p] = f4(fn, 0.0f);
+                for (int j = 0; j < 3; ++j) {
+                    F3 vn = fn;
+                    if (sm) {
+                        const float* q = m.tn + 9 * (size_t)ti + 3 * j;
+                        vn = F3{q[0], q[1], q[2]};
+                        if (!m.tn_unit) vn = dir_or(vn, F3{0, 0, 1});
+                    }
+                    S.prim_vn[3 * p + j] = f4(vn, 0.0f);
+                }
+                S.prim_boundary[p] = m.boundary ? 1 : 0;
+                if (any_uv) {
+                    float4 u0 = {0, 0, 0, 0}, u1 = {0, 0, 0, 0};
+                    if ((size_t)ti < m.nuv) {
+                        const auto& q = m.uv[ti];
+                        u0.x = q[0]; u0.y = q[1]; u0.z = q[2]; u0.w = q[3]; u1.x = q[4]; u1.y = q[5]; u1.z = 1.0f;
+                    }
+                    S.prim_uv[2 * p] = u0;
+                    S.prim_uv[2 * p + 1] = u1;
+                }
             }
         }
-        int4 pi;
-        pi.x = mesh_index; pi.y = (int)ti; pi.z = light_index; pi.w = sm ? 1 : 0;
-        S.prim_info.push_back(pi);
-        S.prim_fn.push_back(f4(fn, 0.0f));
-        for (int k = 0; k < 3; ++k) S.prim_vn.push_back(sm ? f4(tn[ti][k], 0.0f) : f4(fn, 0.0f));
-        S.prim_boundary.push_back(boundary ? 1 : 0);
-        // UVs (pybind_renderer.hpp:1296-1336); dropped in finish_scene when no prim has any
-        float4 u0 = {0, 0, 0, 0}, u1 = {0, 0, 0, 0};
-        if (ti < uvs.size()) {
-            const auto& q = uvs[ti];
-            u0.x = q[0]; u0.y = q[1]; u0.z = q[2]; u0.w = q[3]; u1.x = q[4]; u1.y = q[5]; u1.z = 1.0f;
+    };
+    const unsigned nt = std::max(1u, std::min((unsigned)(pieces.size() / 2), std::thread::hardware_concurrency()));
+    std::vector<std::thread> pool;
+    pool.reserve(nt);
+    for (unsigned t = 1; t < nt; ++t) {
+        try {
+            pool.emplace_back(work);
+        } catch (const std::system_error&) {
+            break;   // no more threads: the ones there are do the work
         }
-        S.prim_uv.push_back(u0);
-        S.prim_uv.push_back(u1);
     }
-    ++A.mesh_index;
+    work();
+    for (auto& t : pool) t.join();
+    if (bad.load() < A.meshes.size()) bad_index(bad.load());
+    for (const MeshSrc& m : A.meshes) {
+        if (!m.emissive) continue;
+        for (int ti = 0; ti < m.nt; ++ti) {
+            const size_t p = (size_t)m.first + (size_t)ti;
+            const F3 e1 = {S.tri[3 * p + 1].x, S.tri[3 * p + 1].y, S.tri[3 * p + 1].z};
+            const F3 e2 = {S.tri[3 * p + 2].x, S.tri[3 * p + 2].y, S.tri[3 * p + 2].z};
+            const float area = std::sqrt(len2(cross3(e1, e2))) * 0.5f;
+            if (!(area > 1e-6f)) continue;
+            DevLight d;
+            std::memset(&d, 0, sizeof(d));
+            d.pos_type = f4(F3{0, 0, 0}, ibits(LIGHT_EMISSIVE));
+            d.normal_area = S.prim_fn[p];
+            d.normal_area.w = area;
+            d.emission_radius = f4(F3{m.em[0], m.em[1], m.em[2]}, 0.0f);
+            d.v0_shape = S.verts[3 * p];
+            d.v0_shape.w = ibits(0);
+            d.v1_cosc = S.verts[3 * p + 1];
+            d.v2_blend = S.verts[3 * p + 2];
+            S.prim_info[p].z = (int)A.emissive_lights.size();
+            A.emissive_lights.push_back(d);
+        }
+    }
 }
 
 // SceneLights: emissive triangles, then native lights; CDF by cumulative
 // area / total (scene_lights.hpp:103-121) and the CDF search guide.
 void finish_scene(HostScene& S, Assembly& A, const std::vector<NativeLight>& native, const float env[3]) {
-    S.num_meshes = A.mesh_index;
-    bool any_uv = false;
-    for (size_t i = 1; i < S.prim_uv.size() && !any_uv; i += 2) any_uv = S.prim_uv[i].z != 0.0f;
-    if (!any_uv) std::vector<float4>().swap(S.prim_uv);
+    S.num_meshes = (int)A.meshes.size();
+    emit_prims(S, A);
     for (int k = 0; k < 3; ++k) S.env[k] = env[k];
     S.lights = A.emissive_lights;
     S.native_start = (int)S.lights.size();
@@ -466,7 +547,8 @@ void read_mesh(const json& mj, MeshIn& M) {
     M.boundary = boundary; M.vol = vol; M.vol_has_grid = vol_has_grid; M.grid = std::move(grid);
 }
 
-// Appends a read mesh (its node programs relocated after the scene's).
+// Appends a read mesh (its node programs relocated after the scene's); M stays
+// alive until the scene is finished.
 void emit_read_mesh(HostScene& S, Assembly& A, MeshIn& M) {
     const int base = (int)S.tex_ops.size() / 2;
     if (M.use_nodes) {
@@ -474,8 +556,21 @@ void emit_read_mesh(HostScene& S, Assembly& A, MeshIn& M) {
         if (M.nm.emission_n) M.nm.emission_start += base;
         S.tex_ops.insert(S.tex_ops.end(), M.ops.begin(), M.ops.end());
     }
-    emit_mesh(S, A, M.verts, M.tris, M.tn, M.has_tn, M.smooth, M.alb, M.metallic, M.roughness, M.em, M.transmission,
-              M.ior, M.boundary, M.vol, M.vol_has_grid, M.grid, M.uvs, M.use_nodes ? &M.nm : nullptr);
+    static_assert(sizeof(F3) == 3 * sizeof(float) && sizeof(std::array<int, 3>) == 3 * sizeof(int), "packed triples");
+    MeshSrc src{};
+    src.v = reinterpret_cast<const float*>(M.verts.data());
+    src.nv = (int)M.verts.size();
+    src.t = reinterpret_cast<const int*>(M.tris.data());
+    src.nt = (int)M.tris.size();
+    src.tn = M.has_tn ? reinterpret_cast<const float*>(M.tn.data()) : nullptr;
+    src.ntn = M.tn.size();
+    src.tn_unit = true;
+    src.uv = M.uvs.data();
+    src.nuv = M.uvs.size();
+    src.smooth = M.smooth;
+    src.boundary = M.boundary;
+    emit_mesh(S, A, src, M.alb, M.metallic, M.roughness, M.em, M.transmission, M.ior, M.vol, M.vol_has_grid, M.grid,
+              M.use_nodes ? &M.nm : nullptr);
 }
 
 // Byte ranges of the elements of the document's top-level "meshes" array
@@ -600,17 +695,28 @@ bool parse_scene_json(const char* text, size_t length, HostScene& S, std::string
         for (const auto& e : errors)
             if (!e.empty()) { err = e; return false; }
     }
+    Assembly A;
     try {
-        Assembly A;
-        if (split) {
-            for (auto& M : parsed) emit_read_mesh(S, A, M);
-        } else if (j.contains("meshes")) {
+        if (!split && j.contains("meshes")) {
+            parsed.reserve(j["meshes"].size());
             for (const auto& mj : j["meshes"]) {
-                MeshIn M;
-                read_mesh(mj, M);
-                emit_read_mesh(S, A, M);
+                parsed.emplace_back();
+                read_mesh(mj, parsed.back());
+                emit_read_mesh(S, A, parsed.back());
             }
+        } else {
+            for (auto& M : parsed) emit_read_mesh(S, A, M);
         }
+    } catch (const std::exception& e) {
+        err = std::string("malformed scene: ") + e.what();
+        try {
+            check_indices(A);   // a mesh before the one that failed
+        } catch (const std::exception& first) {
+            err = std::string("malformed scene: ") + first.what();
+        }
+        return false;
+    }
+    try {
         std::vector<NativeLight> native;
         if (j.contains("native_lights") && j["native_lights"].is_array()) parse_lights(j["native_lights"], native);
         else if (j.contains("lights") && j["lights"].is_array()) parse_lights(j["lights"], native);
@@ -625,6 +731,11 @@ bool parse_scene_json(const char* text, size_t length, HostScene& S, std::string
         finish_scene(S, A, native, env);
     } catch (const std::exception& e) {
         err = std::string("malformed scene: ") + e.what();
+        try {
+            check_indices(A);
+        } catch (const std::exception& first) {
+            err = std::string("malformed scene: ") + first.what();
+        }
         return false;
     }
     return true;
@@ -632,32 +743,16 @@ bool parse_scene_json(const char* text, size_t length, HostScene& S, std::string
 
 bool build_scene_arrays(const LucidSceneDesc& d, HostScene& S, std::string& err) {
     S = HostScene();
+    Assembly A;
     try {
         if (d.num_meshes < 0 || d.num_lights < 0) throw std::runtime_error("negative mesh or light count");
         if ((d.num_meshes > 0 && !d.meshes) || (d.num_lights > 0 && !d.lights))
             throw std::runtime_error("null mesh or light array");
-        Assembly A;
         for (int mi = 0; mi < d.num_meshes; ++mi) {
             const LucidMeshDesc& m = d.meshes[mi];
             if (m.num_vertices < 0 || m.num_triangles < 0) throw std::runtime_error("negative vertex or triangle count");
             if ((m.num_vertices > 0 && !m.vertices) || (m.num_triangles > 0 && !m.triangles))
                 throw std::runtime_error("mesh " + std::to_string(mi) + ": null vertex or triangle array");
-            std::vector<F3> verts((size_t)m.num_vertices);
-            for (int i = 0; i < m.num_vertices; ++i)
-                verts[i] = F3{m.vertices[3 * i], m.vertices[3 * i + 1], m.vertices[3 * i + 2]};
-            std::vector<std::array<int, 3>> tris((size_t)m.num_triangles);
-            for (int i = 0; i < m.num_triangles; ++i)
-                tris[i] = {m.triangles[3 * i], m.triangles[3 * i + 1], m.triangles[3 * i + 2]};
-            std::vector<std::array<F3, 3>> tn;
-            const bool has_tn = m.triangle_normals != nullptr;
-            if (has_tn) {
-                tn.resize((size_t)m.num_triangles);
-                for (int i = 0; i < m.num_triangles; ++i)
-                    for (int k = 0; k < 3; ++k) {
-                        const float* q = m.triangle_normals + 9 * i + 3 * k;
-                        tn[i][k] = dir_or(F3{q[0], q[1], q[2]}, F3{0, 0, 1});
-                    }
-            }
             DevVolume vol;
             std::memset(&vol, 0, sizeof(vol));
             for (int k = 0; k < 3; ++k) {
@@ -689,14 +784,28 @@ bool build_scene_arrays(const LucidSceneDesc& d, HostScene& S, std::string& err)
             }
             const bool present = vol.density > 0.0f || vol_has_grid;
             const bool boundary = present && !m.surface;
-            emit_mesh(S, A, verts, tris, tn, has_tn, m.smooth != 0, m.base_color, m.metallic, m.roughness, m.emission,
-                      m.transmission, m.ior, boundary, vol, vol_has_grid, grid);
+            MeshSrc src{};
+            src.v = m.vertices;
+            src.nv = m.num_vertices;
+            src.t = m.triangles;
+            src.nt = m.num_triangles;
+            src.tn = m.triangle_normals;
+            src.ntn = (size_t)m.num_triangles;
+            src.smooth = m.smooth != 0;
+            src.boundary = boundary;
+            emit_mesh(S, A, src, m.base_color, m.metallic, m.roughness, m.emission, m.transmission, m.ior, vol,
+                      vol_has_grid, grid);
         }
         std::vector<NativeLight> native;
         for (int li = 0; li < d.num_lights; ++li) native.push_back(light_from_desc(d.lights[li]));
         finish_scene(S, A, native, d.environment);
     } catch (const std::exception& e) {
         err = std::string("malformed scene arrays: ") + e.what();
+        try {
+            check_indices(A);   // a mesh before the one that failed
+        } catch (const std::exception& first) {
+            err = std::string("malformed scene arrays: ") + first.what();
+        }
         return false;
     }
     return true;
@@ -769,8 +878,8 @@ uint64_t fnv_bytes(const T* p, size_t n, uint64_t h) {
     for (size_t i = 0; i < n * sizeof(T); ++i) h = (h ^ b[i]) * 1099511628211ull;
     return h;
 }
-template <class T>
-uint64_t fnv_vec(const std::vector<T>& v, uint64_t h) { return fnv_bytes(v.data(), v.size(), h); }
+template <class T, class Al>
+uint64_t fnv_vec(const std::vector<T, Al>& v, uint64_t h) { return fnv_bytes(v.data(), v.size(), h); }
 }  // namespace
 
 uint64_t scene_digest(const HostScene& S) {
