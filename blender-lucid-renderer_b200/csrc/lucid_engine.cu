@@ -67,6 +67,35 @@ struct DBuf {
     void release() { if (p) cudaFree(p); p = nullptr; n = 0; }
 };
 
+// One device allocation handed out in pieces: the temporaries of a BVH build
+// (some thirty arrays; allocating and freeing each took 3 ms a build).
+struct DeviceArena {
+    unsigned char* p = nullptr;
+    size_t used = 0, cap = 0;
+    DeviceArena() = default;
+    DeviceArena(const DeviceArena&) = delete;
+    DeviceArena& operator=(const DeviceArena&) = delete;
+    ~DeviceArena() { if (p) cudaFree(p); }
+    static size_t round(size_t b) { return (b + 255) & ~(size_t)255; }
+    cudaError_t reserve(size_t bytes) {
+        cudaError_t e = cudaMalloc((void**)&p, bytes);
+        if (e == cudaSuccess) cap = bytes; else p = nullptr;
+        return e;
+    }
+    // null, now and from then on, when the arena is exhausted
+    template <class T>
+    T* take(size_t n) {
+        const size_t b = round(std::max<size_t>(1, n) * sizeof(T));
+        if (used + b > cap) {
+            cap = 0;
+            return nullptr;
+        }
+        T* q = reinterpret_cast<T*>(p + used);
+        used += b;
+        return q;
+    }
+};
+
 struct DeviceScene {
     DBuf<float4> bvh_tris, bnd_tris, bnd_box, big_tris, prim_fn, prim_vn, light_bsph;
     DBuf<int4> prim_info;
@@ -2278,32 +2307,36 @@ __global__ void __launch_bounds__(kPlocBlock) k_ploc_nn(const float* cbox, int c
     nn[i] = bj;
 }
 
-// flag[i]: 1 = creates a node (mutual pair, lower index), keep[i]: cluster
-// survives (unmerged, or the lower index of a merged pair).
-__global__ void k_ploc_flags(const int* nn, int count, int* create, int* keep) {
+// flags[i]: high word 1 = creates a node (mutual pair, lower index), low word
+// 1 = the cluster survives (unmerged, or the lower index of a merged pair);
+// one scan sums both.
+__global__ void k_ploc_flags(const int* nn, int count, unsigned long long* flags) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     int j = nn[i];
     bool mutual = j >= 0 && nn[j] == i;
-    create[i] = (mutual && i < j) ? 1 : 0;
-    keep[i] = (!mutual || i < j) ? 1 : 0;
+    flags[i] = ((mutual && i < j) ? 1ull << 32 : 0ull) | ((!mutual || i < j) ? 1ull : 0ull);
 }
 
 // Merges (node id = base + exclusive scan of create) and compacts the
 // clusters (position = exclusive scan of keep) into the other buffers.
-__global__ void k_ploc_merge(const int* cl, const float* cbox, const int* nn, const int* create, const int* keep,
-                             const int* create_pos, const int* keep_pos, int count, int base, int2* child,
-                             float* nbox, int* cnt_node, const int* cnt_leaf, int* cl_out, float* cbox_out) {
+// totals: the nodes created (high word) and the clusters that survive.
+__global__ void k_ploc_merge(const int* cl, const float* cbox, const int* nn, const unsigned long long* flags,
+                             const unsigned long long* pos, int count, int base, int2* child, float* nbox,
+                             int* cnt_node, const int* cnt_leaf, int* cl_out, float* cbox_out,
+                             unsigned long long* totals) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count || !keep[i]) return;
-    int o = keep_pos[i];
-    if (!create[i]) {
+    if (i >= count) return;
+    if (i == count - 1) *totals = pos[i] + flags[i];
+    if (!(flags[i] & 0xffffffffull)) return;
+    int o = (int)(pos[i] & 0xffffffffull);
+    if (!(flags[i] >> 32)) {
         cl_out[o] = cl[i];
         for (int q = 0; q < 6; ++q) cbox_out[6 * (size_t)o + q] = cbox[6 * (size_t)i + q];
         return;
     }
     int j = nn[i];
-    int id = base + create_pos[i];
+    int id = base + (int)(pos[i] >> 32);
     int a = cl[i], b = cl[j];
     child[id] = make_int2(a, b);
     float m[6];
@@ -2354,6 +2387,174 @@ __global__ void k_gather_tris(const float4* tri, const int* sorted_ids, int n, f
     out[4 * k + 3] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
+// ---- the flattened tree's levels, order and 4-wide collapse ----
+constexpr int kTreeLevels = kStack;   // levels of internal nodes a traversal stack allows for
+struct TreeCounts {
+    int error, leaves, leaf_tris, pad;
+    // level l: list[first[l] .. first[l] + count[l]); the same for the 4-wide tree
+    int first[kTreeLevels + 1], count[kTreeLevels + 1];
+    int wide_first[kTreeLevels + 1], wide_count[kTreeLevels + 1];
+};
+constexpr int kHostWords = (sizeof(TreeCounts) + 7) / 8;
+
+LD void node_codes(const DevNode& nd, int c[2]) {
+    c[0] = __float_as_int(nd.lmin_lc.w);
+    c[1] = __float_as_int(nd.lmax_rc.w);
+}
+
+__global__ void k_tree_root(int root, int n, int* list, int* seen, TreeCounts* tc) {
+    if (root < 0 || root >= n - 1) { tc->error = 1; return; }
+    list[0] = root;
+    seen[root] = 0;
+    tc->count[0] = 1;
+}
+
+// Appends the internal children of level l's nodes as level l + 1.  `seen`
+// is -1 for nodes not reached yet.
+__global__ void __launch_bounds__(256) k_tree_level(const DevNode* nodes, int n, int l, int* list, int* seen,
+                                                    TreeCounts* tc) {
+    const int begin = tc->first[l], end = begin + tc->count[l];
+    if (blockIdx.x == 0 && threadIdx.x == 0) tc->first[l + 1] = end;
+    int leaves = 0, tris = 0;
+    for (int i0 = begin + blockIdx.x * 256; i0 < end; i0 += gridDim.x * 256) {
+        const int i = i0 + (int)threadIdx.x;
+        for (int s = 0; s < 2; ++s) {
+            int c = -1;
+            bool inner = false;
+            if (i < end) {
+                int cc[2];
+                node_codes(nodes[list[i]], cc);
+                c = cc[s];
+                if (c < 0) {
+                    const int start = ~c >> 3, count = (~c & 7) + 1;
+                    if (start < 0 || start + count > n) tc->error = 1;
+                    ++leaves;
+                    tris += count;
+                } else if (c >= n - 1 || atomicExch(&seen[c], 0) != -1) {
+                    tc->error = 1;
+                } else {
+                    inner = true;
+                }
+            }
+            const int at = warp_append(&tc->count[l + 1], inner);
+            if (inner) list[end + at] = c;   // each node is reached once: below n - 1
+        }
+    }
+    leaves = __reduce_add_sync(0xffffffffu, leaves);
+    tris = __reduce_add_sync(0xffffffffu, tris);
+    if (lane_id() == 0 && leaves) {
+        atomicAdd(&tc->leaves, leaves);
+        atomicAdd(&tc->leaf_tris, tris);
+    }
+}
+
+// Internal nodes of each subtree, level by level from the last.
+__global__ void __launch_bounds__(256) k_tree_inner(const DevNode* nodes, int l, const int* list, const TreeCounts* tc,
+                                                    int* inner) {
+    const int end = tc->first[l] + tc->count[l];
+    for (int i = tc->first[l] + blockIdx.x * 256 + (int)threadIdx.x; i < end; i += gridDim.x * 256) {
+        int c[2];
+        node_codes(nodes[list[i]], c);
+        inner[list[i]] = 1 + (c[0] >= 0 ? inner[c[0]] : 0) + (c[1] >= 0 ? inner[c[1]] : 0);
+    }
+}
+
+// Depth-first places from the root down, and the nodes written there.
+__global__ void __launch_bounds__(256) k_tree_place(const DevNode* nodes, int l, const int* list, const TreeCounts* tc,
+                                                    const int* inner, int* place, DevNode* out) {
+    const int end = tc->first[l] + tc->count[l];
+    for (int i = tc->first[l] + blockIdx.x * 256 + (int)threadIdx.x; i < end; i += gridDim.x * 256) {
+        DevNode nd = nodes[list[i]];
+        const int p = l == 0 ? 0 : place[list[i]];
+        int c[2];
+        node_codes(nd, c);
+        if (c[0] >= 0) {
+            place[c[0]] = p + 1;
+            nd.lmin_lc.w = __int_as_float(p + 1);
+        }
+        if (c[1] >= 0) {
+            const int q = p + 1 + (c[0] >= 0 ? inner[c[0]] : 0);
+            place[c[1]] = q;
+            nd.lmax_rc.w = __int_as_float(q);
+        }
+        out[p] = nd;
+    }
+}
+
+__global__ void k_wide_root(int root, int* list, TreeCounts* tc) {
+    list[0] = root;
+    tc->wide_count[0] = 1;
+}
+
+// One level of the 4-wide collapse: starting from a node's two children, the
+// internal child with the largest box is replaced by its own two children
+// until there are four (or only leaves).
+__global__ void __launch_bounds__(256) k_wide_level(const DevNode* nodes, int l, int* list, TreeCounts* tc,
+                                                    DevNode4* out) {
+    const int begin = tc->wide_first[l], end = begin + tc->wide_count[l];
+    if (blockIdx.x == 0 && threadIdx.x == 0) tc->wide_first[l + 1] = end;
+    for (int i0 = begin + blockIdx.x * 256; i0 < end; i0 += gridDim.x * 256) {
+        const int i = i0 + (int)threadIdx.x;
+        float4 lo[4], hi[4];
+        int code[4], cnt = 0, inner = 0;
+        if (i < end) {
+            const DevNode nd = nodes[list[i]];
+            int c[2];
+            node_codes(nd, c);
+            lo[0] = nd.lmin_lc; hi[0] = nd.lmax_rc; code[0] = c[0];
+            lo[1] = nd.rmin; hi[1] = nd.rmax; code[1] = c[1];
+            cnt = 2;
+            while (cnt < 4) {
+                int best = -1;
+                double ba = -1.0;
+                for (int k = 0; k < cnt; ++k) {
+                    if (code[k] < 0) continue;
+                    const double dx = (double)hi[k].x - lo[k].x, dy = (double)hi[k].y - lo[k].y,
+                                 dz = (double)hi[k].z - lo[k].z;
+                    const double a = dx * dy + dy * dz + dz * dx;
+                    if (a > ba) { ba = a; best = k; }
+                }
+                if (best < 0) break;
+                const DevNode ch = nodes[code[best]];
+                node_codes(ch, c);
+                lo[best] = ch.lmin_lc; hi[best] = ch.lmax_rc; code[best] = c[0];
+                lo[cnt] = ch.rmin; hi[cnt] = ch.rmax; code[cnt] = c[1];
+                ++cnt;
+            }
+            for (int k = 0; k < cnt; ++k) inner += code[k] >= 0;
+        }
+        // one place range per node, siblings together
+        int before = inner;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, before, o);
+            if ((int)lane_id() >= o) before += y;
+        }
+        const int total = __shfl_sync(0xffffffffu, before, 31);
+        int base = 0;
+        if (lane_id() == 0 && total) base = atomicAdd(&tc->wide_count[l + 1], total);
+        int at = end + __shfl_sync(0xffffffffu, base, 0) + before - inner;
+        if (i >= end) continue;
+        DevNode4 q;
+        float* f[6] = {&q.xmin.x, &q.xmax.x, &q.ymin.x, &q.ymax.x, &q.zmin.x, &q.zmax.x};
+        int out_code[4];
+        for (int k = 0; k < 4; ++k) {
+            const bool used = k < cnt;
+            f[0][k] = used ? lo[k].x : 0.0f; f[1][k] = used ? hi[k].x : 0.0f;
+            f[2][k] = used ? lo[k].y : 0.0f; f[3][k] = used ? hi[k].y : 0.0f;
+            f[4][k] = used ? lo[k].z : 0.0f; f[5][k] = used ? hi[k].z : 0.0f;
+            out_code[k] = !used ? kEmptyChild : code[k];
+            if (used && code[k] >= 0) {
+                list[at] = code[k];
+                out_code[k] = at++;
+            }
+        }
+        q.child = make_int4(out_code[0], out_code[1], out_code[2], out_code[3]);
+        q.pad = make_int4(0, 0, 0, 0);
+        out[i] = q;
+    }
+}
+
 // ---------------------------------------------------------------- Engine
 static inline cudaStream_t S(void* s) { return (cudaStream_t)s; }
 
@@ -2376,6 +2577,7 @@ Engine::~Engine() {
     for (void* e : render_ev_)
         if (e) cudaEventDestroy((cudaEvent_t)e);
     if (host_counts_) cudaFreeHost(host_counts_);
+    if (host_words_) cudaFreeHost(host_words_);
     if (stream_) cudaStreamDestroy(S(stream_));
 }
 
@@ -2613,48 +2815,41 @@ int Engine::upload_scene(HostScene&& hs) {
     return LUCID_OK;
 }
 
-// PLOC rounds on the device; the host reads four integers per round to know
-// the surviving cluster count.  Returns LUCID_OK with root = -1 when the
+// PLOC rounds on the device; the host reads one word per round to know the
+// surviving cluster count.  Returns LUCID_OK with root = -1 when the
 // clustering needs more than kPlocMaxRounds rounds (the caller then builds
 // the Karras tree instead).
-int Engine::build_ploc(const float4* verts, const int* sorted_ids, int n, int2* child, int2* range, float* nbox,
-                       int* slot_ids, int& root) {
+int Engine::build_ploc(void* arena, const float4* verts, const int* sorted_ids, int n, int2* child, int2* range,
+                       float* nbox, int* slot_ids, int& root) {
+    DeviceArena& A = *static_cast<DeviceArena*>(arena);
     constexpr int kPlocMaxRounds = 4096;
     cudaStream_t st = S(stream_);
     root = -1;
-    DBuf<int> cl0, cl1, nn, create, keep, create_pos, keep_pos, cnt_leaf, cnt_node, off_node, leaf_pos;
-    DBuf<float> cb0, cb1;
-    CK(cl0.alloc(n)); CK(cl1.alloc(n)); CK(nn.alloc(n)); CK(create.alloc(n)); CK(keep.alloc(n));
-    CK(create_pos.alloc(n)); CK(keep_pos.alloc(n)); CK(cnt_leaf.alloc(n)); CK(cnt_node.alloc(n - 1));
-    CK(off_node.alloc(n - 1)); CK(leaf_pos.alloc(n)); CK(cb0.alloc((size_t)6 * n)); CK(cb1.alloc((size_t)6 * n));
+    int* cl[2] = {A.take<int>(n), A.take<int>(n)};
+    float* cb[2] = {A.take<float>((size_t)6 * n), A.take<float>((size_t)6 * n)};
+    int *nn = A.take<int>(n), *cnt_leaf = A.take<int>(n), *cnt_node = A.take<int>(n), *off_node = A.take<int>(n),
+        *leaf_pos = A.take<int>(n);
+    unsigned long long *flags = A.take<unsigned long long>(n), *pos = A.take<unsigned long long>(n),
+                       *d_totals = A.take<unsigned long long>(1);
     size_t temp = 0;
-    CK(cub::DeviceScan::ExclusiveSum(nullptr, temp, create.p, create_pos.p, n, st));
-    DBuf<unsigned char> d_temp;
-    CK(d_temp.alloc(temp));
-    k_ploc_init<<<(n + 255) / 256, 256, 0, st>>>(verts, sorted_ids, n, cl0.p, cb0.p, cnt_leaf.p);
-    int* cl[2] = {cl0.p, cl1.p};
-    float* cb[2] = {cb0.p, cb1.p};
+    CK(cub::DeviceScan::ExclusiveSum(nullptr, temp, flags, pos, n, st));
+    unsigned char* d_temp = A.take<unsigned char>(temp);
+    if (!d_temp) return fail(LUCID_ERR_OOM, "BVH build: temporaries exceed their estimate");
+    k_ploc_init<<<(n + 255) / 256, 256, 0, st>>>(verts, sorted_ids, n, cl[0], cb[0], cnt_leaf);
     int cur = 0, count = n, base = 0;
     std::vector<std::pair<int, int>> rounds;
-    int h[4];
     while (count > 1) {
         if ((int)rounds.size() >= kPlocMaxRounds) return LUCID_OK;
-        k_ploc_nn<<<(count + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, st>>>(cb[cur], count, nn.p);
-        k_ploc_flags<<<(count + 255) / 256, 256, 0, st>>>(nn.p, count, create.p, keep.p);
+        k_ploc_nn<<<(count + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, st>>>(cb[cur], count, nn);
+        k_ploc_flags<<<(count + 255) / 256, 256, 0, st>>>(nn, count, flags);
         size_t t1 = temp;
-        CK(cub::DeviceScan::ExclusiveSum(d_temp.p, t1, create.p, create_pos.p, count, st));
-        t1 = temp;
-        CK(cub::DeviceScan::ExclusiveSum(d_temp.p, t1, keep.p, keep_pos.p, count, st));
-        k_ploc_merge<<<(count + 255) / 256, 256, 0, st>>>(cl[cur], cb[cur], nn.p, create.p, keep.p, create_pos.p,
-                                                         keep_pos.p, count, base, child, nbox, cnt_node.p,
-                                                         cnt_leaf.p, cl[cur ^ 1], cb[cur ^ 1]);
+        CK(cub::DeviceScan::ExclusiveSum(d_temp, t1, flags, pos, count, st));
+        k_ploc_merge<<<(count + 255) / 256, 256, 0, st>>>(cl[cur], cb[cur], nn, flags, pos, count, base, child, nbox,
+                                                         cnt_node, cnt_leaf, cl[cur ^ 1], cb[cur ^ 1], d_totals);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(&h[0], create_pos.p + count - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(&h[1], create.p + count - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(&h[2], keep_pos.p + count - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(&h[3], keep.p + count - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(host_words_, d_totals, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        int m = h[0] + h[1], survivors = h[2] + h[3];
+        const int m = (int)(host_words_[0] >> 32), survivors = (int)(host_words_[0] & 0xffffffffull);
         if (m <= 0 || survivors != count - m) return fail(LUCID_ERR_CUDA, "BVH clustering made no progress");
         rounds.push_back({base, m});
         base += m;
@@ -2663,14 +2858,12 @@ int Engine::build_ploc(const float4* verts, const int* sorted_ids, int n, int2* 
     }
     if (base != n - 1) return fail(LUCID_ERR_CUDA, "BVH clustering produced a wrong node count");
     const int r = n - 2;   // the last node created is the root
-    CK(cudaMemsetAsync(off_node.p + r, 0, sizeof(int), st));
+    CK(cudaMemsetAsync(off_node + r, 0, sizeof(int), st));
     for (auto it = rounds.rbegin(); it != rounds.rend(); ++it)
-        k_ploc_offsets<<<(it->second + 255) / 256, 256, 0, st>>>(child, cnt_node.p, it->first, it->second, off_node.p,
-                                                                 leaf_pos.p);
-    k_ploc_finish<<<(n + 255) / 256, 256, 0, st>>>(sorted_ids, leaf_pos.p, n, child, off_node.p, cnt_node.p, range,
-                                                  slot_ids);
+        k_ploc_offsets<<<(it->second + 255) / 256, 256, 0, st>>>(child, cnt_node, it->first, it->second, off_node,
+                                                                 leaf_pos);
+    k_ploc_finish<<<(n + 255) / 256, 256, 0, st>>>(sorted_ids, leaf_pos, n, child, off_node, cnt_node, range, slot_ids);
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(st));
     ploc_rounds_ = (int)rounds.size();
     root = r;
     return LUCID_OK;
@@ -2806,35 +2999,32 @@ int Engine::build_bvh() {
     bvh_nodes_ = 0; bvh_leaves_ = 0; bvh_depth_ = 0;
     if (n == 0) { v.root = v.root2 = 0; v.nodes = nullptr; v.nodes2 = nullptr; v.bvh_tris = nullptr; return LUCID_OK; }
     cudaStream_t st = S(stream_);
-    DBuf<float4> d_tri, d_verts;
-    DBuf<int> d_ids, d_vals, d_vals_sorted, d_parent, d_leaf_parent, d_arrive, d_bounds;
-    DBuf<unsigned long long> d_keys, d_keys_sorted;
-    DBuf<int2> d_child, d_range;
-    DBuf<float> d_nbox;
-    CK(d_tri.alloc(H.tri.size()));
-    CK(cudaMemcpyAsync(d_tri.p, H.tri.data(), H.tri.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
-    CK(d_verts.alloc(H.verts.size()));
-    CK(cudaMemcpyAsync(d_verts.p, H.verts.data(), H.verts.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
-    CK(d_ids.alloc(n));
-    CK(cudaMemcpyAsync(d_ids.p, real.data(), n * sizeof(int), cudaMemcpyHostToDevice, st));
-    CK(d_bounds.alloc(6));
+    if (!host_words_) CK(cudaHostAlloc((void**)&host_words_, kHostWords * sizeof(unsigned long long), cudaHostAllocDefault));
+    size_t sort_temp = 0, scan_temp = 0;
+    CK(cub::DeviceRadixSort::SortPairs(nullptr, sort_temp, (unsigned long long*)nullptr, (unsigned long long*)nullptr,
+                                       (int*)nullptr, (int*)nullptr, n, 0, 63, st));
+    CK(cub::DeviceScan::ExclusiveSum(nullptr, scan_temp, (unsigned long long*)nullptr, (unsigned long long*)nullptr, n, st));
+    // per triangle: ids, keys and values 28, children, ranges, boxes and
+    // slots 44, clustering 92, flattened nodes, levels, subtree sizes and
+    // places 76, the Karras fallback's 12; each array rounded to 256 bytes
+    DeviceArena A;
+    CK(A.reserve((H.tri.size() + H.verts.size()) * sizeof(float4) + (size_t)n * 252 + sort_temp + scan_temp + (64 << 10)));
+    float4 *d_tri = A.take<float4>(H.tri.size()), *d_verts = A.take<float4>(H.verts.size());
+    int *d_ids = A.take<int>(n), *d_vals = A.take<int>(n), *d_vals_sorted = A.take<int>(n), *d_bounds = A.take<int>(6);
+    unsigned long long *d_keys = A.take<unsigned long long>(n), *d_keys_sorted = A.take<unsigned long long>(n);
+    unsigned char* d_temp = A.take<unsigned char>(sort_temp);
+    CK(cudaMemcpyAsync(d_tri, H.tri.data(), H.tri.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(d_verts, H.verts.data(), H.verts.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(d_ids, real.data(), n * sizeof(int), cudaMemcpyHostToDevice, st));
     int init[6] = {0x7fffffff, 0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000, (int)0x80000000};
-    CK(cudaMemcpyAsync(d_bounds.p, init, sizeof(init), cudaMemcpyHostToDevice, st));
-    k_centroid_bounds<<<std::max(1, std::min(4 * num_sms_, (n + 127) / 128)), 128, 0, st>>>(d_verts.p, d_ids.p, n,
-                                                                                             d_bounds.p);
-    CK(d_keys.alloc(n)); CK(d_keys_sorted.alloc(n)); CK(d_vals.alloc(n)); CK(d_vals_sorted.alloc(n));
-    k_morton<<<(n + 255) / 256, 256, 0, st>>>(d_verts.p, d_ids.p, n, d_bounds.p, d_keys.p, d_vals.p);
-    size_t temp = 0;
-    CK(cub::DeviceRadixSort::SortPairs(nullptr, temp, d_keys.p, d_keys_sorted.p, d_vals.p, d_vals_sorted.p, n, 0, 63,
-                                       st));
-    DBuf<unsigned char> d_temp;
-    CK(d_temp.alloc(temp));
-    CK(cub::DeviceRadixSort::SortPairs(d_temp.p, temp, d_keys.p, d_keys_sorted.p, d_vals.p, d_vals_sorted.p, n, 0, 63,
-                                       st));
+    CK(cudaMemcpyAsync(d_bounds, init, sizeof(init), cudaMemcpyHostToDevice, st));
+    k_centroid_bounds<<<std::max(1, std::min(4 * num_sms_, (n + 127) / 128)), 128, 0, st>>>(d_verts, d_ids, n, d_bounds);
+    k_morton<<<(n + 255) / 256, 256, 0, st>>>(d_verts, d_ids, n, d_bounds, d_keys, d_vals);
+    CK(cub::DeviceRadixSort::SortPairs(d_temp, sort_temp, d_keys, d_keys_sorted, d_vals, d_vals_sorted, n, 0, 63, st));
     CK(D.bvh_tris.alloc((size_t)4 * n));
     v.bvh_tris = D.bvh_tris.p;
     if (n <= 4) {
-        k_gather_tris<<<(n + 255) / 256, 256, 0, st>>>(d_tri.p, d_vals_sorted.p, n, D.bvh_tris.p);
+        k_gather_tris<<<(n + 255) / 256, 256, 0, st>>>(d_tri, d_vals_sorted, n, D.bvh_tris.p);
         v.root = leaf_code(0, n);
         v.root2 = v.root;
         v.nodes = nullptr;
@@ -2844,190 +3034,84 @@ int Engine::build_bvh() {
         CK(cudaStreamSynchronize(st));
         return LUCID_OK;
     }
-    CK(d_child.alloc(n - 1)); CK(d_range.alloc(n - 1)); CK(d_nbox.alloc((size_t)6 * (n - 1)));
+    int2 *d_child = A.take<int2>(n), *d_range = A.take<int2>(n);
+    float* d_nbox = A.take<float>((size_t)6 * n);
+    int* d_slot = A.take<int>(n);
     int root = -1;
-    DBuf<int> d_slot;
-    {
-        CK(d_slot.alloc(n));
-        int rc = build_ploc(d_verts.p, d_vals_sorted.p, n, d_child.p, d_range.p, d_nbox.p, d_slot.p, root);
-        if (rc != LUCID_OK) return rc;
-    }
-    const int* slot_ids = root >= 0 ? d_slot.p : d_vals_sorted.p;
-    if (root < 0) {   // Karras LBVH: the fallback when clustering does not converge
-        CK(d_parent.alloc(n - 1)); CK(d_leaf_parent.alloc(n)); CK(d_arrive.alloc(n - 1));
-        CK(cudaMemsetAsync(d_parent.p, 0xff, (n - 1) * sizeof(int), st));   // root's parent = -1
-        CK(cudaMemsetAsync(d_arrive.p, 0, (n - 1) * sizeof(int), st));
-        k_karras<<<(n - 1 + 255) / 256, 256, 0, st>>>(d_keys_sorted.p, n, d_child.p, d_parent.p, d_leaf_parent.p,
-                                                      d_range.p);
-        k_refit<<<(n + 255) / 256, 256, 0, st>>>(d_verts.p, d_vals_sorted.p, n, d_child.p, d_parent.p,
-                                                d_leaf_parent.p, d_arrive.p, d_nbox.p);
+    int rc = build_ploc(&A, d_verts, d_vals_sorted, n, d_child, d_range, d_nbox, d_slot, root);
+    if (rc != LUCID_OK) return rc;
+    const bool ploc = root >= 0;
+    const int* slot_ids = ploc ? d_slot : d_vals_sorted;
+    if (!ploc) {   // Karras LBVH: the fallback when clustering does not converge
+        int *d_parent = A.take<int>(n), *d_leaf_parent = A.take<int>(n), *d_arrive = A.take<int>(n);
+        if (!d_arrive) return fail(LUCID_ERR_OOM, "BVH build: temporaries exceed their estimate");
+        CK(cudaMemsetAsync(d_parent, 0xff, (n - 1) * sizeof(int), st));   // root's parent = -1
+        CK(cudaMemsetAsync(d_arrive, 0, (n - 1) * sizeof(int), st));
+        k_karras<<<(n - 1 + 255) / 256, 256, 0, st>>>(d_keys_sorted, n, d_child, d_parent, d_leaf_parent, d_range);
+        k_refit<<<(n + 255) / 256, 256, 0, st>>>(d_verts, d_vals_sorted, n, d_child, d_parent, d_leaf_parent, d_arrive,
+                                                d_nbox);
         root = 0;
     }
-    k_gather_tris<<<(n + 255) / 256, 256, 0, st>>>(d_tri.p, slot_ids, n, D.bvh_tris.p);
-    DBuf<DevNode>& d_nodes2 = D.nodes2;
-    CK(d_nodes2.alloc(n - 1));
-    float pad = maxabs * 9.5367431640625e-07f + 1e-30f;   // 2^-20 of the scene's coordinate magnitude
-    k_flatten<<<(n - 1 + 255) / 256, 256, 0, st>>>(d_verts.p, slot_ids, n, d_child.p, d_range.p, d_nbox.p, pad,
-                                                  d_nodes2.p);
-    CK(cudaGetLastError());
-    // Reachable node count, leaves and depth (the traversal stack bound).
-    std::vector<DevNode> hn(n - 1);
-    CK(cudaMemcpyAsync(hn.data(), d_nodes2.p, (n - 1) * sizeof(DevNode), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    // The walk also validates the hierarchy before any traversal kernel uses
-    // it: child indices in range, leaf ranges inside the triangle array, and
-    // no node reached twice.
-    // The same walk sums the surface-area cost (node visits + triangle tests
-    // weighted by box area relative to the root's) reported as bvh_sah_.
-    std::vector<std::pair<int, int>> stack{{root, 1}};
-    std::vector<unsigned char> seen(n - 1, 0);
-    int nodes = 0, leaves = 0, depth = 0;
-    long long leaf_tris = 0;
-    auto area = [](const float4& lo, const float4& hi) {
-        double dx = (double)hi.x - lo.x, dy = (double)hi.y - lo.y, dz = (double)hi.z - lo.z;
-        return dx * dy + dy * dz + dz * dx;
-    };
-    double sah = 1.0, root_area = 0.0;
-    {
-        const DevNode& r = hn[root];
-        float4 lo = make_float4(std::min(r.lmin_lc.x, r.rmin.x), std::min(r.lmin_lc.y, r.rmin.y),
-                                std::min(r.lmin_lc.z, r.rmin.z), 0.0f);
-        float4 hi = make_float4(std::max(r.lmax_rc.x, r.rmax.x), std::max(r.lmax_rc.y, r.rmax.y),
-                                std::max(r.lmax_rc.z, r.rmax.z), 0.0f);
-        root_area = std::max(area(lo, hi), 1e-30);
+    k_gather_tris<<<(n + 255) / 256, 256, 0, st>>>(d_tri, slot_ids, n, D.bvh_tris.p);
+    const float pad = maxabs * 9.5367431640625e-07f + 1e-30f;   // 2^-20 of the scene's coordinate magnitude
+    DevNode* d_flat = A.take<DevNode>(n);
+    int *d_list = A.take<int>(n), *d_inner = A.take<int>(n), *d_place = A.take<int>(n);
+    TreeCounts* d_tc = A.take<TreeCounts>(1);
+    if (!d_tc) return fail(LUCID_ERR_OOM, "BVH build: temporaries exceed their estimate");
+    k_flatten<<<(n - 1 + 255) / 256, 256, 0, st>>>(d_verts, slot_ids, n, d_child, d_range, d_nbox, pad, d_flat);
+
+    // Levels of the flattened tree from the root.  The walk also validates
+    // the hierarchy before any traversal kernel uses it: child indices in
+    // range, leaf ranges inside the triangle array, no node reached twice,
+    // every triangle in one leaf.  d_inner (subtree sizes) marks the nodes
+    // reached until it is filled.
+    TreeCounts* const tc = reinterpret_cast<TreeCounts*>(host_words_);
+    CK(cudaMemsetAsync(d_inner, 0xff, (size_t)n * sizeof(int), st));
+    CK(cudaMemsetAsync(d_tc, 0, sizeof(TreeCounts), st));
+    k_tree_root<<<1, 1, 0, st>>>(root, n, d_list, d_inner, d_tc);
+    const int g = num_sms_ * 2;
+    int levels = 0;
+    for (int l = 0; levels == 0 && l < kTreeLevels;) {
+        for (const int end = std::min(kTreeLevels, l + 32); l < end; ++l)   // (levels past the last are empty)
+            k_tree_level<<<g, 256, 0, st>>>(d_flat, n, l, d_list, d_inner, d_tc);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(tc, d_tc, sizeof(TreeCounts), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        if (tc->error) return fail(LUCID_ERR_CUDA, "BVH build produced an invalid hierarchy");
+        while (levels < l && tc->count[levels] > 0) ++levels;
+        if (levels == l) levels = 0;   // more to come
     }
-    while (!stack.empty()) {
-        auto [nd, dep] = stack.back();
-        stack.pop_back();
-        if (nd < 0 || nd >= n - 1 || seen[nd]) return fail(LUCID_ERR_CUDA, "BVH build produced an invalid hierarchy");
-        seen[nd] = 1;
-        ++nodes;
-        depth = std::max(depth, dep);
-        int c[2];
-        std::memcpy(&c[0], &hn[nd].lmin_lc.w, 4);
-        std::memcpy(&c[1], &hn[nd].lmax_rc.w, 4);
-        const double ca[2] = {area(hn[nd].lmin_lc, hn[nd].lmax_rc) / root_area, area(hn[nd].rmin, hn[nd].rmax) / root_area};
-        for (int s = 0; s < 2; ++s) {
-            if (c[s] < 0) {
-                int w = ~c[s], start = w >> 3, count = (w & 7) + 1;
-                if (start < 0 || start + count > n) return fail(LUCID_ERR_CUDA, "BVH leaf out of range");
-                leaf_tris += count;
-                ++leaves;
-                depth = std::max(depth, dep + 1);
-                sah += ca[s] * count;
-            } else {
-                stack.push_back({c[s], dep + 1});
-                sah += ca[s];
-            }
-        }
-    }
-    if (leaf_tris != n) return fail(LUCID_ERR_CUDA, "BVH leaves do not cover every triangle");
-    // Collapse the binary tree into 4-wide nodes: starting from a node's two
-    // children, the internal child with the largest box is replaced by its
-    // own two children until there are four (or only leaves).
-    std::vector<DevNode4> n4;
-    n4.reserve((size_t)nodes / 2 + 1);
-    std::vector<std::pair<int, int>> todo{{root, 0}};   // (binary node, index of its 4-wide node)
-    n4.push_back(DevNode4{});
-    int depth4 = 1;
-    std::vector<int> level4{1};
-    while (!todo.empty()) {
-        auto [bn, idx] = todo.back();
-        todo.pop_back();
-        struct Ch { float4 lo, hi; int code; };
-        Ch ch[4];
-        int cnt = 0;
-        auto children_of = [&](int b, Ch* out) {
-            int c0, c1;
-            std::memcpy(&c0, &hn[b].lmin_lc.w, 4);
-            std::memcpy(&c1, &hn[b].lmax_rc.w, 4);
-            out[0] = {hn[b].lmin_lc, hn[b].lmax_rc, c0};
-            out[1] = {hn[b].rmin, hn[b].rmax, c1};
-        };
-        children_of(bn, ch);
-        cnt = 2;
-        while (cnt < 4) {
-            int best = -1;
-            double ba = -1.0;
-            for (int k = 0; k < cnt; ++k)
-                if (ch[k].code >= 0 && area(ch[k].lo, ch[k].hi) > ba) { ba = area(ch[k].lo, ch[k].hi); best = k; }
-            if (best < 0) break;
-            Ch two[2];
-            children_of(ch[best].code, two);
-            ch[best] = two[0];
-            ch[cnt++] = two[1];
-        }
-        const int my_level = level4[idx];
-        DevNode4 q;
-        float* f[6] = {&q.xmin.x, &q.xmax.x, &q.ymin.x, &q.ymax.x, &q.zmin.x, &q.zmax.x};
-        int codes[4];
-        for (int k = 0; k < 4; ++k) {
-            if (k < cnt) {
-                f[0][k] = ch[k].lo.x; f[1][k] = ch[k].hi.x; f[2][k] = ch[k].lo.y; f[3][k] = ch[k].hi.y;
-                f[4][k] = ch[k].lo.z; f[5][k] = ch[k].hi.z;
-                if (ch[k].code >= 0) {
-                    int ni = (int)n4.size();
-                    n4.push_back(DevNode4{});
-                    level4.push_back(my_level + 1);
-                    depth4 = std::max(depth4, my_level + 1);
-                    todo.push_back({ch[k].code, ni});
-                    codes[k] = ni;
-                } else {
-                    codes[k] = ch[k].code;
-                    depth4 = std::max(depth4, my_level + 1);
-                }
-            } else {
-                for (int a = 0; a < 6; ++a) f[a][k] = 0.0f;
-                codes[k] = kEmptyChild;
-            }
-        }
-        q.child = make_int4(codes[0], codes[1], codes[2], codes[3]);
-        q.pad = make_int4(0, 0, 0, 0);
-        n4[idx] = q;
-    }
-    CK(D.nodes.alloc(n4.size()));
-    CK(cudaMemcpyAsync(D.nodes.p, n4.data(), n4.size() * sizeof(DevNode4), cudaMemcpyHostToDevice, st));
-    CK(cudaStreamSynchronize(st));
+    if (levels == 0 || levels + 1 >= kStack)
+        return fail(LUCID_ERR_OVERFLOW, "BVH depth " + std::to_string(levels + 1) + " exceeds the traversal stack");
+    if (tc->leaf_tris != n) return fail(LUCID_ERR_CUDA, "BVH leaves do not cover every triangle");
+    const int nodes = tc->first[levels - 1] + tc->count[levels - 1], leaves = tc->leaves, depth = levels + 1;
     // Binary nodes in depth-first order (a node, its left subtree, its right
     // subtree; root first): a ray's descent then reads nearby lines, and the
-    // top of the tree shares a few cache lines.
-    {
-        std::vector<int> order(n - 1, -1), stk{root};
-        std::vector<DevNode> dfs;
-        dfs.reserve(nodes);
-        while (!stk.empty()) {
-            int nd = stk.back();
-            stk.pop_back();
-            order[nd] = (int)dfs.size();
-            dfs.push_back(hn[nd]);
-            int c0, c1;
-            std::memcpy(&c0, &hn[nd].lmin_lc.w, 4);
-            std::memcpy(&c1, &hn[nd].lmax_rc.w, 4);
-            if (c1 >= 0) stk.push_back(c1);
-            if (c0 >= 0) stk.push_back(c0);
-        }
-        for (DevNode& d : dfs) {
-            int c0, c1;
-            std::memcpy(&c0, &d.lmin_lc.w, 4);
-            std::memcpy(&c1, &d.lmax_rc.w, 4);
-            if (c0 >= 0) { c0 = order[c0]; std::memcpy(&d.lmin_lc.w, &c0, 4); }
-            if (c1 >= 0) { c1 = order[c1]; std::memcpy(&d.lmax_rc.w, &c1, 4); }
-        }
-        CK(cudaMemcpyAsync(D.nodes2.p, dfs.data(), dfs.size() * sizeof(DevNode), cudaMemcpyHostToDevice, st));
-        CK(cudaStreamSynchronize(st));
-        root = 0;
-    }
+    // top of the tree shares a few cache lines.  Subtree sizes from the last
+    // level up, places from the root down.
+    CK(D.nodes2.alloc((size_t)nodes));
+    for (int l = levels - 1; l >= 0; --l) k_tree_inner<<<g, 256, 0, st>>>(d_flat, l, d_list, d_tc, d_inner);
+    for (int l = 0; l < levels; ++l) k_tree_place<<<g, 256, 0, st>>>(d_flat, l, d_list, d_tc, d_inner, d_place, D.nodes2.p);
+    // 4-wide collapse, a level at a time: node i of the collapse stands for
+    // binary node d_list[i] (the levels' list is done with).
+    CK(D.nodes.alloc((size_t)nodes));
+    k_wide_root<<<1, 1, 0, st>>>(root, d_list, d_tc);
+    for (int l = 0; l < levels; ++l) k_wide_level<<<g, 256, 0, st>>>(d_flat, l, d_list, d_tc, D.nodes.p);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(tc, d_tc, sizeof(TreeCounts), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    int levels4 = 0;
+    while (levels4 < levels && tc->wide_count[levels4] > 0) ++levels4;
+    const int nodes4 = tc->wide_first[levels4 - 1] + tc->wide_count[levels4 - 1], depth4 = levels4 + 1;
     v.nodes = D.nodes.p;
     v.root = 0;
     v.nodes2 = D.nodes2.p;
-    v.root2 = root;
-    bvh_nodes_ = (int)n4.size(); bvh_leaves_ = leaves; bvh_depth_ = depth4; bvh_sah_ = sah;
+    v.root2 = 0;
+    bvh_nodes_ = nodes4; bvh_leaves_ = leaves; bvh_depth_ = depth4;
     if (std::getenv("LUCID_VERBOSE"))
-        std::fprintf(stderr, "[lucid] BVH %s (%d rounds): %d binary nodes, %d leaves, depth %d, SAH cost %.2f; "
-                     "%d 4-wide nodes, depth %d\n",
-                     slot_ids == d_vals_sorted.p ? "lbvh" : "ploc", slot_ids == d_vals_sorted.p ? 0 : ploc_rounds_,
-                     nodes, leaves, depth, sah, (int)n4.size(), depth4);
-    if (3 * (depth4 - 1) >= kStack || depth >= kStack)
+        std::fprintf(stderr, "[lucid] BVH %s (%d rounds): %d binary nodes, %d leaves, depth %d; %d 4-wide nodes, depth %d\n",
+                     ploc ? "ploc" : "lbvh", ploc ? ploc_rounds_ : 0, nodes, leaves, depth, nodes4, depth4);
+    if (3 * (depth4 - 1) >= kStack)
         return fail(LUCID_ERR_OVERFLOW, "BVH depth " + std::to_string(depth) + " exceeds the traversal stack");
     return LUCID_OK;
 }

@@ -147,14 +147,15 @@ private:
     void enqueue_iteration(void* frame_params, int n);
     void job_end_locked();
     int capture_locked(int chunk);
-    int build_ploc(const float4* verts, const int* sorted_ids, int n, int2* child, int2* range, float* nbox,
-                   int* slot_ids, int& root);
+    int build_ploc(void* arena, const float4* verts, const int* sorted_ids, int n, int2* child, int2* range,
+                   float* nbox, int* slot_ids, int& root);
     void free_scene();
 
     int device_ = 0;
     void* stream_ = nullptr;   // cudaStream_t
     void* render_ev_[2] = {nullptr, nullptr};   // cudaEvent_t: start and end of a render call
     int* host_counts_ = nullptr;                // pinned copies of a wave's counters
+    unsigned long long* host_words_ = nullptr;  // pinned: what a BVH build reads back
     int num_sms_ = 0;
     HostScene host_;
     HostCamera cam_;
@@ -178,7 +179,6 @@ private:
     std::string err_;
     LucidRenderStats stats_{};
     int bvh_nodes_ = 0, bvh_leaves_ = 0, bvh_depth_ = 0, num_big_ = 0, ploc_rounds_ = 0;
-    double bvh_sah_ = 0.0;
     // one GPU call at a time per context (the reference's gpu_mutex_); API
     // calls take it through GpuLock, which the async worker yields to
     std::mutex gpu_mu_;
