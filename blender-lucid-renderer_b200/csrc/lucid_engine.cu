@@ -1214,9 +1214,12 @@ static ShadeKernel shade_kernel_batch(int algo) {
 
 // ---------------------------------------------------------------- shading bins
 // The scatter half of the counting sort whose histogram the trace kernels
-// build (bin_class): one atomic per class per warp, paths of a class kept
-// together so neighbouring warps shade the same kind of event.
-constexpr int kBinThreads = 256;
+// build (bin_class): paths of a bin are kept together so neighbouring warps
+// shade the same kind of event.  A block takes kBinTile entries at a time,
+// ranks them within their bins in shared memory and claims each bin's places
+// with one global atomic; with one per bin and warp the few counters most
+// paths go to were what the pass waited for (BINOLD).
+constexpr int kBinThreads = 256, kBinItems = 8, kBinTile = kBinThreads * kBinItems;
 static_assert(kBins % kBinThreads == 0, "bins per scatter thread");
 __global__ void __launch_bounds__(kBinThreads) k_bin_scatter(PathView pv, int* cnt, int identity, int stop,
                                                              const int* qin, int* qb) {
@@ -1247,18 +1250,28 @@ __global__ void __launch_bounds__(kBinThreads) k_bin_scatter(PathView pv, int* c
         for (int j = 0; j < kPer; ++j) base[threadIdx.x * kPer + j] = excl + loc[j];
     }
     __syncthreads();
-    // whole warps iterate together (match/shuffle below need every lane)
-    for (int i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
-        int i = i0 + (int)threadIdx.x;
-        bool act = i < n;
-        int id = act ? (identity ? i : qin[i]) : 0;
-        int c = act ? (int)pv.cls[i] : -1;
-        unsigned peers = __match_any_sync(0xffffffffu, c);
-        int leader = __ffs(peers) - 1;
-        int pos = 0;
-        if (act && (int)lane_id() == leader) pos = atomicAdd(&cnt[8 + kBins + c], __popc(peers));
-        pos = __shfl_sync(0xffffffffu, pos, leader);
-        if (act) qb[base[c] + pos + __popc(peers & lanemask_lt())] = id;
+    __shared__ int h[kBins];
+    for (int i0 = blockIdx.x * kBinTile; i0 < n; i0 += gridDim.x * kBinTile) {
+        for (int b = threadIdx.x; b < kBins; b += kBinThreads) h[b] = 0;
+        __syncthreads();
+        int id[kBinItems], key[kBinItems], rank[kBinItems];
+#pragma unroll
+        for (int j = 0; j < kBinItems; ++j) {
+            const int i = i0 + j * kBinThreads + (int)threadIdx.x;
+            key[j] = i < n ? (int)pv.cls[i] : -1;
+            id[j] = i < n && !identity ? qin[i] : i;
+        }
+#pragma unroll
+        for (int j = 0; j < kBinItems; ++j)
+            if (key[j] >= 0) rank[j] = atomicAdd(&h[key[j]], 1);
+        __syncthreads();
+        for (int b = threadIdx.x; b < kBins; b += kBinThreads)
+            if (h[b]) h[b] = base[b] + atomicAdd(&cnt[8 + kBins + b], h[b]);
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kBinItems; ++j)
+            if (key[j] >= 0) qb[h[key[j]] + rank[j]] = id[j];
+        __syncthreads();
     }
 }
 

@@ -360,7 +360,14 @@ LD void trav_begin(Trav& s, const DevScene& sc, V3 o, V3 d, float tmin, float tm
     }
     if (sc.num_bvh_tris == 0) return;
     s.node = ANY ? sc.root : sc.root2;
-    trav_settle(s);   // the whole BVH may be one leaf
+    if (s.node >= 0) return;
+    if (LIST) {   // the whole BVH is one leaf: as good as listed
+        if (ANY) s.any_hit = test_leaf_any(sc.bvh_tris, s.node, o, d, tmin, tmax);
+        else test_leaf_closest(sc.bvh_tris, s.node, o, d, tmin, s.h);
+        s.node = kTravDone;
+    } else {
+        trav_settle(s);
+    }
 }
 
 LD bool trav_inner(int node) { return (unsigned)node < (unsigned)kTravDone; }   // a node to visit, or kTravPop
