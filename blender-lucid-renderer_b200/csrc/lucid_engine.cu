@@ -827,9 +827,6 @@ struct ShadeResult {
     bool cont, shadow;
     RGB add;      // radiance of the event (zero: none)
 };
-struct NoSync {
-    LD void operator()() const {}
-};
 struct BlockSync {
     LD void operator()() const { __syncthreads(); }
 };
@@ -1490,17 +1487,21 @@ __global__ void __launch_bounds__(128, MINB) k_shadow_lb(DevScene sc0, PathView 
 //
 // What bounds it is the latency of one warp's dependent instructions (a few
 // warps per scheduler, each waiting for its slowest lane), not throughput:
-// 128 registers and four resident blocks per SM, 96x64 1 spp in 204 us of
-// device time against 580 us for the wavefront's 34 launches (80 registers
-// 215 us, 64 registers 215 us; 16, 8, 4 lanes per warp 214, 206, 231 us).
+// 128 registers and four resident blocks per SM (80 registers 5 % slower),
+// the warps of a block in phase as in k_shade (volume 333x207: 625 -> 430 us,
+// 800x600: 477 -> 430 us in here), at least eight lanes a warp (1M-triangle
+// 960x540 frame, the last paths: 1,026 us with all 32, 895 us with 16, 897 us
+// with 4).  96x64 1 spp takes 169 us on the device, against 580 us for the 34
+// launches of a wavefront.
 struct PathsCount {
     int cursor;
     int pad[3];
     unsigned long long segments, shadows;
 };
 
+constexpr int kPathsThreads = 128, kMinLanes = 8;
 template <int ALGO, bool MULTI>
-__global__ void __launch_bounds__(128, 4) k_paths(DevScene sc0, FrameParams f0, PathView pv, const BatchJob* jobs,
+__global__ void __launch_bounds__(kPathsThreads, 512 / kPathsThreads) k_paths(DevScene sc0, FrameParams f0, PathView pv, const BatchJob* jobs,
                                                    int njobs, int slots, int fma0, int depths, int stop,
                                                    PathsCount* cnt) {
     __shared__ int sbase[MULTI ? kMaxBatchPieces : 1];
@@ -1521,7 +1522,10 @@ __global__ void __launch_bounds__(128, 4) k_paths(DevScene sc0, FrameParams f0, 
     }
     int2 stack[kStack];
     Trav s;
-    bool active = false, exhausted = false, ok = true;
+    // few paths are spread over the warps there are: each then waits for fewer
+    // lanes and runs fewer kinds of event
+    const int warps = (int)(gridDim.x * blockDim.x) / 32, lanes = min(32, max(kMinLanes, (slots + warps - 1) / warps));
+    bool active = false, exhausted = (int)lane_id() >= lanes, ok = true;
     int id = 0, sid = 0;
     unsigned nseg = 0, nsh = 0;
     PathRegs ps;
@@ -1579,10 +1583,7 @@ __global__ void __launch_bounds__(128, 4) k_paths(DevScene sc0, FrameParams f0, 
                 }
             }
         }
-        if (__ballot_sync(0xffffffffu, active) == 0) {
-            if (__ballot_sync(0xffffffffu, !exhausted) == 0) break;
-            continue;
-        }
+        if (__syncthreads_or(active || !exhausted) == 0) break;
         const DevScene& sc = scene();
         HitRec h;
         h.t = 1e30f; h.u = h.v = 0.0f; h.prim = -1;
@@ -1644,11 +1645,13 @@ __global__ void __launch_bounds__(128, 4) k_paths(DevScene sc0, FrameParams f0, 
         const ShadeResult r =
             shade_segment<ALGO, false>(sc, active, f0.max_depth, records, pv, id, ps,
                                        make_float4(h.t, h.u, h.v, __int_as_float(h.prim)),
-                                       make_float2(__int_as_float(li), lt), sr, NoSync());
+                                       make_float2(__int_as_float(li), lt), sr, BlockSync());
         result = result + r.add;
         __syncwarp();
         if (r.shadow) {
-            const bool occ = shadowed_skip_boundaries<true>(sc, sr.o, sr.d, sr.len, ok);
+            // (a sample that would add nothing is traced only to be counted)
+            const bool adds = records || sr.inc.r != 0.0f || sr.inc.g != 0.0f || sr.inc.b != 0.0f;
+            const bool occ = adds && shadowed_skip_boundaries<true>(sc, sr.o, sr.d, sr.len, ok);
             if (!occ) result = result + sr.inc;
             ++nsh;
             if (records) {
@@ -3224,7 +3227,7 @@ static WavePlan wave_plan(int device, int sms, int algo, bool guide, int profile
             o[1] = query(w.ks.trace, 128);
             o[2] = query(w.ks.shade, kShadeThreads);
             o[3] = query(w.ks.shadow, 128);
-            o[4] = query(w.paths, 128);
+            o[4] = query(w.paths, kPathsThreads);
             o[0] = batch ? query(k_trace_primary_batch, 128) : query(k_trace_primary_t<false>, 128);
         }
         w.g_trace0 = sms * o[0];
@@ -3301,10 +3304,11 @@ static void enqueue_wave(const WavePlan& w, const DevScene& sc, const FrameParam
         fma0 = m <= sc.coord_bound;
         slots = ((f.tile_w + 7) / 8) * ((f.tile_h + 3) / 4) * 32 * (f.n_wave / std::max(f.npix, 1));
     }
-    if (w.depths == 0) grid = std::min(grid, (slots + 127) / 128);
+    constexpr int kBlockLanes = kMinLanes * kPathsThreads / 32;
+    if (w.depths == 0) grid = std::min(grid, (slots + kBlockLanes - 1) / kBlockLanes);
     cudaMemsetAsync(pc, 0, sizeof(PathsCount), st);
     mark(K_PATHS, w.depths, [&] {
-        w.paths<<<grid, 128, 0, st>>>(sc, f, base, jobs, njobs, slots, fma0, w.depths, w.stop, pc);
+        w.paths<<<grid, kPathsThreads, 0, st>>>(sc, f, base, jobs, njobs, slots, fma0, w.depths, w.stop, pc);
     });
 }
 
