@@ -24,6 +24,7 @@
 #include <condition_variable>
 #include <future>
 #include <cub/cub.cuh>
+#include <thrust/iterator/counting_iterator.h>
 #include <array>
 #include <map>
 #include <mutex>
@@ -63,6 +64,12 @@ struct DBuf {
         cudaError_t e = cudaMalloc(&p, count * sizeof(T));
         if (e == cudaSuccess) n = count; else p = nullptr;
         return e;
+    }
+    // As alloc, keeping an allocation that holds `count` and is at most about
+    // twice as large (contents undefined either way).
+    cudaError_t fit(size_t count) {
+        if (p && n >= count && n <= 2 * count + 4096) return cudaSuccess;
+        return alloc(count);
     }
     void release() { if (p) cudaFree(p); p = nullptr; n = 0; }
 };
@@ -2102,8 +2109,17 @@ __global__ void k_debug(DevScene sc, FrameParams f, int mode, float4* out, int* 
 // 63-bit Morton codes of triangle centroids, radix sort, one thread per
 // internal node, bottom-up refit with arrival counters; subtrees of at most
 // four triangles are collapsed into leaves when the nodes are flattened.
-LD int ord_f(float f) { int i = __float_as_int(f); return i >= 0 ? i : i ^ 0x7fffffff; }
-LD float unord_f(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
+__host__ __device__ __forceinline__ int ord_f(float f) {
+    int i;
+    memcpy(&i, &f, 4);
+    return i >= 0 ? i : i ^ 0x7fffffff;
+}
+__host__ __device__ __forceinline__ float unord_f(int i) {
+    i = i >= 0 ? i : i ^ 0x7fffffff;
+    float f;
+    memcpy(&f, &i, 4);
+    return f;
+}
 LD V3 centroid(const float4* verts, int prim) {
     V3 a = f3(verts[3 * prim]), b = f3(verts[3 * prim + 1]), c = f3(verts[3 * prim + 2]);
     return (a + b + c) * (1.0f / 3.0f);
@@ -2393,15 +2409,91 @@ __global__ void k_ploc_finish(const int* sorted_ids, const int* leaf_pos, int n,
     }
 }
 
-__global__ void k_gather_tris(const float4* tri, const int* sorted_ids, int n, float4* out) {
+// Triangle k of the BVH order: v0 | prim, v1 - v0, v2 - v0.
+__global__ void k_gather_tris(const float4* verts, const int* sorted_ids, int n, float4* out) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    int prim = sorted_ids[k];
-    out[4 * k] = tri[3 * prim];
-    out[4 * k + 1] = tri[3 * prim + 1];
-    out[4 * k + 2] = tri[3 * prim + 2];
-    out[4 * k + 3] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int prim = sorted_ids[k];
+    const float4 a = verts[3 * (size_t)prim], b = verts[3 * (size_t)prim + 1], c = verts[3 * (size_t)prim + 2];
+    out[4 * (size_t)k] = make_float4(a.x, a.y, a.z, __int_as_float(prim));
+    out[4 * (size_t)k + 1] = make_float4(b.x - a.x, b.y - a.y, b.z - a.z, 0.0f);
+    out[4 * (size_t)k + 2] = make_float4(c.x - a.x, c.y - a.y, c.z - a.z, 0.0f);
+    out[4 * (size_t)k + 3] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
+
+// ---- per-prim values the upload leaves to the device ----
+// Face normals as the scene assembly computes them (the same float
+// operations), and each prim's shading class from its mesh's.
+__global__ void k_prim_values(const float4* verts, const int4* info, const unsigned char* mesh_cls, int n, float4* fn,
+                              unsigned char* cls) {
+    int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    const V3 a = f3(verts[3 * (size_t)p]), b = f3(verts[3 * (size_t)p + 1]), c = f3(verts[3 * (size_t)p + 2]);
+    const V3 f = make_dir_or(cross(b - a, c - a), v3(0.f, 1.f, 0.f));
+    fn[p] = make_float4(f.x, f.y, f.z, 0.0f);
+    cls[p] = mesh_cls[info[p].x];
+}
+// Bounds of the prims in the BVH or its list, and the largest coordinate
+// magnitude of all (ordered-int form, starting from +-1e30 and 0).
+struct PrimBounds {
+    int lo[3], hi[3], maxabs;
+    int big;   // candidates found by k_big_candidates
+};
+__global__ void __launch_bounds__(256) k_prim_bounds(const float4* verts, const unsigned char* boundary, int n,
+                                                     PrimBounds* out) {
+    float lo[3] = {1e30f, 1e30f, 1e30f}, hi[3] = {-1e30f, -1e30f, -1e30f}, m = 0.0f;
+    for (int p = blockIdx.x * 256 + (int)threadIdx.x; p < n; p += gridDim.x * 256) {
+        const bool in = !boundary[p];
+        for (int k = 0; k < 3; ++k) {
+            const float4 q = verts[3 * (size_t)p + k];
+            const float c[3] = {q.x, q.y, q.z};
+            for (int a = 0; a < 3; ++a) {
+                m = fmaxf(m, fabsf(c[a]));
+                if (in) { lo[a] = fminf(lo[a], c[a]); hi[a] = fmaxf(hi[a], c[a]); }
+            }
+        }
+    }
+    for (int a = 0; a < 3; ++a) {
+        const int l = __reduce_min_sync(0xffffffffu, ord_f(lo[a])), h = __reduce_max_sync(0xffffffffu, ord_f(hi[a]));
+        if (lane_id() == 0) {
+            atomicMin(&out->lo[a], l);
+            atomicMax(&out->hi[a], h);
+        }
+    }
+    const int mm = __reduce_max_sync(0xffffffffu, ord_f(m));
+    if (lane_id() == 0) atomicMax(&out->maxabs, mm);
+}
+// Prims whose bounding-box diagonal exceeds `thr`: (prim, diagonal), at most
+// cap of them in any order, and how many there are.
+__global__ void k_big_candidates(const float4* verts, const unsigned char* boundary, int n, float thr, int cap,
+                                 PrimBounds* b, int2* out) {
+    int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n || boundary[p]) return;
+    float lo[3] = {1e30f, 1e30f, 1e30f}, hi[3] = {-1e30f, -1e30f, -1e30f};
+    for (int k = 0; k < 3; ++k) {
+        const float4 q = verts[3 * (size_t)p + k];
+        const float c[3] = {q.x, q.y, q.z};
+        for (int a = 0; a < 3; ++a) { lo[a] = fminf(lo[a], c[a]); hi[a] = fmaxf(hi[a], c[a]); }
+    }
+    const float d = sqrtf((hi[0] - lo[0]) * (hi[0] - lo[0]) + (hi[1] - lo[1]) * (hi[1] - lo[1]) +
+                          (hi[2] - lo[2]) * (hi[2] - lo[2]));
+    if (!(d > thr)) return;
+    const int at = atomicAdd(&b->big, 1);
+    if (at < cap) out[at] = make_int2(p, __float_as_int(d));
+}
+// Prims of the BVH: neither boundary-only nor in the list of large ones.
+constexpr int kMaxBig = 32;
+struct InBvh {
+    const unsigned char* boundary;
+    int big[kMaxBig];
+    int nbig;
+    __device__ bool operator()(int p) const {
+        if (boundary[p]) return false;
+        for (int k = 0; k < nbig; ++k)
+            if (big[k] == p) return false;
+        return true;
+    }
+};
 
 // ---- the flattened tree's levels, order and 4-wide collapse ----
 constexpr int kTreeLevels = kStack;   // levels of internal nodes a traversal stack allows for
@@ -2647,9 +2739,11 @@ void Engine::scene_stats_locked(int out8[8]) const {
 
 int Engine::stats(LucidRenderStats* out) const { *out = stats_; return LUCID_OK; }
 
+// The next scene's arrays take the place of the last one's (allocating and
+// freeing some twenty of them took 4 ms a load) unless another engine still
+// uses it or it is an edited version of one.
 void Engine::free_scene() {
-    if (ds_.use_count() > 1) ds_ = std::make_shared<DeviceScene>();   // still used by a sharing engine
-    else ds_->release();
+    if (ds_.use_count() > 1 || ds_->base) ds_ = std::make_shared<DeviceScene>();
     scene_loaded_ = false;
 }
 
@@ -2773,24 +2867,20 @@ int Engine::upload_scene(HostScene&& hs) {
     const HostScene& H = host_;
     // boundary triangles (brute force list) and per-prim shading data
     std::vector<float4> bnd;
-    for (int p = 0; p < H.num_prims; ++p)
+    for (int p = 0; H.num_boundary_meshes > 0 && p < H.num_prims; ++p)
         if (H.prim_boundary[p])
             for (int k = 0; k < 3; ++k) bnd.push_back(H.tri[3 * p + k]);
     auto up = [&](auto& buf, const auto& vec) -> cudaError_t {
-        cudaError_t e = buf.alloc(vec.size());
+        cudaError_t e = buf.fit(vec.size());
         if (e != cudaSuccess) return e;
         if (vec.empty()) return cudaSuccess;
         return cudaMemcpyAsync(buf.p, vec.data(), vec.size() * sizeof(vec[0]), cudaMemcpyHostToDevice, S(stream_));
     };
-    // each prim's shading class for a surface hit (the material part of
-    // bin_class, decided once here instead of per hit)
-    std::vector<unsigned char> cls(H.prim_info.size());
-    for (size_t p = 0; p < cls.size(); ++p) cls[p] = prim_shading_class(H.materials[H.prim_info[p].x]);
     CK(up(D.bnd_tris, bnd));
     CK(up(D.prim_info, H.prim_info));
-    CK(up(D.prim_cls, cls));
-    CK(up(D.prim_fn, H.prim_fn));
     CK(up(D.prim_vn, H.prim_vn));
+    CK(D.prim_fn.fit(H.prim_fn.size()));       // k_prim_values
+    CK(D.prim_cls.fit(H.prim_info.size()));
     CK(up(D.materials, H.materials));
     CK(up(D.tex_ops, H.tex_ops));
     CK(up(D.prim_uv, H.prim_uv));
@@ -2888,34 +2978,53 @@ int Engine::build_ploc(void* arena, const float4* verts, const int* sorted_ids, 
 int Engine::build_bvh() {
     DeviceScene& D = *ds_;
     const HostScene& H = host_;
+    cudaStream_t st = S(stream_);
+    const int np = H.num_prims;
+    if (!host_words_) CK(cudaHostAlloc((void**)&host_words_, kHostWords * sizeof(unsigned long long), cudaHostAllocDefault));
+    size_t sort_temp = 0, scan_temp = 0, select_temp = 0;
+    CK(cub::DeviceRadixSort::SortPairs(nullptr, sort_temp, (unsigned long long*)nullptr, (unsigned long long*)nullptr,
+                                       (int*)nullptr, (int*)nullptr, np, 0, 63, st));
+    CK(cub::DeviceScan::ExclusiveSum(nullptr, scan_temp, (unsigned long long*)nullptr, (unsigned long long*)nullptr, np, st));
+    CK(cub::DeviceSelect::If(nullptr, select_temp, thrust::make_counting_iterator(0), (int*)nullptr, (int*)nullptr, np,
+                             InBvh{}, st));
+    // per triangle: vertices 48, ids, keys, values and flags 29, children,
+    // ranges, boxes and slots 44, clustering 92, flattened nodes, levels,
+    // subtree sizes and places 76, the Karras fallback's 12; each array
+    // rounded to 256 bytes
+    constexpr int kCandidates = 4096;
+    DeviceArena A;
+    CK(A.reserve((size_t)np * 301 + sort_temp + scan_temp + select_temp + H.materials.size() + (128 << 10)));
+    float4* d_verts = A.take<float4>((size_t)3 * np);
+    unsigned char *d_boundary = A.take<unsigned char>(np), *d_mesh_cls = A.take<unsigned char>(H.materials.size());
+    PrimBounds* d_pb = A.take<PrimBounds>(1);
+    int2* d_cand = A.take<int2>(kCandidates);
+    if (!d_cand) return fail(LUCID_ERR_OOM, "BVH build: temporaries exceed their estimate");
+    CK(cudaMemcpyAsync(d_verts, H.verts.data(), H.verts.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(d_boundary, H.prim_boundary.data(), (size_t)np, cudaMemcpyHostToDevice, st));
     // Scene bounds, then split off the largest triangles: at most kMaxBig
     // whose bounding-box diagonal exceeds a quarter of the scene's.
     float lo[3] = {1e30f, 1e30f, 1e30f}, hi[3] = {-1e30f, -1e30f, -1e30f};
     float maxabs = 0.0f;
-    std::vector<float> diag(H.num_prims, 0.0f);
-    for (int p = 0; p < H.num_prims; ++p) {
-        if (H.prim_boundary[p]) continue;
-        float pl[3] = {1e30f, 1e30f, 1e30f}, ph[3] = {-1e30f, -1e30f, -1e30f};
-        for (int k = 0; k < 3; ++k) {
-            const float4& q = H.verts[3 * p + k];
-            const float c[3] = {q.x, q.y, q.z};
-            for (int a = 0; a < 3; ++a) {
-                pl[a] = std::min(pl[a], c[a]); ph[a] = std::max(ph[a], c[a]);
-                maxabs = std::max(maxabs, std::fabs(c[a]));
-            }
-        }
-        for (int a = 0; a < 3; ++a) { lo[a] = std::min(lo[a], pl[a]); hi[a] = std::max(hi[a], ph[a]); }
-        diag[p] = std::sqrt((ph[0] - pl[0]) * (ph[0] - pl[0]) + (ph[1] - pl[1]) * (ph[1] - pl[1]) +
-                            (ph[2] - pl[2]) * (ph[2] - pl[2]));
+    PrimBounds* const pb = reinterpret_cast<PrimBounds*>(host_words_);
+    if (np > 0) {
+        // each prim's shading class for a surface hit (the material part of
+        // bin_class) is decided once here instead of per hit
+        std::vector<unsigned char> mesh_cls(H.materials.size());
+        for (size_t k = 0; k < mesh_cls.size(); ++k) mesh_cls[k] = prim_shading_class(H.materials[k]);
+        CK(cudaMemcpyAsync(d_mesh_cls, mesh_cls.data(), mesh_cls.size(), cudaMemcpyHostToDevice, st));
+        k_prim_values<<<(np + 255) / 256, 256, 0, st>>>(d_verts, D.prim_info.p, d_mesh_cls, np, D.prim_fn.p, D.prim_cls.p);
+        for (int a = 0; a < 3; ++a) { pb->lo[a] = ord_f(lo[a]); pb->hi[a] = ord_f(hi[a]); }
+        pb->maxabs = ord_f(0.0f);
+        pb->big = 0;
+        CK(cudaMemcpyAsync(d_pb, pb, sizeof(PrimBounds), cudaMemcpyHostToDevice, st));
+        k_prim_bounds<<<std::min(4 * num_sms_, (np + 255) / 256), 256, 0, st>>>(d_verts, d_boundary, np, d_pb);
+        CK(cudaMemcpyAsync(pb, d_pb, sizeof(PrimBounds), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        for (int a = 0; a < 3; ++a) { lo[a] = unord_f(pb->lo[a]); hi[a] = unord_f(pb->hi[a]); }
+        maxabs = unord_f(pb->maxabs);
     }
     // secondary-ray origins lie on triangles (boundary ones included) or
     // inside volume boxes: all of them bound the FMA slab test's error
-    for (int p = 0; p < H.num_prims; ++p)
-        if (H.prim_boundary[p])
-            for (int k = 0; k < 3; ++k) {
-                const float4& q = H.verts[3 * p + k];
-                maxabs = std::max(maxabs, std::max(std::fabs(q.x), std::max(std::fabs(q.y), std::fabs(q.z))));
-            }
     for (const DevVolume& vol : H.volumes)
         for (int a = 0; a < 3; ++a)
             maxabs = std::max(maxabs, std::max(std::fabs(vol.wmin[a]), std::fabs(vol.wmax[a])));
@@ -2926,7 +3035,7 @@ int Engine::build_bvh() {
         std::vector<float4> boxes;
         const float bpad = maxabs * 9.5367431640625e-07f + 1e-30f;
         int k = 0;
-        for (int p = 0; p < H.num_prims; ++p) {
+        for (int p = 0; H.num_boundary_meshes > 0 && p < np; ++p) {
             if (!H.prim_boundary[p]) continue;
             const int mesh = H.prim_info[(size_t)p].x;
             bool fresh = boxes.empty();
@@ -2964,7 +3073,7 @@ int Engine::build_bvh() {
             std::memcpy(&boxes[g + 1].w, &count, 4);
         }
         DeviceScene& Db = D;
-        cudaError_t e = Db.bnd_box.alloc(std::max<size_t>(1, boxes.size()));
+        cudaError_t e = Db.bnd_box.fit(std::max<size_t>(1, boxes.size()));
         if (e != cudaSuccess) return fail(LUCID_ERR_OOM, "boundary box allocation failed");
         if (!boxes.empty())
             CK(cudaMemcpyAsync(Db.bnd_box.p, boxes.data(), boxes.size() * sizeof(float4), cudaMemcpyHostToDevice,
@@ -2975,26 +3084,50 @@ int Engine::build_bvh() {
     }
     float sdiag = std::sqrt((hi[0] - lo[0]) * (hi[0] - lo[0]) + (hi[1] - lo[1]) * (hi[1] - lo[1]) +
                             (hi[2] - lo[2]) * (hi[2] - lo[2]));
-    const int kMaxBig = 32;
-    std::vector<int> bigc;
-    for (int p = 0; p < H.num_prims; ++p)
-        if (!H.prim_boundary[p] && diag[p] > 0.25f * sdiag) bigc.push_back(p);
-    std::sort(bigc.begin(), bigc.end(), [&](int a, int b) { return diag[a] > diag[b] || (diag[a] == diag[b] && a < b); });
-    if ((int)bigc.size() > kMaxBig) bigc.resize(kMaxBig);
+    int nonbnd = np;
+    if (H.num_boundary_meshes > 0)
+        for (int p = 0; p < np; ++p) nonbnd -= H.prim_boundary[p] ? 1 : 0;
+    std::vector<std::pair<float, int>> cand;   // (diagonal, prim)
+    if (np > 0) {
+        k_big_candidates<<<(np + 255) / 256, 256, 0, st>>>(d_verts, d_boundary, np, 0.25f * sdiag, kCandidates, d_pb, d_cand);
+        std::vector<int2> found(kCandidates);
+        CK(cudaMemcpyAsync(pb, d_pb, sizeof(PrimBounds), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(found.data(), d_cand, kCandidates * sizeof(int2), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        if (pb->big <= kCandidates) {
+            for (int k = 0; k < pb->big; ++k) {
+                float d;
+                std::memcpy(&d, &found[(size_t)k].y, 4);
+                cand.push_back({d, found[(size_t)k].x});
+            }
+        } else {   // more than the list holds: all of them, on the host
+            for (int p = 0; p < np; ++p) {
+                if (H.prim_boundary[p]) continue;
+                float pl[3] = {1e30f, 1e30f, 1e30f}, ph[3] = {-1e30f, -1e30f, -1e30f};
+                for (int k = 0; k < 3; ++k) {
+                    const float4& q = H.verts[3 * (size_t)p + k];
+                    const float c[3] = {q.x, q.y, q.z};
+                    for (int a = 0; a < 3; ++a) { pl[a] = std::min(pl[a], c[a]); ph[a] = std::max(ph[a], c[a]); }
+                }
+                const float d = std::sqrt((ph[0] - pl[0]) * (ph[0] - pl[0]) + (ph[1] - pl[1]) * (ph[1] - pl[1]) +
+                                          (ph[2] - pl[2]) * (ph[2] - pl[2]));
+                if (d > 0.25f * sdiag) cand.push_back({d, p});
+            }
+        }
+    }
+    std::sort(cand.begin(), cand.end(), [](const auto& a, const auto& b) {
+        return a.first > b.first || (a.first == b.first && a.second < b.second);
+    });
+    if ((int)cand.size() > kMaxBig) cand.resize(kMaxBig);
     // keep at least one triangle in the BVH so tiny scenes still build one
-    int nonbnd = 0;
-    for (int p = 0; p < H.num_prims; ++p) nonbnd += !H.prim_boundary[p];
-    if ((int)bigc.size() == nonbnd) bigc.clear();
-    std::vector<unsigned char> is_big(H.num_prims, 0);
+    if ((int)cand.size() == nonbnd) cand.clear();
+    std::vector<int> bigc;
+    for (const auto& c : cand) bigc.push_back(c.second);
+    std::sort(bigc.begin(), bigc.end());
     std::vector<float4> big;
-    for (int p : bigc) is_big[p] = 1;
-    for (int p = 0; p < H.num_prims; ++p)
-        if (is_big[p]) for (int k = 0; k < 3; ++k) big.push_back(H.tri[3 * p + k]);
-    std::vector<int> real;
-    real.reserve(H.num_prims);
-    for (int p = 0; p < H.num_prims; ++p)
-        if (!H.prim_boundary[p] && !is_big[p]) real.push_back(p);
-    int n = (int)real.size();
+    for (int p : bigc)
+        for (int k = 0; k < 3; ++k) big.push_back(H.tri[3 * (size_t)p + k]);
+    const int n = nonbnd - (int)bigc.size();
     DevScene& v = D.view;
     v.coord_bound = maxabs;
     for (int a = 0; a < 3; ++a) {
@@ -3003,7 +3136,7 @@ int Engine::build_bvh() {
         v.bin_scale[a] = ext > 0.0f ? (float)kCellDim / ext : 0.0f;
     }
     {
-        cudaError_t e = D.big_tris.alloc(big.size());
+        cudaError_t e = D.big_tris.fit(big.size());
         if (e != cudaSuccess) return fail(LUCID_ERR_OOM, "big triangle list allocation failed");
         if (!big.empty())
             CK(cudaMemcpyAsync(D.big_tris.p, big.data(), big.size() * sizeof(float4), cudaMemcpyHostToDevice, S(stream_)));
@@ -3014,33 +3147,25 @@ int Engine::build_bvh() {
     v.num_bvh_tris = n;
     bvh_nodes_ = 0; bvh_leaves_ = 0; bvh_depth_ = 0;
     if (n == 0) { v.root = v.root2 = 0; v.nodes = nullptr; v.nodes2 = nullptr; v.bvh_tris = nullptr; return LUCID_OK; }
-    cudaStream_t st = S(stream_);
-    if (!host_words_) CK(cudaHostAlloc((void**)&host_words_, kHostWords * sizeof(unsigned long long), cudaHostAllocDefault));
-    size_t sort_temp = 0, scan_temp = 0;
-    CK(cub::DeviceRadixSort::SortPairs(nullptr, sort_temp, (unsigned long long*)nullptr, (unsigned long long*)nullptr,
-                                       (int*)nullptr, (int*)nullptr, n, 0, 63, st));
-    CK(cub::DeviceScan::ExclusiveSum(nullptr, scan_temp, (unsigned long long*)nullptr, (unsigned long long*)nullptr, n, st));
-    // per triangle: ids, keys and values 28, children, ranges, boxes and
-    // slots 44, clustering 92, flattened nodes, levels, subtree sizes and
-    // places 76, the Karras fallback's 12; each array rounded to 256 bytes
-    DeviceArena A;
-    CK(A.reserve((H.tri.size() + H.verts.size()) * sizeof(float4) + (size_t)n * 252 + sort_temp + scan_temp + (64 << 10)));
-    float4 *d_tri = A.take<float4>(H.tri.size()), *d_verts = A.take<float4>(H.verts.size());
-    int *d_ids = A.take<int>(n), *d_vals = A.take<int>(n), *d_vals_sorted = A.take<int>(n), *d_bounds = A.take<int>(6);
+    int *d_ids = A.take<int>(n), *d_vals = A.take<int>(n), *d_vals_sorted = A.take<int>(n), *d_bounds = A.take<int>(6),
+        *d_num = A.take<int>(1);
     unsigned long long *d_keys = A.take<unsigned long long>(n), *d_keys_sorted = A.take<unsigned long long>(n);
-    unsigned char* d_temp = A.take<unsigned char>(sort_temp);
-    CK(cudaMemcpyAsync(d_tri, H.tri.data(), H.tri.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(d_verts, H.verts.data(), H.verts.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(d_ids, real.data(), n * sizeof(int), cudaMemcpyHostToDevice, st));
+    unsigned char *d_temp = A.take<unsigned char>(sort_temp), *d_select = A.take<unsigned char>(select_temp);
+    if (!d_select) return fail(LUCID_ERR_OOM, "BVH build: temporaries exceed their estimate");
+    InBvh in_bvh{};
+    in_bvh.boundary = d_boundary;
+    in_bvh.nbig = (int)bigc.size();
+    for (size_t k = 0; k < bigc.size(); ++k) in_bvh.big[k] = bigc[k];
+    CK(cub::DeviceSelect::If(d_select, select_temp, thrust::make_counting_iterator(0), d_ids, d_num, np, in_bvh, st));
     int init[6] = {0x7fffffff, 0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000, (int)0x80000000};
     CK(cudaMemcpyAsync(d_bounds, init, sizeof(init), cudaMemcpyHostToDevice, st));
     k_centroid_bounds<<<std::max(1, std::min(4 * num_sms_, (n + 127) / 128)), 128, 0, st>>>(d_verts, d_ids, n, d_bounds);
     k_morton<<<(n + 255) / 256, 256, 0, st>>>(d_verts, d_ids, n, d_bounds, d_keys, d_vals);
     CK(cub::DeviceRadixSort::SortPairs(d_temp, sort_temp, d_keys, d_keys_sorted, d_vals, d_vals_sorted, n, 0, 63, st));
-    CK(D.bvh_tris.alloc((size_t)4 * n));
+    CK(D.bvh_tris.fit((size_t)4 * n));
     v.bvh_tris = D.bvh_tris.p;
     if (n <= 4) {
-        k_gather_tris<<<(n + 255) / 256, 256, 0, st>>>(d_tri, d_vals_sorted, n, D.bvh_tris.p);
+        k_gather_tris<<<(n + 255) / 256, 256, 0, st>>>(d_verts, d_vals_sorted, n, D.bvh_tris.p);
         v.root = leaf_code(0, n);
         v.root2 = v.root;
         v.nodes = nullptr;
@@ -3068,7 +3193,7 @@ int Engine::build_bvh() {
                                                 d_nbox);
         root = 0;
     }
-    k_gather_tris<<<(n + 255) / 256, 256, 0, st>>>(d_tri, slot_ids, n, D.bvh_tris.p);
+    k_gather_tris<<<(n + 255) / 256, 256, 0, st>>>(d_verts, slot_ids, n, D.bvh_tris.p);
     const float pad = maxabs * 9.5367431640625e-07f + 1e-30f;   // 2^-20 of the scene's coordinate magnitude
     DevNode* d_flat = A.take<DevNode>(n);
     int *d_list = A.take<int>(n), *d_inner = A.take<int>(n), *d_place = A.take<int>(n);
@@ -3105,12 +3230,12 @@ int Engine::build_bvh() {
     // subtree; root first): a ray's descent then reads nearby lines, and the
     // top of the tree shares a few cache lines.  Subtree sizes from the last
     // level up, places from the root down.
-    CK(D.nodes2.alloc((size_t)nodes));
+    CK(D.nodes2.fit((size_t)nodes));
     for (int l = levels - 1; l >= 0; --l) k_tree_inner<<<g, 256, 0, st>>>(d_flat, l, d_list, d_tc, d_inner);
     for (int l = 0; l < levels; ++l) k_tree_place<<<g, 256, 0, st>>>(d_flat, l, d_list, d_tc, d_inner, d_place, D.nodes2.p);
     // 4-wide collapse, a level at a time: node i of the collapse stands for
     // binary node d_list[i] (the levels' list is done with).
-    CK(D.nodes.alloc((size_t)nodes));
+    CK(D.nodes.fit((size_t)nodes));
     k_wide_root<<<1, 1, 0, st>>>(root, d_list, d_tc);
     for (int l = 0; l < levels; ++l) k_wide_level<<<g, 256, 0, st>>>(d_flat, l, d_list, d_tc, D.nodes.p);
     CK(cudaGetLastError());

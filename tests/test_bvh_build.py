@@ -16,6 +16,9 @@ def _triangles(kind, n):
     elif kind == "coincident":   # groups of equal triangles: equal Morton codes and boxes
         c = rng.uniform(-1.0, 1.0, (max(1, n // 7), 1, 3))
         v = (c + rng.uniform(-0.3, 0.3, (max(1, n // 7), 3, 3)))[np.arange(n) % max(1, n // 7)]
+    elif kind == "long":         # every one spans the scene: more than the list of large ones holds
+        a = rng.uniform(-1.0, 1.0, (n, 1, 3))
+        v = np.concatenate([a, -a, a + rng.uniform(-0.02, 0.02, (n, 1, 3))], 1)
     elif kind == "degenerate":   # points and slivers among the others
         v = rng.uniform(-1.0, 1.0, (n, 1, 3)) + rng.uniform(-0.2, 0.2, (n, 3, 3))
         v[::3, 1] = v[::3, 0]
@@ -30,7 +33,8 @@ def _triangles(kind, n):
 
 @pytest.mark.parametrize("kind,n", [("random", 1), ("random", 4), ("random", 5), ("random", 6), ("random", 9),
                                     ("random", 33), ("random", 257), ("random", 4097), ("coincident", 5),
-                                    ("coincident", 700), ("degenerate", 300), ("chain", 900)])
+                                    ("coincident", 700), ("degenerate", 300), ("chain", 900), ("long", 40),
+                                    ("long", 4100)])
 def test_small_and_awkward_trees_match_the_oracle(kind, n):
     import lucid_capi
     import lucid_scenes as ls
@@ -48,3 +52,28 @@ def test_small_and_awkward_trees_match_the_oracle(kind, n):
     for f in ("primary_mesh", "primary_tri", "bounces", "nee_tests", "nee_occluded", "hash"):
         np.testing.assert_array_equal(recs[f], rref[f])
     np.testing.assert_allclose(img, ref, rtol=1e-4, atol=1e-5)
+
+
+def test_a_context_reloads_scenes_of_other_sizes():
+    """One context through scenes that grow and shrink, with and without
+    lights, media and large triangles: each renders as on a context of its
+    own."""
+    import lucid_capi
+    import lucid_scenes as ls
+    from parity_util import render_gpu
+    room, rcam = ls.cornell_variant(3, 5000)
+    v, t = _triangles("random", 60)
+    few = {"meshes": [ls.mesh(v, t, ls.material((0.6, 0.5, 0.4), 0.0, 0.6))], "native_lights": [],
+           "environment": {"color": [0.2, 0.2, 0.3], "strength": 1.0}}
+    fcam = (0.1, 0.15, 3.1, 0.0, -0.02, -1.0, 0.0, 1.0, 0.0, 50.0)
+    lit, lcam = ls.all_lights_scene("/tmp")
+    order = [(room, rcam), (few, fcam), (lit, lcam), (few, fcam), (room, rcam), (lit, lcam)]
+    one = lucid_capi.Context(0)
+    for scene, cam in order:
+        got, grec = render_gpu(one, scene, cam, "volume_mis", 48, 40, 2, 6)
+        own = lucid_capi.Context(0)
+        want, wrec = render_gpu(own, scene, cam, "volume_mis", 48, 40, 2, 6)
+        own.close()
+        np.testing.assert_array_equal(got, want)
+        np.testing.assert_array_equal(grec, wrec)
+    one.close()
