@@ -103,6 +103,42 @@ struct DeviceArena {
     }
 };
 
+// Pinned host memory for what a call reads back (a few kilobytes a context):
+// page-locking a block takes about a millisecond, so up to kPinnedKept blocks
+// that closed contexts gave back are kept for the next ones.
+constexpr size_t kPinnedBytes = 48 << 10;
+constexpr size_t kPinnedKept = 16;
+namespace {
+std::mutex g_pinned_mu;
+std::vector<void*>& pinned_blocks() {
+    static std::vector<void*>* v = new std::vector<void*>();   // (no CUDA call from a static destructor)
+    return *v;
+}
+cudaError_t pinned_take(void** p) {
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        std::vector<void*>& v = pinned_blocks();
+        if (!v.empty()) {
+            *p = v.back();
+            v.pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaHostAlloc(p, kPinnedBytes, cudaHostAllocPortable);
+}
+void pinned_give(void* p) {
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        std::vector<void*>& v = pinned_blocks();
+        if (v.size() < kPinnedKept) {
+            v.push_back(p);
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+}  // namespace
+
 struct DeviceScene {
     DBuf<float4> bvh_tris, bnd_tris, bnd_box, big_tris, prim_fn, prim_vn, light_bsph;
     DBuf<int4> prim_info;
@@ -2503,7 +2539,6 @@ struct TreeCounts {
     int first[kTreeLevels + 1], count[kTreeLevels + 1];
     int wide_first[kTreeLevels + 1], wide_count[kTreeLevels + 1];
 };
-constexpr int kHostWords = (sizeof(TreeCounts) + 7) / 8;
 
 LD void node_codes(const DevNode& nd, int c[2]) {
     c[0] = __float_as_int(nd.lmin_lc.w);
@@ -2684,8 +2719,7 @@ Engine::~Engine() {
     delete diag_dev_;
     for (void* e : render_ev_)
         if (e) cudaEventDestroy((cudaEvent_t)e);
-    if (host_counts_) cudaFreeHost(host_counts_);
-    if (host_words_) cudaFreeHost(host_words_);
+    if (host_block_) pinned_give(host_block_);
     if (stream_) cudaStreamDestroy(S(stream_));
 }
 
@@ -2953,9 +2987,10 @@ int Engine::build_ploc(void* arena, const float4* verts, const int* sorted_ids, 
         k_ploc_merge<<<(count + 255) / 256, 256, 0, st>>>(cl[cur], cb[cur], nn, flags, pos, count, base, child, nbox,
                                                          cnt_node, cnt_leaf, cl[cur ^ 1], cb[cur ^ 1], d_totals);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(host_words_, d_totals, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+        unsigned long long* const word = static_cast<unsigned long long*>(host_block_);
+        CK(cudaMemcpyAsync(word, d_totals, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        const int m = (int)(host_words_[0] >> 32), survivors = (int)(host_words_[0] & 0xffffffffull);
+        const int m = (int)(*word >> 32), survivors = (int)(*word & 0xffffffffull);
         if (m <= 0 || survivors != count - m) return fail(LUCID_ERR_CUDA, "BVH clustering made no progress");
         rounds.push_back({base, m});
         base += m;
@@ -2980,7 +3015,8 @@ int Engine::build_bvh() {
     const HostScene& H = host_;
     cudaStream_t st = S(stream_);
     const int np = H.num_prims;
-    if (!host_words_) CK(cudaHostAlloc((void**)&host_words_, kHostWords * sizeof(unsigned long long), cudaHostAllocDefault));
+    static_assert(sizeof(TreeCounts) <= kPinnedBytes, "what a build reads back");
+    if (!host_block_) CK(pinned_take(&host_block_));
     size_t sort_temp = 0, scan_temp = 0, select_temp = 0;
     CK(cub::DeviceRadixSort::SortPairs(nullptr, sort_temp, (unsigned long long*)nullptr, (unsigned long long*)nullptr,
                                        (int*)nullptr, (int*)nullptr, np, 0, 63, st));
@@ -3005,7 +3041,7 @@ int Engine::build_bvh() {
     // whose bounding-box diagonal exceeds a quarter of the scene's.
     float lo[3] = {1e30f, 1e30f, 1e30f}, hi[3] = {-1e30f, -1e30f, -1e30f};
     float maxabs = 0.0f;
-    PrimBounds* const pb = reinterpret_cast<PrimBounds*>(host_words_);
+    PrimBounds* const pb = static_cast<PrimBounds*>(host_block_);
     if (np > 0) {
         // each prim's shading class for a surface hit (the material part of
         // bin_class) is decided once here instead of per hit
@@ -3206,7 +3242,7 @@ int Engine::build_bvh() {
     // range, leaf ranges inside the triangle array, no node reached twice,
     // every triangle in one leaf.  d_inner (subtree sizes) marks the nodes
     // reached until it is filled.
-    TreeCounts* const tc = reinterpret_cast<TreeCounts*>(host_words_);
+    TreeCounts* const tc = static_cast<TreeCounts*>(host_block_);
     CK(cudaMemsetAsync(d_inner, 0xff, (size_t)n * sizeof(int), st));
     CK(cudaMemsetAsync(d_tc, 0, sizeof(TreeCounts), st));
     k_tree_root<<<1, 1, 0, st>>>(root, n, d_list, d_inner, d_tc);
@@ -3988,8 +4024,9 @@ int Engine::render_impl(const LucidRenderParams& p, float* out_host, LucidSample
     stats_ = LucidRenderStats{};
     double seg = 0, shadows = 0;
     // pinned: the first eight counters of each depth, then the error words
-    if (!host_counts_) CK(cudaHostAlloc((void**)&host_counts_, sizeof(int) * (8 * (kMaxDepth + 1) + kErrorInts), cudaHostAllocDefault));
-    int* const hcnt = host_counts_;
+    static_assert(sizeof(int) * (8 * (kMaxDepth + 1) + kErrorInts) <= kPinnedBytes, "a call's counters");
+    if (!host_block_) CK(pinned_take(&host_block_));
+    int* const hcnt = static_cast<int*>(host_block_);
     int* const herr = hcnt + 8 * (kMaxDepth + 1);
     const bool one_wave = spw >= p.samples;
     std::vector<double> kind_units(K_NUM, 0.0);

@@ -154,8 +154,7 @@ private:
     int device_ = 0;
     void* stream_ = nullptr;   // cudaStream_t
     void* render_ev_[2] = {nullptr, nullptr};   // cudaEvent_t: start and end of a render call
-    int* host_counts_ = nullptr;                // pinned copies of a wave's counters
-    unsigned long long* host_words_ = nullptr;  // pinned: what a BVH build reads back
+    void* host_block_ = nullptr;   // pinned: what a render call or BVH build reads back (used under the GPU lock)
     int num_sms_ = 0;
     HostScene host_;
     HostCamera cam_;
