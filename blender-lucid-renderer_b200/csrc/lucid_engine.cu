@@ -3313,21 +3313,23 @@ int Engine::ensure_pool(long long paths, bool records) {
 }
 
 namespace {
-// Algorithmic bytes per unit of work (compulsory SoA traffic; BVH node and
+// Algorithmic bytes per unit of work (compulsory path traffic: the fields a
+// kernel needs, not the whole 32-byte sectors of their records; BVH node and
 // triangle fetches are scene-dependent and excluded):
 //   trace : ray 32 + queue id 4 + hit 16 + light hit 8
 //           + the hit prim's class 1 and the shading bin 2 (binning)   = 63 / ray
 //   shade : queue 4 + hit 24 + ray 32 + throughput 16 + radiance 16 + rng 16
 //           + prim info/normal 32 + material 48  (reads)
 //           + rng 16 + radiance 16 + throughput 16 + ray 32 + queue 4
-//           + shadow record 48 + shadow queue 4  (writes)           = 340 / path
-//   shadow: queue 4 + shadow record 48 + radiance 16 read + 16 write  = 84 / ray
+//           + shadow record 48, path id inside  (writes)            = 336 / path
+//   shadow: shadow record 48 + queue 4 (first segment to traversal)
+//           + radiance 16 read + 16 write                            = 84 / ray
 //   raygen: rng 16 + ray 32 + throughput 16 + radiance 16            = 80 / path
 //   camera trace (generates its rays): the raygen writes 80 + hit 16
 //           + light hit 8 + prim class 1 + shading bin 2               = 107 / ray
 //   film  : radiance 16 / path + film 32 / pixel
 //   bin   : queue id 4 + shading bin 2 + binned id 4 (scatter)       = 10 / path
-constexpr double kBytesTrace0 = 107, kBytesTrace = 63, kBytesShade = 340, kBytesShadow = 84, kBytesRaygen = 80, kBytesFilm = 16,
+constexpr double kBytesTrace0 = 107, kBytesTrace = 63, kBytesShade = 336, kBytesShadow = 84, kBytesRaygen = 80, kBytesFilm = 16,
                  kBytesBin = 10, kBytesPaths = 80;
 //   paths : prim info/normal 32 + material 48 per segment (the state stays in registers)
 //   guide : queue 4 + hit 24 + ray 32 + raw outputs 160 w              = 220 / path
@@ -3417,7 +3419,7 @@ static WavePlan wave_plan(int device, int sms, int algo, bool guide, int profile
 
 // Launches one wave.  primary(pv, cnt): the camera-ray kernel; infer(depth,
 // pv, cnt, queue): guide inference before a depth's shading; mark(kind,
-// depth, launch): runs each launch (inside profiling events).
+// depth, kernels, launch): runs a step's launches (inside profiling events).
 template <class Primary, class Infer, class Mark>
 static void enqueue_wave(const WavePlan& w, const DevScene& sc, const FrameParams& f, const PathView& base, int* qb,
                          int max_depth, cudaStream_t st, Primary primary, Infer infer, Mark mark,
@@ -3432,11 +3434,11 @@ static void enqueue_wave(const WavePlan& w, const DevScene& sc, const FrameParam
         int* qout = (depth & 1) ? base.q0 : base.q1;
         pv.q0 = qin;
         const int stop = depth == 0 ? -1 : w.stop;
+        const bool traced = jobs || sc.num_bvh_tris > 0;
         if (depth == 0)
-            mark(K_TRACE0, depth, [&] { primary(pv, cnt); });
+            mark(K_TRACE0, depth, 1, [&] { primary(pv, cnt); });
         else
-            mark(K_TRACE, depth, [&] {
-                const int traced = jobs || sc.num_bvh_tris > 0;
+            mark(K_TRACE, depth, 1 + traced, [&] {
                 if (traced) w.ks.trace<<<w.g_trace, 128, 0, st>>>(sc, pv, cnt, stop);
                 const auto post = jobs ? k_trace_post<true> : k_trace_post<false>;
                 post<<<w.g_post, kPostThreads, 0, st>>>(sc, pv, cnt, stop, traced, f.records, w.bins);
@@ -3444,17 +3446,18 @@ static void enqueue_wave(const WavePlan& w, const DevScene& sc, const FrameParam
         infer(depth, pv, cnt, qin);
         int identity = depth == 0;
         if (w.bins >= 0) {
-            mark(K_BIN, depth, [&] { k_bin_scatter<<<w.g_bin, kBinThreads, 0, st>>>(pv, cnt, identity, stop, qin, qb); });
+            mark(K_BIN, depth, 1, [&] { k_bin_scatter<<<w.g_bin, kBinThreads, 0, st>>>(pv, cnt, identity, stop, qin, qb); });
             identity = 0;
         }
-        mark(K_SHADE, depth, [&] {
+        mark(K_SHADE, depth, 1, [&] {
             w.ks.shade<<<w.g_shade, kShadeThreads, 0, st>>>(sc, f, pv, cnt, cnt_next, identity, stop,
                                                             w.bins >= 0 ? qb : qin, qout);
         });
-        mark(K_SHADOW, depth, [&] {
+        const bool any_bvh = jobs || sc.num_bvh_tris > 0 || sc.num_bnd_tris > 0;
+        mark(K_SHADOW, depth, 1 + any_bvh, [&] {
             const auto pre = jobs ? k_shadow_pre<true> : k_shadow_pre<false>;
             pre<<<w.g_post, kPostThreads, 0, st>>>(sc, pv, cnt, f.records);
-            if (jobs || sc.num_bvh_tris > 0 || sc.num_bnd_tris > 0)
+            if (any_bvh)
                 w.ks.shadow<<<w.g_shadow, 128, 0, st>>>(sc, pv, cnt, f.records);
         });
     }
@@ -3468,7 +3471,7 @@ static void enqueue_wave(const WavePlan& w, const DevScene& sc, const FrameParam
     constexpr int kBlockLanes = kMinLanes * kPathsThreads / 32;
     if (w.depths == 0) grid = std::min(grid, (slots + kBlockLanes - 1) / kBlockLanes);
     cudaMemsetAsync(pc, 0, sizeof(PathsCount), st);
-    mark(K_PATHS, w.depths, [&] {
+    mark(K_PATHS, w.depths, 1, [&] {
         w.paths<<<grid, kPathsThreads, 0, st>>>(sc, f, base, jobs, njobs, slots, fma0, w.depths, w.stop, pc);
     });
 }
@@ -3489,8 +3492,8 @@ static void wave_totals(const WavePlan& w, const int* c, const PathsCount& pc, d
 // amortise each persistent kernel's tail (measured on the 1M-triangle
 // frame, samples/s: 4 Mi paths 287 M, 16 Mi 390 M, 64 Mi 429 M, the whole
 // 133 M-path frame 435 M; with the current kernels 64 Mi 608 M against 622 M
-// for the whole frame), so up to 256 Mi paths (43 GB of path state), bounded
-// to a fifth of the free device memory (about 170 bytes per path).
+// for the whole frame), so up to 256 Mi paths (47 GB of path state), bounded
+// to a fifth of the free device memory (about 174 bytes per path).
 long long Engine::default_wave_paths(bool records) const {
     constexpr long long kMaxWave = 1LL << 28;
     // path state 64, hit 32, shadow record 48, radiance 16, three int queues
@@ -4008,7 +4011,7 @@ int Engine::render_impl(const LucidRenderParams& p, float* out_host, LucidSample
             attr = true;
         }
     }
-    struct Launch { int kind; cudaEvent_t a, b; int depth; };
+    struct Launch { int kind; cudaEvent_t a, b; int depth; int kernels = 1; };
     std::vector<Launch> launches;
     auto ev_begin = [&](int kind, int depth) -> int {
         if (!profile) return -1;
@@ -4085,8 +4088,9 @@ int Engine::render_impl(const LucidRenderParams& p, float* out_host, LucidSample
                 ds_->view, pv, cnt, depth == 0, qin, static_cast<const __nv_bfloat16*>(guide_->net.weights_bf16()),
                 guide_->net.master());
             ev_end(k);
-        }, [&](int kind, int depth, auto&& launch) {
+        }, [&](int kind, int depth, int kernels, auto&& launch) {
             const int k = ev_begin(kind, depth);
+            if (k >= 0) launches[(size_t)k].kernels = kernels;
             launch();
             ev_end(k);
         });
@@ -4167,7 +4171,7 @@ int Engine::render_impl(const LucidRenderParams& p, float* out_host, LucidSample
         for (auto& l : launches) {
             float ms = 0.0f;
             cudaEventElapsedTime(&ms, l.a, l.b);
-            stats_.kinds[l.kind].launches += 1;
+            stats_.kinds[l.kind].launches += l.kernels;
             stats_.kinds[l.kind].total_ms += ms;
             cudaEventDestroy(l.a);
             cudaEventDestroy(l.b);
@@ -4190,7 +4194,7 @@ static int algo_from_name(const char* name) {
 }
 
 long long Engine::batch_bytes(long long pixels, long long wave_paths) {
-    // path state (170 B) and scene index (2 B) per path with slack, film and
+    // path state (174 B) and scene index (2 B) per path with slack, film and
     // output per pixel, the job and scene tables
     return wave_paths * 178 + pixels * 32 + (2 << 20);
 }
@@ -4354,7 +4358,7 @@ int Engine::render_batch(const BatchItem* items, int n, const char* algorithm, l
         pv.sid = P.sid.p;
         enqueue_wave(w, scene_tab[0], fshade, pv, P.qb.p, depth, st, [&](const PathView& v, int* cnt) {
             k_trace_primary_batch<<<w.g_trace0, 128, 0, st>>>(v, d_jobs, (int)tab.size(), (int)slots, n_wave, cnt, w.bins);
-        }, [](int, const PathView&, int*, const int*) {}, [](int, int, auto&& launch) { launch(); },
+        }, [](int, const PathView&, int*, const int*) {}, [](int, int, int, auto&& launch) { launch(); },
         d_jobs, (int)tab.size(), (int)slots);
         for (const PieceFilm& pf : films) {
             const int np_j = (int)(film_off[(size_t)pf.job + 1] - film_off[(size_t)pf.job]);
@@ -4485,7 +4489,7 @@ struct JobState {
 
 long long Engine::job_bytes(int w, int h, int chunk) {
     const long long np = (long long)w * h;
-    return (long long)chunk * np * 176 + np * 32 + (1 << 20);   // path state (170 B) with slack
+    return (long long)chunk * np * 176 + np * 32 + (1 << 20);   // path state (174 B) with slack
 }
 
 void Engine::enqueue_iteration(void* fp, int n) {
@@ -4500,7 +4504,7 @@ void Engine::enqueue_iteration(void* fp, int n) {
     if (w.depths > 0) cudaMemsetAsync(P.counters.p, 0, sizeof(int) * kCountersPerDepth * (w.depths + 1), st);
     enqueue_wave(w, ds_->view, f, P.view, P.qb.p, J.depth, st, [&](const PathView& pv, int* cnt) {
         k_trace_primary_for(ds_->view, f.pos)<<<w.g_trace0, 128, 0, st>>>(ds_->view, f, pv, cnt, 0, w.bins);
-    }, [](int, const PathView&, int*, const int*) {}, [](int, int, auto&& launch) { launch(); });
+    }, [](int, const PathView&, int*, const int*) {}, [](int, int, int, auto&& launch) { launch(); });
     k_film<<<(f.npix + 255) / 256, 256, 0, st>>>(f.npix, n, P.rad.p, P.film.p);
 }
 
@@ -4967,7 +4971,7 @@ int Engine::render_noalloc(const LucidRenderParams& p, float* d_out) {
         if (w.depths > 0) CK(cudaMemsetAsync(v.counters, 0, sizeof(int) * kCountersPerDepth * (w.depths + 1), st));
         enqueue_wave(w, ds_->view, f, v, nullptr, p.max_depth, st, [&](const PathView& pv, int* cnt) {
             k_trace_primary_for(ds_->view, f.pos)<<<w.g_trace0, 128, 0, st>>>(ds_->view, f, pv, cnt, 0, -1);
-        }, [](int, const PathView&, int*, const int*) {}, [](int, int, auto&& launch) { launch(); });
+        }, [](int, const PathView&, int*, const int*) {}, [](int, int, int, auto&& launch) { launch(); });
         k_film<<<(f.npix + 255) / 256, 256, 0, st>>>(f.npix, this_spw, v.rad, film);
         CK(cudaGetLastError());
         // no wait here: stream order keeps the next wave behind this film sum
