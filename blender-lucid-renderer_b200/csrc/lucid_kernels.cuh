@@ -113,6 +113,19 @@ LD bool test_leaf_any(const float4* tris, int code, V3 o, V3 d, float tmin, floa
     return false;
 }
 
+// Reciprocal direction for the slab tests, finite for every finite direction:
+// the FMA form below needs it.  With 1/0 = inf it computes -o*inf + b*inf, for a
+// box on both sides of the coordinate 0 NaN at one plane and an infinity of the
+// wrong sign at the other, so that a ray inside the slab missed the box: rays
+// to a sun straight overhead passed through whatever stands over a coordinate
+// plane, and the centre column of an unjittered camera along an axis was empty.
+// A component below 2^-60 counts as 2^-60 of its sign: over the distances a hit
+// can have that moves the ray by far less than the boxes' padding, and products
+// with coordinates up to 2^67 stay finite.  The reciprocals of all other
+// components keep their bits; the triangle test takes the direction itself.
+LD float slab_inv(float d) { return 1.0f / copysignf(fmaxf(fabsf(d), 8.673617379884035e-19f), d); }
+LD V3 slab_inv(V3 d) { return v3(slab_inv(d.x), slab_inv(d.y), slab_inv(d.z)); }
+
 // Conservative slab test of one box; returns entry distance in tn.
 LD bool box_hit(float4 bmin, float4 bmax, V3 o, V3 inv, float tmin, float tfar_lim, float& tn) {
     float tx0 = (bmin.x - o.x) * inv.x, tx1 = (bmax.x - o.x) * inv.x;
@@ -151,8 +164,8 @@ LD bool list_any(const float4* tris, int count, V3 o, V3 d, float tmin, float tm
 // secondary and shadow ray): t = b*inv - o*inv with one fused rounding.  Its
 // absolute error, about 5 * max|coordinate| * 2^-24 in distance units, is
 // 16x below the 2^-20 * max|coordinate| padding of every BVH box, so the
-// test stays conservative.  Camera rays, whose origin can be far outside the
-// scene, use box_hit above.
+// test stays conservative (inv: slab_inv, finite).  Camera rays, whose origin
+// can be far outside the scene, use box_hit above.
 LD bool box_hit_fma(float4 bmin, float4 bmax, V3 ooi, V3 inv, float tmin, float tfar_lim, float& tn) {
     float tx0 = __fmaf_rn(bmin.x, inv.x, ooi.x), tx1 = __fmaf_rn(bmax.x, inv.x, ooi.x);
     float ty0 = __fmaf_rn(bmin.y, inv.y, ooi.y), ty1 = __fmaf_rn(bmax.y, inv.y, ooi.y);
@@ -254,7 +267,7 @@ LD bool bvh_closest(const DevScene& sc, V3 o, V3 d, float tmin, HitRec& h) {
     if (sc.num_big_tris) list_closest(sc.big_tris, sc.num_big_tris, o, d, tmin, h);
     if (sc.num_bvh_tris == 0) return true;
     if (sc.root2 < 0) { test_leaf_closest(sc.bvh_tris, sc.root2, o, d, tmin, h); return true; }
-    V3 inv = v3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+    const V3 inv = slab_inv(d);
     const V3 ooi = v3(-o.x * inv.x, -o.y * inv.y, -o.z * inv.z);
     int2 stack[kStack];   // (code, entry distance)
     int sp = 0;
@@ -308,7 +321,7 @@ LD bool bvh_any(const DevScene& sc, V3 o, V3 d, float tmin, float tmax, bool& ok
     if (sc.num_big_tris && list_any(sc.big_tris, sc.num_big_tris, o, d, tmin, tmax)) return true;
     if (sc.num_bvh_tris == 0) return false;
     if (sc.root < 0) return test_leaf_any(sc.bvh_tris, sc.root, o, d, tmin, tmax);
-    V3 inv = v3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+    const V3 inv = slab_inv(d);
     const V3 ooi = v3(-o.x * inv.x, -o.y * inv.y, -o.z * inv.z);
     int stack[kStack];
     int sp = 0;
@@ -371,7 +384,7 @@ LD void trav_none(Trav& s) {
 template <bool ANY, bool LIST = true>
 LD void trav_begin(Trav& s, const DevScene& sc, V3 o, V3 d, float tmin, float tmax) {
     s.o = o; s.d = d;
-    s.inv = v3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+    s.inv = slab_inv(d);
     s.ooi = v3(-o.x * s.inv.x, -o.y * s.inv.y, -o.z * s.inv.z);
     s.tmin = tmin;
     s.h.t = tmax; s.h.u = 0.0f; s.h.v = 0.0f; s.h.prim = -1;
