@@ -415,12 +415,17 @@ LD void trav_begin(Trav& s, const DevScene& sc, V3 o, V3 d, float tmin, float tm
 
 LD bool trav_done(const Trav& s) { return s.node == kTravDone && s.leaf == 0; }
 
+// Full: the top entry in registers and kStack below it; an entry more is
+// dropped (a hit may be missed), so a pop never reads past the stack.
+LD bool trav_full(const Trav& s) { return s.sp > kStack; }
+
 // Closest hit.  Stack entries are (code, entry distance).
 LD void trav_push(Trav& s, int2* stack, int code, float t, bool& ok) {
-    if (s.sp > 0) {
-        if (s.sp <= kStack) stack[s.sp - 1] = make_int2(s.top, __float_as_int(s.top_t));
-        else ok = false;
+    if (trav_full(s)) {
+        ok = false;
+        return;
     }
+    if (s.sp > 0) stack[s.sp - 1] = make_int2(s.top, __float_as_int(s.top_t));
     s.top = code;
     s.top_t = t;
     ++s.sp;
@@ -502,10 +507,11 @@ LD void trav_tri(Trav& s, const DevScene& sc) {
 
 // Any hit: the same over the 4-wide tree, its stack holding codes only.
 LD void trav_push_any(Trav& s, int* stack, int code, bool& ok) {
-    if (s.sp > 0) {
-        if (s.sp <= kStack) stack[s.sp - 1] = s.top;
-        else ok = false;
+    if (trav_full(s)) {
+        ok = false;
+        return;
     }
+    if (s.sp > 0) stack[s.sp - 1] = s.top;
     s.top = code;
     ++s.sp;
 }

@@ -1,5 +1,6 @@
 """The traversal code of the CUDA kernels compiled for the host
-(traversal_host.cpp): the box tests against the exact slab test in 64 bits."""
+(traversal_host.cpp): the box tests against the exact slab test in 64 bits, and
+the traversal stack at and past its capacity."""
 import ctypes
 import os
 import shutil
@@ -71,3 +72,17 @@ def test_box_tests_never_lose_a_box_the_ray_meets(host, scale, zeros):
         assert not (meets & (g == 0)).any()
         # and it rejects: at most the margins' share of the boxes beside the ray
         assert ((g != 0) & ~meets).mean() < 0.02
+
+
+@pytest.mark.parametrize("any_hit", [0, 1])
+@pytest.mark.parametrize("extra", [-90, -1, 0, 1, 2, 40])
+def test_stack_at_and_past_its_capacity(host, any_hit, extra):
+    # the top entry is in registers: kStack + 1 entries fit, what comes after is
+    # dropped and reported, and no pop reads past the stack
+    room = host.host_stack_size() + 1
+    pushes = room + extra
+    codes, ok = (ctypes.c_int * 1024)(), ctypes.c_int()
+    n = host.host_push_pop(any_hit, pushes, 0x7eadbee, codes, ctypes.byref(ok))
+    kept = min(pushes, room)
+    assert list(codes[:n]) == list(range(kept, 0, -1))
+    assert bool(ok.value) == (pushes <= room)

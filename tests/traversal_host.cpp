@@ -46,3 +46,38 @@ extern "C" void host_box_tests(int n, const float* o, const float* d, const floa
         sub_form[k] = box_hit(a, b, O, s.inv, tmin, tmax, tn);
     }
 }
+
+// Pushes `pushes` entries (codes 1, 2, ...) on a query's stack and pops until
+// it is done, on a stack of kStack entries followed by `canary`: the codes
+// popped, in order, go to `codes`.  Returns how many; *ok as the traversal
+// reports it.
+template <bool ANY, class Entry>
+static int push_pop(int pushes, int canary, int* codes, int* ok) {
+    struct { Entry stack[kStack]; Entry beyond[64]; } mem;
+    for (Entry& e : mem.beyond) std::memcpy(&e, &canary, sizeof(int));
+    Trav s;
+    trav_none(s);
+    s.h.t = 1e30f;
+    s.node = kTravPop;
+    bool good = true;
+    for (int k = 1; k <= pushes; ++k) {
+        if constexpr (ANY) trav_push_any(s, mem.stack, k, good);
+        else trav_push(s, mem.stack, k, (float)k, good);
+    }
+    int n = 0;
+    for (;;) {
+        s.node = kTravPop;
+        if constexpr (ANY) trav_pop_any(s, mem.stack);
+        else trav_pop(s, mem.stack);
+        if (s.node == kTravDone || n >= 4 * kStack) break;
+        codes[n++] = s.node;
+    }
+    *ok = good;
+    for (Entry& e : mem.beyond)
+        if (std::memcmp(&e, &canary, sizeof(int)) != 0) return -1;   // written past the stack
+    return n;
+}
+extern "C" int host_stack_size() { return kStack; }
+extern "C" int host_push_pop(int any, int pushes, int canary, int* codes, int* ok) {
+    return any ? push_pop<true, int>(pushes, canary, codes, ok) : push_pop<false, int2>(pushes, canary, codes, ok);
+}
