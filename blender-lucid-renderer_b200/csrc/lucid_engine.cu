@@ -3697,10 +3697,13 @@ int Engine::render_diag_impl(const LucidRenderParams& p, float* out_host, float*
     f.records = 0;
 
     stats_ = LucidRenderStats{};
-    cudaEvent_t t0, t1, ka, kb, ca, cb;
-    cudaEventCreate(&t0);
-    cudaEventCreate(&t1);
-    for (cudaEvent_t* e : {&ka, &kb, &ca, &cb}) cudaEventCreate(e);
+    struct Events {   // destroyed on every return
+        cudaEvent_t e[6] = {};
+        Events() { for (cudaEvent_t& x : e) cudaEventCreate(&x); }
+        ~Events() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
+    } events;
+    const cudaEvent_t t0 = events.e[0], t1 = events.e[1], ka = events.e[2], kb = events.e[3], ca = events.e[4],
+                      cb = events.e[5];
     cudaEventRecord(t0, st);
     int status = LUCID_OK;
     int waves = 0;
@@ -3788,7 +3791,6 @@ int Engine::render_diag_impl(const LucidRenderParams& p, float* out_host, float*
         }
     }
     if (replay.valid()) replay_ms += replay.get();
-    for (cudaEvent_t e : {ka, kb, ca, cb}) cudaEventDestroy(e);
     // where a diagnostic render's time goes: the path kernel (raygen
     // included), the record copies to the host, and the host replay
     const char* names[3] = {"k_diag_paths", "diag_record_copy", "diag_replay_host"};
