@@ -499,22 +499,19 @@ constexpr int kBinVolume = 1, kBinCells = 2;
 constexpr long long kCellBinPaths = 1LL << 24;   // waves from this size on use the cells
 struct BinHist {
     int* h;
-    LD void clear(int bins) {
-        if (bins >= 0)
-            for (int i = threadIdx.x; i < kBins; i += blockDim.x) h[i] = 0;
+    LD void clear() {
+        for (int i = threadIdx.x; i < kBins; i += blockDim.x) h[i] = 0;
         __syncthreads();
     }
     // `at`: the ray's place in the queue
     LD void add(const DevScene& sc, const PathView& pv, int at, int bins, int prim, float t, int li, float lt, V3 o,
                 V3 d) {
-        if (bins < 0) return;
         const int c = bin_class(sc, prim, t, li, lt, o, d, (bins & kBinVolume) != 0);
         const int key = c * kCells + ((bins & kBinCells) && (c & 7) != 0 ? bin_cell(sc, o + d * t) : 0);
         pv.cls[at] = (unsigned short)key;
         atomicAdd(&h[key], 1);
     }
-    LD void flush(int bins, int* cnt) {
-        if (bins < 0) return;
+    LD void flush(int* cnt) {
         __syncthreads();
         for (int i = threadIdx.x; i < kBins; i += blockDim.x)
             if (h[i]) atomicAdd(&cnt[8 + i], h[i]);
@@ -530,7 +527,7 @@ __global__ void __launch_bounds__(128) k_trace_primary_t(DevScene sc, FrameParam
                                                        int records, int bins) {
     __shared__ int hist[kBins];
     BinHist bh{hist};
-    bh.clear(bins);
+    bh.clear();
     const int n = f.n_wave;
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt[0] = n;
     const V3 o = v3(f.pos[0], f.pos[1], f.pos[2]);
@@ -568,7 +565,7 @@ __global__ void __launch_bounds__(128) k_trace_primary_t(DevScene sc, FrameParam
             pv.rec_hash[id] = hs;
         }
     }
-    bh.flush(bins, cnt);
+    bh.flush(cnt);
     if (!ok) atomicAdd(&pv.errors[0], 1);
 }
 
@@ -611,7 +608,7 @@ __global__ void __launch_bounds__(128) k_trace_primary_batch(PathView pv, const 
     __shared__ int sbase[kMaxBatchPieces];
     for (int i = threadIdx.x; i < njobs; i += blockDim.x) sbase[i] = jobs[i].slot_base;
     BinHist bh{hist};
-    bh.clear(bins);   // ends with a block barrier, which also publishes sbase
+    bh.clear();   // ends with a block barrier, which also publishes sbase
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt[0] = n;
     const int lane = (int)lane_id();
     bool ok = true;
@@ -645,7 +642,7 @@ __global__ void __launch_bounds__(128) k_trace_primary_batch(PathView pv, const 
         pv.hit[id].light = make_float4(__int_as_float(-1), 1e30f, 0.f, 0.f);   // lights are invisible to camera rays
         bh.add(sc, pv, id, bins, h.prim, h.t, -1, 1e30f, o, d);
     }
-    bh.flush(bins, cnt);
+    bh.flush(cnt);
     if (!ok) atomicAdd(&pv.errors[0], 1);
 }
 
@@ -715,7 +712,7 @@ __global__ void __launch_bounds__(kPostThreads) k_trace_post(DevScene sc0, PathV
     const int n = *(volatile int*)&cnt[0];
     if (n <= stop) return;
     BinHist bh{hist};
-    bh.clear(bins);
+    bh.clear();
     bool ok = true;
     for (int i = blockIdx.x * kPostThreads + threadIdx.x; i < n; i += gridDim.x * kPostThreads) {
         const int id = pv.q0[i];
@@ -766,7 +763,7 @@ __global__ void __launch_bounds__(kPostThreads) k_trace_post(DevScene sc0, PathV
             pv.rec_hash[id] = hs;
         }
     }
-    bh.flush(bins, cnt);
+    bh.flush(cnt);
     if (!ok) atomicAdd(&pv.errors[0], 1);
 }
 
@@ -1211,8 +1208,7 @@ LD ShadeResult shade_path(const DevScene& sc, const FrameParams& f, const PathVi
 constexpr int kShadeThreads = 256;
 template <int ALGO, bool GUIDE = false, int MINB = 8, bool MULTI = false>
 __global__ void __launch_bounds__(kShadeThreads, MINB / 2) k_shade(DevScene sc, FrameParams f, PathView pv, int* cnt,
-                                                         int* cnt_next, int identity, int stop, const int* qin,
-                                                         int* qout) {
+                                                         int* cnt_next, int stop, const int* qin, int* qout) {
     __shared__ int s_base[2];
     const int n = *(volatile int*)&cnt[0];
     if (n <= stop) return;
@@ -1222,14 +1218,14 @@ __global__ void __launch_bounds__(kShadeThreads, MINB / 2) k_shade(DevScene sc, 
         const int base = s_base[it];
         if (base >= n) break;
         const int i = base + (int)threadIdx.x;
-        const int id = i < n ? (identity ? i : qin[i]) : -1;
+        const int id = i < n ? qin[i] : -1;
         const ShadeResult r = shade_path<ALGO, GUIDE>(path_scene<MULTI>(sc, pv, id), f, pv, id, &cnt[1]);
         const int at = warp_append(&cnt_next[0], r.cont);
         if (r.cont) qout[at] = id;
     }
 }
 
-using ShadeKernel = void (*)(DevScene, FrameParams, PathView, int*, int*, int, int, const int*, int*);
+using ShadeKernel = void (*)(DevScene, FrameParams, PathView, int*, int*, int, const int*, int*);
 template <int MINB>
 static ShadeKernel shade_kernel_lb(int algo, bool guide) {
     if (guide && algo == ALGO_MIS) return k_shade<ALGO_MIS, true, MINB>;
@@ -3388,10 +3384,10 @@ struct WavePlan {
     PathsKernel paths;
     int g_trace0 = 1, g_trace = 1, g_shade = 1, g_shadow = 1, g_bin = 1, g_paths = 1, g_post = 1;   // blocks
     int depths = 0, stop = -1;
-    int bins = -1;   // shading bins (BinHist); -1: the queues are shaded as they are
+    int bins = 0;    // shading bins (BinHist)
 };
-static WavePlan wave_plan(int device, int sms, int algo, bool guide, int profile, bool batch, bool binned,
-                          long long paths, int max_depth) {
+static WavePlan wave_plan(int device, int sms, int algo, bool guide, int profile, bool batch, long long paths,
+                          int max_depth) {
     WavePlan w;
     w.ks = batch ? launch_set_batch(algo) : launch_set(algo, guide, profile);
     w.paths = batch ? paths_kernel<true>(algo) : paths_kernel<false>(algo);
@@ -3421,9 +3417,8 @@ static WavePlan wave_plan(int device, int sms, int algo, bool guide, int profile
     }
     w.g_bin = sms * 8;
     w.g_post = sms * 4;
-    if (binned)
-        w.bins = ((algo == ALGO_VOLUME_MIS || algo == ALGO_VOLUME_SIMPLE) ? kBinVolume : 0) |
-                 (paths >= kCellBinPaths ? kBinCells : 0);
+    w.bins = ((algo == ALGO_VOLUME_MIS || algo == ALGO_VOLUME_SIMPLE) ? kBinVolume : 0) |
+             (paths >= kCellBinPaths ? kBinCells : 0);
     w.depths = std::max(0, max_depth);
     if (guide || max_depth < 1) return w;
     if (paths <= kPathsWave) {
@@ -3437,6 +3432,26 @@ static WavePlan wave_plan(int device, int sms, int algo, bool guide, int profile
     return w;
 }
 
+// k_paths for what the wavefront leaves of a wave (all of it where depths is 0).
+template <class Mark>
+static void enqueue_paths(const WavePlan& w, const DevScene& sc, const FrameParams& f, const PathView& base,
+                          cudaStream_t st, Mark mark, const BatchJob* jobs, int njobs, int slots) {
+    PathsCount* pc = reinterpret_cast<PathsCount*>(base.errors + 4);
+    int grid = w.g_paths, fma0 = 0;
+    if (!jobs) {
+        const float m = std::max(std::fabs(f.pos[0]), std::max(std::fabs(f.pos[1]), std::fabs(f.pos[2])));
+        fma0 = m <= sc.coord_bound;
+        if (w.depths == 0)
+            slots = ((f.tile_w + 7) / 8) * ((f.tile_h + 3) / 4) * 32 * (f.n_wave / std::max(f.npix, 1));
+    }
+    constexpr int kBlockLanes = kMinLanes * kPathsThreads / 32;
+    if (w.depths == 0) grid = std::min(grid, (slots + kBlockLanes - 1) / kBlockLanes);
+    cudaMemsetAsync(pc, 0, sizeof(PathsCount), st);
+    mark(K_PATHS, w.depths, 1, [&] {
+        w.paths<<<grid, kPathsThreads, 0, st>>>(sc, f, base, jobs, njobs, slots, fma0, w.depths, w.stop, pc);
+    });
+}
+
 // Launches one wave.  primary(pv, cnt): the camera-ray kernel; infer(depth,
 // pv, cnt, queue): guide inference before a depth's shading; mark(kind,
 // depth, kernels, launch): runs a step's launches (inside profiling events).
@@ -3444,7 +3459,6 @@ template <class Primary, class Infer, class Mark>
 static void enqueue_wave(const WavePlan& w, const DevScene& sc, const FrameParams& f, const PathView& base, int* qb,
                          int max_depth, cudaStream_t st, Primary primary, Infer infer, Mark mark,
                          const BatchJob* jobs = nullptr, int njobs = 0, int slots = 0) {
-    PathsCount* pc = reinterpret_cast<PathsCount*>(base.errors + 4);
     for (int depth = 0; depth < w.depths; ++depth) {
         int* cnt = base.counters + kCountersPerDepth * depth;
         int* cnt_next = base.counters + kCountersPerDepth * (depth + 1);
@@ -3464,14 +3478,9 @@ static void enqueue_wave(const WavePlan& w, const DevScene& sc, const FrameParam
                 post<<<w.g_post, kPostThreads, 0, st>>>(sc, pv, cnt, stop, traced, f.records, w.bins);
             });
         infer(depth, pv, cnt, qin);
-        int identity = depth == 0;
-        if (w.bins >= 0) {
-            mark(K_BIN, depth, 1, [&] { k_bin_scatter<<<w.g_bin, kBinThreads, 0, st>>>(pv, cnt, identity, stop, qin, qb); });
-            identity = 0;
-        }
+        mark(K_BIN, depth, 1, [&] { k_bin_scatter<<<w.g_bin, kBinThreads, 0, st>>>(pv, cnt, depth == 0, stop, qin, qb); });
         mark(K_SHADE, depth, 1, [&] {
-            w.ks.shade<<<w.g_shade, kShadeThreads, 0, st>>>(sc, f, pv, cnt, cnt_next, identity, stop,
-                                                            w.bins >= 0 ? qb : qin, qout);
+            w.ks.shade<<<w.g_shade, kShadeThreads, 0, st>>>(sc, f, pv, cnt, cnt_next, stop, qb, qout);
         });
         const bool any_bvh = jobs || sc.num_bvh_tris > 0 || sc.num_bnd_tris > 0;
         mark(K_SHADOW, depth, 1 + any_bvh, [&] {
@@ -3482,18 +3491,7 @@ static void enqueue_wave(const WavePlan& w, const DevScene& sc, const FrameParam
         });
     }
     if (max_depth < 1 || (w.depths == max_depth && w.stop < 0)) return;
-    int grid = w.g_paths, fma0 = 0;
-    if (!jobs) {
-        const float m = std::max(std::fabs(f.pos[0]), std::max(std::fabs(f.pos[1]), std::fabs(f.pos[2])));
-        fma0 = m <= sc.coord_bound;
-        slots = ((f.tile_w + 7) / 8) * ((f.tile_h + 3) / 4) * 32 * (f.n_wave / std::max(f.npix, 1));
-    }
-    constexpr int kBlockLanes = kMinLanes * kPathsThreads / 32;
-    if (w.depths == 0) grid = std::min(grid, (slots + kBlockLanes - 1) / kBlockLanes);
-    cudaMemsetAsync(pc, 0, sizeof(PathsCount), st);
-    mark(K_PATHS, w.depths, 1, [&] {
-        w.paths<<<grid, kPathsThreads, 0, st>>>(sc, f, base, jobs, njobs, slots, fma0, w.depths, w.stop, pc);
-    });
+    enqueue_paths(w, sc, f, base, st, mark, jobs, njobs, slots);
 }
 
 // Adds up the segments and shadow rays of a wave whose first eight counters
@@ -4013,7 +4011,7 @@ int Engine::render_impl(const LucidRenderParams& p, float* out_host, LucidSample
     f.npix = (int)np;
     f.records = records ? 1 : 0;
 
-    const WavePlan w = wave_plan(device_, num_sms_, algo_, guide, launch_profile_, false, true, wave_paths, p.max_depth);
+    const WavePlan w = wave_plan(device_, num_sms_, algo_, guide, launch_profile_, false, wave_paths, p.max_depth);
     PathView gv = P.view;   // the path view with the guide's buffers when guiding
     if (guide) {
         int rc2 = guide_buffers(wave_paths);
@@ -4373,7 +4371,7 @@ int Engine::render_batch(const BatchItem* items, int n, const char* algorithm, l
         CK(cudaMemcpyAsync(const_cast<BatchJob*>(d_jobs), tab.data(), tab.size() * sizeof(BatchJob),
                            cudaMemcpyHostToDevice, st));
         const int n_wave = (int)used;
-        const WavePlan w = wave_plan(device_, num_sms_, algo, false, 0, true, true, n_wave, depth);
+        const WavePlan w = wave_plan(device_, num_sms_, algo, false, 0, true, n_wave, depth);
         if (w.depths > 0) CK(cudaMemsetAsync(P.counters.p, 0, sizeof(int) * kCountersPerDepth * (w.depths + 1), st));
         PathView pv = P.view;
         pv.scenes = d_scenes;
@@ -4522,7 +4520,7 @@ void Engine::enqueue_iteration(void* fp, int n) {
     f.s0 = 0;
     f.samples = n;
     f.n_wave = n * f.npix;
-    const WavePlan w = wave_plan(device_, num_sms_, algo_, false, J.profile, false, true, f.n_wave, J.depth);
+    const WavePlan w = wave_plan(device_, num_sms_, algo_, false, J.profile, false, f.n_wave, J.depth);
     if (w.depths > 0) cudaMemsetAsync(P.counters.p, 0, sizeof(int) * kCountersPerDepth * (w.depths + 1), st);
     enqueue_wave(w, ds_->view, f, P.view, P.qb.p, J.depth, st, [&](const PathView& pv, int* cnt) {
         k_trace_primary_for(ds_->view, f.pos)<<<w.g_trace0, 128, 0, st>>>(ds_->view, f, pv, cnt, 0, w.bins);
@@ -4888,25 +4886,21 @@ void Engine::async_worker() {
 // that hands out every byte), or a latency-critical thread such as a
 // viewport draw callback that must not call cudaMalloc/cudaFree because
 // those calls can synchronise the whole device.  lucid_cuda_render_noalloc
-// serves them with the same kernels as lucid_cuda_render_device, but its
-// working memory (path state, queues, counters, film) lives in the
+// serves them with the whole-path kernel of lucid_cuda_render_device, but its
+// working memory (a wave's radiance, the error words, the film) lives in the
 // fixed-size device array below, which every GPU that loads this library
 // holds until the process exits.  The scene itself was allocated earlier by
 // lucid_cuda_load_scene_json.
 constexpr int kNoAllocPaths = 65536;              // paths per wave
 constexpr int kNoAllocPixels = 65536;             // tile pixels (e.g. 256 x 256)
 constexpr int kNoAllocMaxDepth = 64;
+static_assert(kNoAllocPaths <= kPathsWave, "its waves run in k_paths, which keeps a path's state in registers");
 constexpr size_t kNoAllocAlign = 256;
 constexpr size_t na_round(size_t b) { return (b + kNoAllocAlign - 1) / kNoAllocAlign * kNoAllocAlign; }
-constexpr size_t kNaState = na_round(sizeof(PathState) * kNoAllocPaths);
-constexpr size_t kNaHit = na_round(sizeof(PathHit) * kNoAllocPaths);
-constexpr size_t kNaShadow = na_round(sizeof(ShadowRec) * kNoAllocPaths);
 constexpr size_t kNaRad = na_round(sizeof(float4) * kNoAllocPaths);
-constexpr size_t kNaQ = na_round(sizeof(int) * kNoAllocPaths);
-constexpr size_t kNaCnt = na_round(sizeof(int) * kCountersPerDepth * (kNoAllocMaxDepth + 1));
 constexpr size_t kNaErr = na_round(sizeof(int) * kErrorInts);
 constexpr size_t kNaFilm = na_round(sizeof(float4) * kNoAllocPixels);
-constexpr size_t kNoAllocBytes = kNaState + kNaHit + kNaShadow + kNaRad + 2 * kNaQ + kNaCnt + kNaErr + kNaFilm;   // ~12 MB
+constexpr size_t kNoAllocBytes = kNaRad + kNaErr + kNaFilm;   // 2 MB
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
@@ -4957,17 +4951,9 @@ int Engine::render_noalloc(const LucidRenderParams& p, float* d_out) {
         base = g_noalloc_addr[device_];
     }
     PathView v{};
-    size_t off = 0;
-    auto take = [&](size_t bytes) { unsigned char* q = base + off; off += bytes; return (void*)q; };
-    v.st = (PathState*)take(kNaState); v.hit = (PathHit*)take(kNaHit); v.sh = (ShadowRec*)take(kNaShadow);
-    v.rad = (float4*)take(kNaRad);
-    int* q0 = (int*)take(kNaQ);
-    int* q1 = (int*)take(kNaQ);
-    v.counters = (int*)take(kNaCnt);
-    v.errors = (int*)take(kNaErr);
-    float4* film = (float4*)take(kNaFilm);
-    v.q0 = q0; v.q1 = q1;
-    v.rec_prim = nullptr; v.rec_cnt = nullptr; v.rec_hash = nullptr;
+    v.rad = (float4*)base;
+    v.errors = (int*)(base + kNaRad);
+    float4* film = (float4*)(base + kNaRad + kNaErr);
 
     cudaStream_t st = S(stream_);
     // the array keeps the previous call's contents: clear what starts at zero
@@ -4989,11 +4975,8 @@ int Engine::render_noalloc(const LucidRenderParams& p, float* d_out) {
         int this_spw = std::min(spw, p.samples - s0);
         f.s0 = s0;
         f.n_wave = (int)(this_spw * np);
-        const WavePlan w = wave_plan(device_, num_sms_, algo_, false, 0, false, false, f.n_wave, p.max_depth);
-        if (w.depths > 0) CK(cudaMemsetAsync(v.counters, 0, sizeof(int) * kCountersPerDepth * (w.depths + 1), st));
-        enqueue_wave(w, ds_->view, f, v, nullptr, p.max_depth, st, [&](const PathView& pv, int* cnt) {
-            k_trace_primary_for(ds_->view, f.pos)<<<w.g_trace0, 128, 0, st>>>(ds_->view, f, pv, cnt, 0, -1);
-        }, [](int, const PathView&, int*, const int*) {}, [](int, int, int, auto&& launch) { launch(); });
+        const WavePlan w = wave_plan(device_, num_sms_, algo_, false, 0, false, f.n_wave, p.max_depth);
+        enqueue_paths(w, ds_->view, f, v, st, [](int, int, int, auto&& launch) { launch(); }, nullptr, 0, 0);
         k_film<<<(f.npix + 255) / 256, 256, 0, st>>>(f.npix, this_spw, v.rad, film);
         CK(cudaGetLastError());
         // no wait here: stream order keeps the next wave behind this film sum

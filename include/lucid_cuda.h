@@ -231,7 +231,7 @@ int lucid_cuda_render_device(LucidCudaCtx* ctx, const LucidRenderParams* params,
  * calls which can synchronise the whole device.  Same result as
  * lucid_cuda_render_device (d_out_rgba: device pointer, tile_w*tile_h*4
  * floats), but all working memory sits in one fixed static device array of
- * about 12 MB that every GPU loading this library holds until exit.
+ * about 2 MB that every GPU loading this library holds until exit.
  * Limits: tile_w*tile_h <= 65536 pixels, 1 <= max_depth <= 64, no sample
  * records; larger requests return LUCID_ERR_INVALID.  Path diagnostics and
  * path guiding keep buffers of their own: while either is on for the
