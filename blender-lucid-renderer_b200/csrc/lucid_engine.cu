@@ -4910,6 +4910,16 @@ namespace {
 // address).
 std::mutex g_noalloc_mu;
 unsigned char* g_noalloc_addr[64] = {};
+// Calls on one device, whichever context they are made on, take turns with the
+// array: held until the call's work on it is done.
+std::mutex g_noalloc_turn[64];
+struct NoAllocTurn {
+    std::unique_lock<std::mutex> lk;
+    cudaStream_t st;
+    bool done = false;   // the stream has been waited for
+    NoAllocTurn(int device, cudaStream_t s) : lk(g_noalloc_turn[device]), st(s) {}
+    ~NoAllocTurn() { if (!done) cudaStreamSynchronize(st); }   // (then lk is released)
+};
 }  // namespace
 
 int Engine::render_noalloc(const LucidRenderParams& p, float* d_out) {
@@ -4956,6 +4966,7 @@ int Engine::render_noalloc(const LucidRenderParams& p, float* d_out) {
     float4* film = (float4*)(base + kNaRad + kNaErr);
 
     cudaStream_t st = S(stream_);
+    NoAllocTurn turn(device_, st);
     // the array keeps the previous call's contents: clear what starts at zero
     CK(cudaMemsetAsync(film, 0, sizeof(float4) * np, st));
     CK(cudaMemsetAsync(v.errors, 0, sizeof(int) * kErrorInts, st));
@@ -4985,6 +4996,7 @@ int Engine::render_noalloc(const LucidRenderParams& p, float* d_out) {
     int herr[4] = {0, 0, 0, 0};
     CK(cudaMemcpyAsync(herr, v.errors, sizeof(herr), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    turn.done = true;
     if (herr[0] != 0) return fail(LUCID_ERR_OVERFLOW, "BVH traversal stack overflow");
     if (status == LUCID_ERR_CANCELLED) return fail(LUCID_ERR_CANCELLED, "render cancelled");
     return LUCID_OK;

@@ -238,10 +238,9 @@ int lucid_cuda_render_device(LucidCudaCtx* ctx, const LucidRenderParams* params,
  * context, the call returns LUCID_ERR_INVALID.  The first call on a
  * device looks up the array's device address (cudaGetSymbolAddress) with
  * that device current; make that first call before any stream capture.
- * Every call on a device shares the array: calls that overlap on the GPU
- * (from several threads or contexts) race and must be serialised by the
- * caller.  The scene must already be loaded (lucid_cuda_load_scene_json
- * allocates). */
+ * Every call on a device shares the array: calls from several threads or
+ * contexts run one after another, each waiting for the ones before it.  The
+ * scene must already be loaded (lucid_cuda_load_scene_json allocates). */
 int lucid_cuda_render_noalloc(LucidCudaCtx* ctx, const LucidRenderParams* params, float* d_out_rgba);
 /* Batched jobs.  No counterpart in the reference: the add-on gives every
  * session its own Renderer and renders each job with its own calls
