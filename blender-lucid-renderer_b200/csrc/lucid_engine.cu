@@ -2791,7 +2791,8 @@ int Engine::stats(LucidRenderStats* out) const { *out = stats_; return LUCID_OK;
 
 // The next scene's arrays take the place of the last one's (allocating and
 // freeing some twenty of them took 4 ms a load) unless another engine still
-// uses it or it is an edited version of one.
+// uses it or it is an edited version of one (see upload_scene for a scene
+// that does not fit beside them).
 void Engine::free_scene() {
     if (ds_.use_count() > 1 || ds_->base) ds_ = std::make_shared<DeviceScene>();
     scene_loaded_ = false;
@@ -2890,7 +2891,10 @@ int Engine::load_scene_json(const char* json, size_t len) {
     HostScene hs;
     std::string err;
     free_scene();
-    if (!parse_scene_json(json, len, hs, err)) return fail(LUCID_ERR_INVALID, err);
+    if (!parse_scene_json(json, len, hs, err)) {
+        ds_->release();
+        return fail(LUCID_ERR_INVALID, err);
+    }
     return upload_scene(std::move(hs));
 }
 
@@ -2905,14 +2909,33 @@ int Engine::load_scene_arrays(const LucidSceneDesc& desc) {
     HostScene hs;
     std::string err;
     free_scene();
-    if (!build_scene_arrays(desc, hs, err)) return fail(LUCID_ERR_INVALID, err);
+    if (!build_scene_arrays(desc, hs, err)) {
+        ds_->release();
+        return fail(LUCID_ERR_INVALID, err);
+    }
     return upload_scene(std::move(hs));
 }
 
 // Uploads a flattened scene and builds its BVH (the caller holds the GPU
-// lock with the device current and the stream created).
+// lock with the device current and the stream created).  Where the last
+// scene's arrays leave too little memory the upload starts again without
+// them, and a load that fails keeps none.
 int Engine::upload_scene(HostScene&& hs) {
     host_ = std::move(hs);
+    int rc = upload_host_scene();
+    if (rc == LUCID_ERR_OOM) {
+        cudaGetLastError();   // the failed allocation's, which the next launch check would take for its own
+        ds_->release();
+        rc = upload_host_scene();
+    }
+    if (rc != LUCID_OK) {
+        cudaGetLastError();
+        ds_->release();
+    }
+    return rc;
+}
+
+int Engine::upload_host_scene() {
     DeviceScene& D = *ds_;
     const HostScene& H = host_;
     // boundary triangles (brute force list) and per-prim shading data

@@ -141,6 +141,7 @@ private:
     long long default_wave_paths(bool records) const;
     int build_bvh();
     int upload_scene(HostScene&& hs);
+    int upload_host_scene();
     int ensure_stream();
     int guide_buffers(long long paths);
     void scene_stats_locked(int out8[8]) const;

@@ -1,0 +1,81 @@
+"""GPU tests of the device memory of scene loads: a load that fails keeps none of
+the arrays of the scene before it, and a scene that fits without them loads."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+def _cloud(n):
+    import lucid_scenes as ls
+    rng = np.random.default_rng(n)
+    v = (rng.uniform(-1, 1, (n, 1, 3)) + rng.uniform(-0.01, 0.01, (n, 3, 3))).reshape(-1, 3)
+    return ls.scene_arrays({"meshes": [ls.mesh(v, np.arange(3 * n).reshape(n, 3), ls.material())], "native_lights": [],
+                            "environment": {"color": [0.2, 0.2, 0.3], "strength": 1.0}}, json_rounding=False)
+
+
+def _free():
+    import torch
+    return torch.cuda.mem_get_info()[0]
+
+
+def _warm(ctx):
+    """The kernels, the stream and the read-back block of a load are there."""
+    ctx.load_scene_arrays(_cloud(2000))
+
+
+@pytest.mark.parametrize("how", ["json", "arrays"])
+def test_a_load_that_fails_keeps_no_arrays(how):
+    import lucid_capi
+    ctx = lucid_capi.Context(0)
+    try:
+        _warm(ctx)
+        before = _free()
+        ctx.load_scene_arrays(_cloud(400_000))
+        held = before - _free()
+        assert held > 64 * MB
+        with pytest.raises(Exception):
+            if how == "json":
+                ctx.load_scene_json('{"meshes": [')
+            else:
+                bad = _cloud(8)
+                bad["meshes"][0]["triangles"][-1] = 9999
+                ctx.load_scene_arrays(bad)
+        assert _free() >= before - 8 * MB
+        ctx.load_scene_arrays(_cloud(2000))   # and the context goes on
+    finally:
+        ctx.close()
+
+
+def test_a_scene_that_fits_without_the_last_one_loads():
+    import torch
+    import lucid_capi
+    ctx = lucid_capi.Context(0)
+    try:
+        _warm(ctx)
+        big = _cloud(500_000)
+        before = _free()
+        ctx.load_scene_arrays(big)
+        held = before - _free()
+        # the next scene's build takes 301 bytes a triangle of temporaries (75 MB):
+        # more than is left beside the big one, whose arrays are not twice too
+        # large for it; without them there is room for its 50 MB as well
+        left = 55 * MB
+        assert held > 80 * MB
+        fill = torch.empty(_free() - left, dtype=torch.uint8, device="cuda")
+        try:
+            assert _free() < 70 * MB
+            ctx.load_scene_arrays(_cloud(260_000))
+            # a scene that cannot fit is refused, and the next one is not
+            with pytest.raises(Exception):
+                ctx.load_scene_arrays(_cloud(1_500_000))
+            ctx.load_scene_arrays(_cloud(2000))
+        finally:
+            del fill
+            torch.cuda.empty_cache()
+        ctx.set_camera(0.1, 0.15, 3.1, 0.0, -0.02, -1.0, 0.0, 1.0, 0.0, 50.0)
+        assert float(ctx.render(16, 16, samples=1)[0].sum()) > 0
+    finally:
+        ctx.close()
