@@ -2935,14 +2935,21 @@ int Engine::upload_scene(HostScene&& hs) {
     return rc;
 }
 
+// The first boundary-only prim from p on; num_prims when there is none.
+static int next_boundary(const HostScene& H, int p) {
+    if (H.num_boundary_meshes == 0 || p >= H.num_prims) return H.num_prims;
+    const unsigned char* const b = H.prim_boundary.data();
+    const void* q = std::memchr(b + p, 1, (size_t)(H.num_prims - p));
+    return q ? (int)(static_cast<const unsigned char*>(q) - b) : H.num_prims;
+}
+
 int Engine::upload_host_scene() {
     DeviceScene& D = *ds_;
     const HostScene& H = host_;
     // boundary triangles (brute force list) and per-prim shading data
     std::vector<float4> bnd;
-    for (int p = 0; H.num_boundary_meshes > 0 && p < H.num_prims; ++p)
-        if (H.prim_boundary[p])
-            for (int k = 0; k < 3; ++k) bnd.push_back(H.tri[3 * p + k]);
+    for (int p = next_boundary(H, 0); p < H.num_prims; p = next_boundary(H, p + 1))
+        for (int k = 0; k < 3; ++k) bnd.push_back(H.tri[3 * p + k]);
     auto up = [&](auto& buf, const auto& vec) -> cudaError_t {
         cudaError_t e = buf.fit(vec.size());
         if (e != cudaSuccess) return e;
@@ -3110,8 +3117,7 @@ int Engine::build_bvh() {
         std::vector<float4> boxes;
         const float bpad = maxabs * 9.5367431640625e-07f + 1e-30f;
         int k = 0;
-        for (int p = 0; H.num_boundary_meshes > 0 && p < np; ++p) {
-            if (!H.prim_boundary[p]) continue;
+        for (int p = next_boundary(H, 0); p < np; p = next_boundary(H, p + 1)) {
             const int mesh = H.prim_info[(size_t)p].x;
             bool fresh = boxes.empty();
             if (!fresh) {
@@ -3159,9 +3165,7 @@ int Engine::build_bvh() {
     }
     float sdiag = std::sqrt((hi[0] - lo[0]) * (hi[0] - lo[0]) + (hi[1] - lo[1]) * (hi[1] - lo[1]) +
                             (hi[2] - lo[2]) * (hi[2] - lo[2]));
-    int nonbnd = np;
-    if (H.num_boundary_meshes > 0)
-        for (int p = 0; p < np; ++p) nonbnd -= H.prim_boundary[p] ? 1 : 0;
+    const int nonbnd = np - D.view.num_bnd_tris;
     std::vector<std::pair<float, int>> cand;   // (diagonal, prim)
     if (np > 0) {
         k_big_candidates<<<(np + 255) / 256, 256, 0, st>>>(d_verts, d_boundary, np, 0.25f * sdiag, kCandidates, d_pb, d_cand);
