@@ -3313,8 +3313,11 @@ int Engine::build_bvh() {
     for (int l = levels - 1; l >= 0; --l) k_tree_inner<<<g, 256, 0, st>>>(d_flat, l, d_list, d_tc, d_inner);
     for (int l = 0; l < levels; ++l) k_tree_place<<<g, 256, 0, st>>>(d_flat, l, d_list, d_tc, d_inner, d_place, D.nodes2.p);
     // 4-wide collapse, a level at a time: node i of the collapse stands for
-    // binary node d_list[i] (the levels' list is done with).
-    CK(D.nodes.fit((size_t)nodes));
+    // binary node d_list[i] (the levels' list is done with).  A 4-wide node with
+    // inner children takes in three binary nodes and has at most four of them,
+    // one without takes in one at least: (2 nodes + 1) / 3 at most (the
+    // 1M-triangle scene has 159,152 for 320,882 binary nodes).
+    CK(D.nodes.fit(((size_t)nodes * 2 + 1) / 3));
     k_wide_root<<<1, 1, 0, st>>>(root, d_list, d_tc);
     for (int l = 0; l < levels; ++l) k_wide_level<<<g, 256, 0, st>>>(d_flat, l, d_list, d_tc, D.nodes.p);
     CK(cudaGetLastError());

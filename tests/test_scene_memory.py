@@ -1,5 +1,6 @@
 """GPU tests of the device memory of scene loads: a load that fails keeps none of
-the arrays of the scene before it, and a scene that fits without them loads."""
+the arrays of the scene before it, a scene that fits without them loads, and the
+4-wide nodes take no more room than there can be of them."""
 import numpy as np
 import pytest
 
@@ -77,5 +78,36 @@ def test_a_scene_that_fits_without_the_last_one_loads():
             torch.cuda.empty_cache()
         ctx.set_camera(0.1, 0.15, 3.1, 0.0, -0.02, -1.0, 0.0, 1.0, 0.0, 50.0)
         assert float(ctx.render(16, 16, samples=1)[0].sum()) > 0
+    finally:
+        ctx.close()
+
+
+def test_room_for_the_4_wide_nodes_there_can_be():
+    import lucid_capi
+    ctx = lucid_capi.Context(0)
+    try:
+        _warm(ctx)
+        before = _free()
+        n = 1_500_000
+        ctx.load_scene_arrays(_cloud(n))
+        held = before - _free()
+        stats = ctx.scene_stats()
+        nodes4, nodes2 = int(stats[6]), int(stats[7]) - 1   # (a binary tree over its leaves)
+        assert nodes4 <= (2 * nodes2 + 1) // 3
+        # per prim: info 16, class 1, normals 64, BVH triangle 64; 64 a binary node, 128 a 4-wide one
+        need = n * 145 + nodes2 * 64 + (2 * nodes2 + 1) // 3 * 128
+        assert held < need + 16 * MB   # (allocations come in 2 MB)
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("n", [5, 6, 7, 8, 9, 10, 13, 17, 29, 64, 100, 333, 1025, 20_001])
+def test_4_wide_nodes_stay_below_their_bound(n):
+    import lucid_capi
+    ctx = lucid_capi.Context(0)
+    try:
+        ctx.load_scene_arrays(_cloud(n))
+        stats = ctx.scene_stats()
+        assert 1 <= int(stats[6]) <= (2 * (int(stats[7]) - 1) + 1) // 3
     finally:
         ctx.close()
