@@ -3408,7 +3408,7 @@ static_assert(K_NUM <= LUCID_MAX_KERNEL_KINDS, "kernel kinds");
 // depth launched).  `depths` bounds the launches of a wave whose queue
 // shrinks as usual (two depths, and one more for each doubling from 2^19
 // paths on); where it shrinks more slowly k_paths takes a longer queue.
-constexpr long long kPathsWave = 1LL << 17;
+constexpr long long kPathsWave = Engine::kPathsWave;
 struct WavePlan {
     LaunchSet ks;
     PathsKernel paths;

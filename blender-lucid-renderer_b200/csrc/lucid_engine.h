@@ -65,6 +65,7 @@ public:
     void set_combining(bool on) { combine_ = on; }
     static void combine_stats(int device, long long* batches, long long* calls);
     static constexpr long long kCombinePaths = 1LL << 22;
+    static constexpr long long kPathsWave = 1LL << 17;   // paths up to which a wave runs in one kernel
     // Device memory of a batch: path state for wave_paths paths and films of `pixels`.
     static long long batch_bytes(long long pixels, long long wave_paths);
     int render_debug(int tx, int ty, int tw, int th, int fw, int fh, const char* mode, float* out_host);

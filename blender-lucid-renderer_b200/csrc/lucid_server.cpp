@@ -368,9 +368,11 @@ int Server::pick_chunk(Engine& e, Job& j, int id, int& offset) {
         if (d.interactive && ms > kInteractiveMs) break;
     }
     // then the launch profiles (resident CTAs per SM) at that size, when the
-    // job has samples left for a trial of each
+    // job has samples left for a trial of each and iterations that reach the
+    // wavefront kernels: smaller ones are the same launches under both
     int best_profile = 0, cur_profile = 0;
-    for (int prof = 1; prof < 2 && offset + best <= d.samples; ++prof) {
+    const bool wavefront = (long long)best * d.width * d.height > Engine::kPathsWave;
+    for (int prof = 1; wavefront && prof < 2 && offset + best <= d.samples; ++prof) {
         int rc = e.job_set_profile(prof, false);
         if (rc != LUCID_OK) return -rc;
         cur_profile = prof;
