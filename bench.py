@@ -102,9 +102,9 @@ SM_COUNT, SCHEDULERS_PER_SM = 148, 4
 
 def issue_roofline(kern: dict, sm_mhz):
     """Issue-slot roofline of the traversal and shading kernels: warp
-    instructions per unit of work (ncu smsp__inst_executed.sum over a whole
-    render, divided by its units; profiles/*.md 'inst_per_unit' lines) times
-    the kernel's live unit rate, against one warp instruction per scheduler
+    instructions per unit of work (ncu smsp__inst_executed.sum over a
+    480x270, 8 spp render of the scene, divided by its units; profiles/*.md
+    'inst_per_unit' lines) times the kernel's live unit rate, against one warp instruction per scheduler
     per cycle (148 SMs x 4 schedulers x the median SM clock sampled during
     the timed region).  'lanes' is the mean active lanes per issued
     instruction from the same capture (SIMT efficiency = lanes / 32)."""
@@ -118,7 +118,8 @@ def issue_roofline(kern: dict, sm_mhz):
             continue
         rate = ipu * v["units"] / (v["total_ms"] / 1000.0)
         out[k] = {"inst_per_unit": ipu, "achieved_ginst_s": rate / 1e9, "peak_ginst_s": peak / 1e9,
-                  "frac": rate / peak, "lanes": profile_figure("lanes_per_inst", k)}
+                  "frac": rate / peak, "lanes": profile_figure("lanes_per_inst", k),
+                  "counts_from": "480x270, 8 spp"}
     return out or None
 
 
@@ -396,9 +397,9 @@ def diagnostics(device: int) -> dict:
     """Path diagnostics at scale (render_tile with diagnostics enabled: the
     diagnostic integrators, device path records, the film replayed on the
     host in the reference's loop order): the Cornell configuration's 16x16
-    recording window at 16 spp, and a 1920x1080 Cornell frame at 4 spp with
-    the standard preset (subsample 2), each against the same render without
-    diagnostics."""
+    recording window at 16 spp, and a 1920x1080 Cornell frame (--width and
+    --height for a smaller one) at 4 spp with the standard preset (subsample
+    2), each against the same render without diagnostics."""
     import lucid_capi
     import lucid_scenes as ls
     sc, cam = ls.cornell_box()
@@ -408,7 +409,7 @@ def diagnostics(device: int) -> dict:
     c.set_algorithm("mis")
     out = {}
     for name, (tx, ty, tw, th, fw, fh, spp) in {"cornell_window_16x16_16spp": (120, 120, 16, 16, 256, 256, 16),
-                                               "cornell_1920x1080_4spp_standard": (0, 0, 1920, 1080, 1920, 1080, 4)}.items():
+                                               f"cornell_{W}x{H}_4spp_standard": (0, 0, W, H, W, H, 4)}.items():
         c.diag_disable()
         c.render(tw, th, fw, fh, spp, 0, 8, tile_x=tx, tile_y=ty)   # warm
         t0 = time.perf_counter()
