@@ -1568,9 +1568,9 @@ __global__ void __launch_bounds__(kPathsThreads, 512 / kPathsThreads) k_paths(De
             slots = *(volatile const int*)&pv.counters[kCountersPerDepth * d];
             if (slots <= stop || d == depths) break;
         }
-        if (slots == 0) return;
         q = (d & 1) ? pv.q1 : pv.q0;
     }
+    if (slots == 0) return;
     int2 stack[kStack];
     Trav s;
     // few paths are spread over the warps there are: each then waits for fewer
@@ -2947,6 +2947,26 @@ int Engine::upload_scene(HostScene&& hs) {
     return rc;
 }
 
+// What a no-allocation render launches, launched once per device with nothing
+// to do: the first launch of a kernel loads its code, and the first with a
+// larger stack than any before it makes the driver allocate local memory for
+// every thread the device can hold (120 MB for k_paths).  Both would be device
+// allocations of the first render_noalloc call (and fail it where another
+// allocator holds the rest).  Without the memory the load succeeds all the
+// same: a render may find more of it.
+static void reserve_kernel_memory(int device, cudaStream_t st) {
+    static std::mutex mu;
+    static bool done[64] = {};
+    std::lock_guard<std::mutex> lk(mu);
+    if (device < 0 || device >= 64 || done[device]) return;
+    for (int algo = 0; algo < 5; ++algo)
+        paths_kernel<false>(algo)<<<1, kPathsThreads, 0, st>>>(DevScene{}, FrameParams{}, PathView{}, nullptr, 0, 0, 0, 0,
+                                                               -1, nullptr);
+    k_film<<<1, 32, 0, st>>>(0, 0, nullptr, nullptr);
+    k_output<<<1, 32, 0, st>>>(0, 0, nullptr, nullptr);
+    done[device] = cudaGetLastError() == cudaSuccess;
+}
+
 // The first boundary-only prim from p on; num_prims when there is none.
 static int next_boundary(const HostScene& H, int p) {
     if (H.num_boundary_meshes == 0 || p >= H.num_prims) return H.num_prims;
@@ -3008,6 +3028,7 @@ int Engine::upload_host_scene() {
     v.has_boundary = v.num_bnd_tris > 0;
     int rc = build_bvh();
     if (rc != LUCID_OK) return rc;
+    reserve_kernel_memory(device_, S(stream_));
     CK(cudaStreamSynchronize(S(stream_)));
     scene_loaded_ = true;
     return LUCID_OK;
