@@ -123,9 +123,12 @@ LD bool test_leaf_any(const float4* tris, int code, V3 o, V3 d, float tmin, floa
 // can have that moves the ray by far less than the boxes' padding, and products
 // with coordinates up to 2^67 stay finite.  The reciprocals of all other
 // components keep their bits; the triangle test takes the direction itself.
-// (1M-triangle 1920x1080, 64 spp frame: camera rays 15.3 -> 16.1 ms, shadow rays
-// 37.0 -> 36.1 ms, closest hits the same.)
-LD float slab_inv(float d) { return 1.0f / copysignf(fmaxf(fabsf(d), 8.673617379884035e-19f), d); }
+// (1M-triangle 1920x1080, 64 spp frame: camera rays 15.3 -> 15.6 ms, shadow rays
+// 37.0 -> 36.2 ms, closest hits the same.)
+LD float slab_inv(float d) {
+    const float most = 1.152921504606846976e18f;   // 2^60
+    return fminf(fmaxf(1.0f / d, -most), most);
+}
 LD V3 slab_inv(V3 d) { return v3(slab_inv(d.x), slab_inv(d.y), slab_inv(d.z)); }
 
 // Conservative slab test of one box; returns entry distance in tn.
@@ -269,7 +272,10 @@ LD bool bvh_closest(const DevScene& sc, V3 o, V3 d, float tmin, HitRec& h) {
     if (sc.num_big_tris) list_closest(sc.big_tris, sc.num_big_tris, o, d, tmin, h);
     if (sc.num_bvh_tris == 0) return true;
     if (sc.root2 < 0) { test_leaf_closest(sc.bvh_tris, sc.root2, o, d, tmin, h); return true; }
-    const V3 inv = slab_inv(d);
+    V3 inv = slab_inv(d);
+    // (opaque: the compiler else holds more of their making through the walk, 56
+    // registers in place of 48 in the camera kernel, 15.9 ms in place of 15.6)
+    asm volatile("" : "+f"(inv.x), "+f"(inv.y), "+f"(inv.z));
     const V3 ooi = v3(-o.x * inv.x, -o.y * inv.y, -o.z * inv.z);
     int2 stack[kStack];   // (code, entry distance)
     int sp = 0;
